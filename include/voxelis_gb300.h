@@ -198,7 +198,8 @@ int vx_build_dense_async(vx_interner *it, uint32_t n, const vx_tree *trees_dev,
 /* Batched to_vec (utils/common.rs:158-246): out receives n dense [y][z][x] grids of side 2^d, one
  * per tree, back to back; every tree must have the same depth d. With VX_MEM_DEVICE `out` is device
  * memory (16-byte aligned); with VX_MEM_HOST the grids are produced in pieces of whole 32-row slabs
- * and copied out. HBM-write-bound: one CTA per 32^3 cube expands the cube's subtree in shared memory. */
+ * and copied out. One thread resolves a quad (4^3 voxels) from the root
+ * down. */
 int vx_trees_to_dense(vx_interner *it, uint32_t n, const vx_tree *trees, void *out, vx_mem mem);
 /* Asynchronous form, all arguments in device memory, trees checked on the device (a tree whose
  * depth is not `depth` reports VX_E_INVALID_ARG at the next sync and leaves its grid zero). */

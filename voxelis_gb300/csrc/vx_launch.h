@@ -154,7 +154,6 @@ cudaError_t launch_get_many(const DevInterner &I, uint64_t n, const uint32_t *tr
 // to_vec over trees of depth d into [y][z][x] grids: cubes [cube_begin, cube_begin + n_cubes) of side
 // min(32, 2^d), ordered (tree, cy, cz, cx); cube_begin must start a cy-slab and `out` points at that
 // slab's first element.
-size_t to_dense_smem_bytes(int d, int vbits);
 cudaError_t launch_to_dense(const DevInterner &I, const uint32_t *trees, int d, uint64_t cube_begin,
                             uint64_t n_cubes, void *out, int num_sms, cudaStream_t s);
 // Occupancy masks of n_trees dense grids of side 2^d placed at offsets (x, y, z) of a 64^3 builder:

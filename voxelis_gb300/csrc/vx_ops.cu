@@ -12,6 +12,8 @@
 //                 the children's references, interner/mod.rs:767-772), its LIFO free list and its
 //                 32768-entry release queue (P3 lifts the limit).
 //   rehash        rebuilds the branch table from the live nodes once tombstones accumulate.
+#include <type_traits>
+
 #include "vx_launch.h"
 
 namespace vxg {
@@ -655,152 +657,141 @@ __global__ void count_live_kernel(DevInterner I, unsigned long long *out2) {
 
 
 // ---- to_vec: DAG -> dense grid (utils/common.rs:158-246) ----------------------------------------
-// One CTA per cube of side C = 2^lc (lc = min(d, 5)) of one tree; cubes are ordered (tree, cy, cz,
-// cx), so a run of whole cy-slabs is one contiguous range of the output. Thread 0 descends from the
-// root to the cube's root (d - lc levels); EMPTY or a leaf met on the way, or as the cube root, makes
-// the cube uniform (EMPTY children are never visited by to_vec, leaving the default; a leaf fills
-// its whole sub-cube). Otherwise the cube's subtree is expanded level by level in shared memory,
-// 8^k ids at level k in Morton order, a leaf or EMPTY replicating into its 8 children; the last
-// level resolves each voxel to the value of the node covering it (a leaf's value, or the value of a
-// node at depth d, as to_vec's else-branch does) and the CTA writes the cube row by row with 16-byte
-// stores.
+// One thread per quad (4^3 voxels). The thread descends from its tree's root to the quad's node (d - 2
+// levels; lanes of a warp share most of the path, so these loads are L1 hits); EMPTY or a leaf met on
+// the way makes the quad uniform (EMPTY children are never visited by to_vec, leaving the default; a
+// leaf fills its whole sub-cube). Otherwise the quad's 8 groups are resolved to voxels: EMPTY, a leaf's
+// value, or the values of the nodes at depth d, as to_vec's else-branch does. The 16 rows of 4 voxels go
+// straight from registers to the output.
+// Nothing is staged: no shared memory, no CTA barrier, every quad independent; bound by instruction
+// issue and the latency of the gathers (ncu: issue 59%, DRAM 17%). Quads of a cube of side 32 are
+// numbered x first, then z, then y: a warp covers 8 x 4 quads of one y, so each of its stores writes
+// whole 32-byte sectors (u8) and its lanes share nodes.
+// 4096 dune chunks of 32^3 u8 (134 MB): 60 us, one 512^3 u8 cave tree: 78 us (132 and 180 us when a CTA
+// expanded each 32^3 cube level by level in 68 KB of shared memory, with a barrier per level). Slower:
+// four lanes resolving four quads together, 16 bytes of a node record each (77 and 118 us); exchanging
+// rows between lanes for 16-byte stores (no gain).
 constexpr int kDenseOutThreads = 256;
 
-__device__ __forceinline__ uint32_t morton_compact3(uint32_t m) {
-    m &= 0x09249249u;
-    m = (m ^ (m >> 2)) & 0x030C30C3u;
-    m = (m ^ (m >> 4)) & 0x0300F00Fu;
-    m = (m ^ (m >> 8)) & 0x030000FFu;
-    m = (m ^ (m >> 16)) & 0x000003FFu;
-    return m;
+__device__ __forceinline__ uint64_t child_ro(const DevInterner &I, uint64_t id, uint32_t k) {
+    return __ldg(reinterpret_cast<const unsigned long long *>(I.children) + 8ull * id_index(id) + k);
 }
 
 template <class T>
-__device__ __forceinline__ uint4 replicate16(uint32_t v) {
-    uint32_t w = sizeof(T) == 1 ? (v & 0xFFu) * 0x01010101u : (v & 0xFFFFu) * 0x00010001u;
-    return make_uint4(w, w, w, w);
+__device__ __forceinline__ uint32_t value_ro(const DevInterner &I, uint64_t id) {
+    return __ldg(reinterpret_cast<const T *>(I.values) + id_index(id));
+}
+
+// The 8 voxels under a bottom group's node (or above it: an EMPTY or leaf ancestor), x fastest, then y,
+// then z, as two bytes or 16-bit elements a word: w[y + 2z] = v(0, y, z) | v(1, y, z) << bits.
+template <class T>
+__device__ __forceinline__ void group_rows(const DevInterner &I, uint64_t g, uint32_t w[4]) {
+    constexpr int B = 8 * sizeof(T);
+    if (g == EMPTY_ID) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) w[r] = 0;
+    } else if (id_is_leaf(g)) {
+        const uint32_t v = value_ro<T>(I, g);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) w[r] = v | (v << B);
+    } else {
+        const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(I.children + 8ull * id_index(g));
+        ulonglong2 c[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) c[r] = __ldg(src + r);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const uint32_t lo = c[r].x ? value_ro<T>(I, c[r].x) : 0u, hi = c[r].y ? value_ro<T>(I, c[r].y) : 0u;
+            w[r] = lo | (hi << B);
+        }
+    }
 }
 
 template <class T>
 __global__ void __launch_bounds__(kDenseOutThreads) to_dense_kernel(DevInterner I, const uint32_t *trees, int d,
-                                                                     int lc, uint64_t cube_begin, uint64_t n_cubes,
-                                                                     T *out) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const uint32_t C = 1u << lc;
-    const uint32_t K = 1u << (d - lc);          // cubes per axis
-    const uint64_t K2 = (uint64_t)K * K, K3 = K2 * K;
-    const uint64_t S = 1ull << d;
-    const uint64_t slab_elems = (uint64_t)C * S * S;
-    const uint32_t tile_elems = C * C * C;
-    T *tile = reinterpret_cast<T *>(smem);
-    uint64_t *lv_big = reinterpret_cast<uint64_t *>(smem + ((tile_elems * sizeof(T) + 15) & ~15u));
-    uint64_t *lv_small = lv_big + (lc >= 1 ? (1u << (3 * (lc - 1))) : 1u);
-    __shared__ uint64_t cube_root;
-    __shared__ int uniform;  // 1: whole cube = cube_val
-    __shared__ uint32_t cube_val;
-    const uint64_t first_slab = cube_begin / K2;
+                                                                     uint64_t cube_begin, uint64_t n_cubes, T *out) {
+    using Row = typename std::conditional<sizeof(T) == 1, uint32_t, uint2>::type;  // 4 voxels along x
+    const int qb = (d < 5 ? d : 5) - 2;    // quads a cube has along an axis, log2
+    const int kb = d - 2 - qb;             // cubes a tree has along an axis, log2
+    const uint32_t qm = (1u << qb) - 1u, km = (1u << kb) - 1u;
+    const uint64_t S = 1ull << d, S2 = S * S;
+    const uint64_t total = n_cubes << (3 * qb);
+    const uint64_t first_row = (cube_begin >> (2 * kb)) << (qb + 2);  // out starts at this y of the trees' stack
     bool bad = false;
-    for (uint64_t c = cube_begin + blockIdx.x; c < cube_begin + n_cubes; c += gridDim.x) {
-        const uint64_t t_idx = c / K3;
-        const uint32_t within = (uint32_t)(c % K3);
-        const uint32_t cx = within % K, cz = (within / K) % K, cy = within / (K * K);
-        if (threadIdx.x == 0) {
-            const uint32_t t = __ldg(trees + t_idx);
-            const int td = t < I.tree_cap ? I.depths[t] : TREE_UNUSED;
-            uint64_t node = EMPTY_ID;
-            int un = 1;
-            uint32_t val = 0;
-            if (td != d) {
-                bad = true;
-            } else {
-                node = I.roots[t];
-                const int L0 = d - lc;
-                for (int depth = 0; depth < L0 && node != EMPTY_ID && id_is_branch(node); ++depth) {
-                    const int sh = L0 - depth - 1;
-                    const uint32_t ci = ((cx >> sh) & 1) | (((cy >> sh) & 1) << 1) | (((cz >> sh) & 1) << 2);
-                    node = I.children[8ull * id_index(node) + ci];
-                }
-                if (node == EMPTY_ID) {
-                    val = 0;
-                } else if (!id_is_branch(node)) {
-                    val = node_value(I, id_index(node));
-                } else {
-                    un = 0;
-                }
-            }
-            cube_root = node;
-            uniform = un;
-            cube_val = val;
-        }
-        __syncthreads();
-        T *dst = out + (c / K2 - first_slab) * slab_elems;  // the cube's cy-slab
-        const uint64_t cube_off = (uint64_t)cz * C * S + (uint64_t)cx * C;
-        if (!uniform) {
-            // level-by-level expansion: level 0 is the cube root; ping-pong between the two id buffers
-            // so that level lc-1 (the parents of the voxels) lands in lv_big
-            uint64_t *cur = ((lc - 1) & 1) ? lv_small : lv_big;
-            if (threadIdx.x == 0) cur[0] = cube_root;
-            __syncthreads();
-            for (int k = 0; k + 1 < lc; ++k) {
-                uint64_t *nxt = (cur == lv_big) ? lv_small : lv_big;
-                const uint32_t m = 1u << (3 * (k + 1));
-                for (uint32_t j = threadIdx.x; j < m; j += blockDim.x) {
-                    const uint64_t p = cur[j >> 3];
-                    uint64_t ch = p;
-                    if (p != EMPTY_ID && id_is_branch(p)) ch = I.children[8ull * id_index(p) + (j & 7)];
-                    nxt[j] = ch;
-                }
-                __syncthreads();
-                cur = nxt;
-            }
-            const uint32_t m = 1u << (3 * (lc - 1));
-            for (uint32_t j = threadIdx.x; j < m; j += blockDim.x) {
-                const uint64_t p = cur[j];
-                uint32_t v8[8];
-                if (p == EMPTY_ID) {
+    for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t cube = cube_begin + (q >> (3 * qb));
+        const uint32_t c = (uint32_t)cube, w = (uint32_t)q;
+        const uint32_t X = ((c & km) << qb) | (w & qm);  // quad coordinates in the tree
+        const uint32_t Z = (((c >> kb) & km) << qb) | ((w >> qb) & qm);
+        const uint32_t Y = (((c >> (2 * kb)) & km) << qb) | ((w >> (2 * qb)) & qm);
+        const uint64_t t_idx = cube >> (3 * kb);
+        const uint32_t t = __ldg(trees + t_idx);
+        uint64_t node = EMPTY_ID;
+        if (t < I.tree_cap && I.depths[t] == d)
+            node = I.roots[t];
+        else
+            bad = true;
+        for (int sh = d - 3; sh >= 0 && node != EMPTY_ID && !id_is_leaf(node); --sh)
+            node = child_ro(I, node, ((X >> sh) & 1) | (((Y >> sh) & 1) << 1) | (((Z >> sh) & 1) << 2));
+        T *dst = out + ((t_idx << d) + 4 * Y - first_row) * S2 + 4 * Z * S + 4 * X;
+        uint64_t g[8];
+        const bool split = node != EMPTY_ID && !id_is_leaf(node);
+        if (split) {
+            const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(I.children + 8ull * id_index(node));
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) v8[k] = 0;
-                } else if (!id_is_branch(p)) {
-                    const uint32_t v = node_value(I, id_index(p));
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) v8[k] = v;
-                } else {
-                    const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(I.children + 8ull * id_index(p));
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const ulonglong2 w = src[k];
-                        v8[2 * k] = w.x ? node_value(I, id_index(w.x)) : 0u;
-                        v8[2 * k + 1] = w.y ? node_value(I, id_index(w.y)) : 0u;
-                    }
-                }
-                const uint32_t bx = morton_compact3(j), by = morton_compact3(j >> 1), bz = morton_compact3(j >> 2);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const uint32_t x = 2 * bx + (k & 1), y = 2 * by + ((k >> 1) & 1), z = 2 * bz + (k >> 2);
-                    tile[(y * C + z) * C + x] = (T)v8[k];
-                }
-            }
-            __syncthreads();
-        }
-        // store the cube: rows of C elements along x
-        const uint32_t row_bytes = C * (uint32_t)sizeof(T);
-        if (row_bytes % 16 == 0) {
-            const uint32_t vec_per_row = row_bytes / 16, rows = C * C;
-            const uint4 fillv = replicate16<T>(cube_val);
-            for (uint32_t q = threadIdx.x; q < rows * vec_per_row; q += blockDim.x) {
-                const uint32_t r = q / vec_per_row, v = q % vec_per_row;
-                const uint32_t y = r / C, z = r % C;
-                uint4 w = uniform ? fillv : reinterpret_cast<const uint4 *>(tile + (size_t)r * C)[v];
-                T *row = dst + cube_off + (uint64_t)y * S * S + (uint64_t)z * S;
-                reinterpret_cast<uint4 *>(row)[v] = w;
+            for (int k = 0; k < 4; ++k) {
+                const ulonglong2 v = __ldg(src + k);
+                g[2 * k] = v.x;
+                g[2 * k + 1] = v.y;
             }
         } else {
-            for (uint32_t q = threadIdx.x; q < tile_elems; q += blockDim.x) {
-                const uint32_t y = q / (C * C), z = (q / C) % C, x = q % C;
-                dst[cube_off + (uint64_t)y * S * S + (uint64_t)z * S + x] = uniform ? (T)cube_val : tile[q];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) g[k] = node;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {  // the two groups along x at (gy, gz)
+            const int gy = k & 1, gz = k >> 1;
+            uint32_t a[4], b[4];
+            group_rows<T>(I, g[2 * k], a);
+            if (split) {
+                group_rows<T>(I, g[2 * k + 1], b);
+            } else {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) b[r] = a[r];
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                Row *p = reinterpret_cast<Row *>(dst + (2 * gy + (r & 1)) * S2 + (2 * gz + (r >> 1)) * S);
+                if constexpr (sizeof(T) == 1)
+                    *p = a[r] | (b[r] << 16);
+                else
+                    *p = make_uint2(a[r], b[r]);
             }
         }
-        __syncthreads();
+    }
+    if (bad) set_error(I, ERR_INVALID, 52);
+}
+
+// Trees of depth 1: one thread per tree, 8 voxels.
+template <class T>
+__global__ void __launch_bounds__(kDenseOutThreads) to_dense_depth1_kernel(DevInterner I, const uint32_t *trees,
+                                                                            uint64_t begin, uint64_t n, T *out) {
+    bool bad = false;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t t = __ldg(trees + begin + i);
+        uint64_t node = EMPTY_ID;
+        if (t < I.tree_cap && I.depths[t] == 1)
+            node = I.roots[t];
+        else
+            bad = true;
+        uint32_t w[4];
+        group_rows<T>(I, node, w);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {  // w[y + 2z] holds row (y, z); the grid is [y][z][x]
+            T *row = out + 8 * i + 4 * (r & 1) + 2 * (r >> 1);
+            row[0] = (T)w[r];
+            row[1] = (T)(w[r] >> (8 * sizeof(T)));
+        }
     }
     if (bad) set_error(I, ERR_INVALID, 52);
 }
@@ -1147,32 +1138,25 @@ __global__ void ser_tail_kernel(DevInterner I, const uint32_t *leaf_rank, const 
     *total = o;
 }
 
-size_t to_dense_smem_bytes(int d, int vbits) {
-    const int lc = d < 5 ? d : 5;
-    const size_t tile = ((size_t)1 << (3 * lc)) * (vbits / 8);
-    const size_t big = lc >= 1 ? ((size_t)1 << (3 * (lc - 1))) : 1;
-    const size_t small = lc >= 2 ? ((size_t)1 << (3 * (lc - 2))) : 1;
-    return ((tile + 15) & ~(size_t)15) + 8 * (big + small);
-}
-
 cudaError_t launch_to_dense(const DevInterner &I, const uint32_t *trees, int d, uint64_t cube_begin,
                             uint64_t n_cubes, void *out, int num_sms, cudaStream_t s) {
     if (n_cubes == 0) return cudaSuccess;
-    const int lc = d < 5 ? d : 5;
-    const size_t smem = to_dense_smem_bytes(d, I.vbits);
-    uint64_t blocks = n_cubes;
-    const uint64_t cap = (uint64_t)num_sms * 8;
+    const uint64_t threads = d == 1 ? n_cubes : n_cubes << (3 * (d < 5 ? d - 2 : 3));
+    uint64_t blocks = (threads + kDenseOutThreads - 1) / kDenseOutThreads;
+    const uint64_t cap = (uint64_t)num_sms * 64;
     if (blocks > cap) blocks = cap;
     count_launches(1);
-    if (I.vbits == 8) {
-        cudaFuncSetAttribute(to_dense_kernel<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        to_dense_kernel<uint8_t><<<(unsigned)blocks, kDenseOutThreads, smem, s>>>(I, trees, d, lc, cube_begin,
-                                                                                  n_cubes, (uint8_t *)out);
-    } else {
-        cudaFuncSetAttribute(to_dense_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        to_dense_kernel<uint16_t><<<(unsigned)blocks, kDenseOutThreads, smem, s>>>(I, trees, d, lc, cube_begin,
-                                                                                   n_cubes, (uint16_t *)out);
-    }
+    auto launch = [&](auto *o) {
+        using T = std::remove_pointer_t<decltype(o)>;
+        if (d == 1)
+            to_dense_depth1_kernel<T><<<(unsigned)blocks, kDenseOutThreads, 0, s>>>(I, trees, cube_begin, n_cubes, o);
+        else
+            to_dense_kernel<T><<<(unsigned)blocks, kDenseOutThreads, 0, s>>>(I, trees, d, cube_begin, n_cubes, o);
+    };
+    if (I.vbits == 8)
+        launch((uint8_t *)out);
+    else
+        launch((uint16_t *)out);
     return cudaGetLastError();
 }
 
