@@ -162,11 +162,11 @@ cudaError_t launch_occupancy(const DevInterner &I, const void *grids, uint32_t n
                              unsigned long long *counts, uint32_t *slot, uint32_t *ids, unsigned long long *mcounts,
                              uint32_t *n_mat, uint32_t mat_cap, unsigned long long *global, unsigned long long *per_mat,
                              unsigned long long *active, int num_sms, cudaStream_t s);
-// Batched occupancy masks, 8-bit voxels: tree t goes to builder builder_of[t]; counts (256 per
-// builder), global, per_mat must be zero on entry.
+// Batched occupancy masks, 8-bit voxels: tree t goes to builder builder_of[t]; head (one word a builder)
+// and next (one a tree) are scratch. Every word of the outputs is written.
 cudaError_t launch_occupancy_many(const DevInterner &I, const uint8_t *grids, uint32_t n_trees, int d,
                                   const uint32_t *builder_of, const uint32_t *offsets, uint32_t n_builders,
-                                  unsigned int *counts, uint32_t *slot, uint32_t max_mat, uint32_t *ids,
+                                  uint32_t *head, uint32_t *next, uint32_t max_mat, uint32_t *ids,
                                   unsigned long long *mcounts, uint32_t *n_mat, unsigned long long *global,
                                   unsigned long long *per_mat, unsigned long long *active, int num_sms, cudaStream_t s);
 // Model serialisation: plan (renumbering, record sizes, offsets, total bytes into *total), then
