@@ -1878,12 +1878,10 @@ int vx_serialize_model(vx_interner *it, uint32_t n_chunks, const vx_tree *trees,
     if (!it || !size || (n_chunks && (!trees || !positions))) return VX_E_INVALID_ARG;
     for (uint32_t k = 0; k < n_chunks; ++k)
         if (!tree_ok(it, trees[k])) return set_err(it, VX_E_INVALID_ARG, "unknown tree handle");
-    const size_t words = serialize_scratch_words(it->dev);
-    const size_t tmpw = scan_tmp_words(it->capacity) * 4;  // the recursive scan's block sums
-    VX_CUDA(it->ws.reserve(Carve::need({words * 4, tmpw * 4, (size_t)n_chunks * 4 + 4, (size_t)n_chunks * 12 + 4, 64})));
+    const size_t words = serialize_scratch_words(it->dev, n_chunks);
+    VX_CUDA(it->ws.reserve(Carve::need({words * 4, (size_t)n_chunks * 4 + 4, (size_t)n_chunks * 12 + 4, 64})));
     Carve c(it->ws.p);
     uint32_t *w = c.take<uint32_t>(words);
-    uint32_t *tmp = c.take<uint32_t>(tmpw);
     uint32_t *dt = c.take<uint32_t>((size_t)n_chunks + 1);
     int32_t *dp = c.take<int32_t>((size_t)n_chunks * 3 + 1);
     unsigned long long *dtotal = c.take<unsigned long long>(2);
@@ -1895,7 +1893,7 @@ int vx_serialize_model(vx_interner *it, uint32_t n_chunks, const vx_tree *trees,
     unsigned long long total = 0;
     {
         Phase ph(it, VX_PROF_GET);
-        VX_CUDA(launch_serialize_plan(it->dev, w, tmp, n_chunks, dt, dtotal, it->num_sms, s));
+        VX_CUDA(launch_serialize_plan(it->dev, w, n_chunks, dt, dtotal, it->num_sms, s));
     }
     VX_CUDA(cudaMemcpyAsync(&total, dtotal, 8, cudaMemcpyDeviceToHost, s));
     int st = sync_and_check(it);
@@ -1907,7 +1905,7 @@ int vx_serialize_model(vx_interner *it, uint32_t n_chunks, const vx_tree *trees,
     uint8_t *dout = static_cast<uint8_t *>(it->staging.p);
     {
         Phase ph(it, VX_PROF_GET);
-        VX_CUDA(launch_serialize_write(it->dev, w, n_chunks, dt, dp, dout, dtotal, it->num_sms, s));
+        VX_CUDA(launch_serialize_write(it->dev, w, n_chunks, dt, dp, dout, it->num_sms, s));
     }
     VX_CUDA(cudaMemcpyAsync(out, dout, total, cudaMemcpyDeviceToHost, s));
     return sync_and_check(it);
@@ -1930,12 +1928,11 @@ int vx_deserialize_model(vx_interner *it, const uint8_t *data, uint64_t n_bytes,
     const VtmScratchSizes z = vtm_scratch_sizes(n_bytes);
     const uint64_t chunk_room = std::min<uint64_t>(max_chunks, z.chunk_cap);  // a chunk record takes 25+ bytes
     VX_CUDA(it->staging.reserve(n_bytes + 64));
-    VX_CUDA(it->ws.reserve(Carve::need({sizeof(VtmSections), z.table_words * 8, z.entry_words * 8, z.leaf_cap * 4,
+    VX_CUDA(it->ws.reserve(Carve::need({sizeof(VtmSections), z.table_words * 8, z.leaf_cap * 4,
                                         z.branch_cap * 4, z.chunk_cap * 4, chunk_room * 4 + 4, chunk_room * 12 + 4})));
     Carve c(it->ws.p);
     VtmSections *sec = c.take<VtmSections>(1);
     uint64_t *tables = c.take<uint64_t>(z.table_words);
-    uint64_t *entries = c.take<uint64_t>(z.entry_words);
     uint32_t *leaf_off = c.take<uint32_t>(z.leaf_cap);
     uint32_t *branch_off = c.take<uint32_t>(z.branch_cap);
     uint32_t *chunk_off = c.take<uint32_t>(z.chunk_cap);
@@ -1951,8 +1948,7 @@ int vx_deserialize_model(vx_interner *it, const uint8_t *data, uint64_t n_bytes,
     VX_CUDA(cudaMemcpyAsync(sec, &h, sizeof(h), cudaMemcpyHostToDevice, s));
     {
         Phase ph(it, VX_PROF_GET);
-        VX_CUDA(launch_vtm_parse(it->dev, bytes, n_bytes, sec, tables, entries, leaf_off, branch_off, chunk_off,
-                                 it->num_sms, s));
+        VX_CUDA(launch_vtm_parse(it->dev, bytes, n_bytes, sec, tables, leaf_off, branch_off, chunk_off, it->num_sms, s));
     }
     VX_CUDA(cudaMemcpyAsync(&h, sec, sizeof(h), cudaMemcpyDeviceToHost, s));
     st = sync_and_check(it);

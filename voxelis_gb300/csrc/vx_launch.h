@@ -171,13 +171,12 @@ cudaError_t launch_occupancy_many(const DevInterner &I, const uint8_t *grids, ui
                                   unsigned long long *per_mat, unsigned long long *active, int num_sms, cudaStream_t s);
 // Model serialisation: plan (renumbering, record sizes, offsets, total bytes into *total), then
 // write (records, counts and chunk records into `out`, which holds *total bytes). `w` holds
-// serialize_scratch_words(I) u32 and is shared by both steps.
-size_t serialize_scratch_words(const DevInterner &I);
-cudaError_t launch_serialize_plan(const DevInterner &I, uint32_t *w, uint32_t *tmp_scan, uint32_t n_chunks,
-                                  const uint32_t *trees, unsigned long long *total, int num_sms, cudaStream_t s);
+// serialize_scratch_words(I, n_chunks) u32 (256-byte aligned) and is shared by both steps.
+size_t serialize_scratch_words(const DevInterner &I, uint32_t n_chunks);
+cudaError_t launch_serialize_plan(const DevInterner &I, uint32_t *w, uint32_t n_chunks, const uint32_t *trees,
+                                  unsigned long long *total, int num_sms, cudaStream_t s);
 cudaError_t launch_serialize_write(const DevInterner &I, uint32_t *w, uint32_t n_chunks, const uint32_t *trees,
-                                   const int32_t *pos, uint8_t *out, unsigned long long *total, int num_sms,
-                                   cudaStream_t s);
+                                   const int32_t *pos, uint8_t *out, int num_sms, cudaStream_t s);
 
 // ---- model deserialisation (vx_vtm.cu) -------------------------------------------------------
 // Section state of one parse, in device memory: sections 0 leaves, 1 branches, 2 chunks. The host
@@ -191,7 +190,7 @@ struct VtmSections {
 struct VtmScratchSizes {
     uint32_t seg_bytes;
     uint64_t n0, n1, n2;                     // tables per level (upper bounds)
-    uint64_t table_words, entry_words;       // u64 words of the tables and the entry states
+    uint64_t table_words;                    // u64 words of the tables
     uint64_t leaf_cap, branch_cap, chunk_cap;  // u32 record offsets per section (upper bounds)
 };
 uint32_t vtm_segment_bytes(uint64_t n_bytes);
@@ -200,8 +199,8 @@ VtmScratchSizes vtm_scratch_sizes(uint64_t n_bytes);
 // leaf_off / branch_off / chunk_off, counts into sec. A stream the reference panics on sets
 // ERR_REF_PANIC and leaves done[] of the failing section 0.
 cudaError_t launch_vtm_parse(const DevInterner &I, const uint8_t *bytes, uint64_t n_bytes, VtmSections *sec,
-                             uint64_t *tables, uint64_t *entries, uint32_t *leaf_off, uint32_t *branch_off,
-                             uint32_t *chunk_off, int num_sms, cudaStream_t s);
+                             uint64_t *tables, uint32_t *leaf_off, uint32_t *branch_off, uint32_t *chunk_off,
+                             int num_sms, cudaStream_t s);
 // Writes the parsed nodes into an interner that holds none (slots 1..L+B), the branch table, the
 // refcounts and the roots of trees[k] (k < C), with the chunk positions into positions[3k..3k+2].
 cudaError_t launch_vtm_place(const DevInterner &I, const uint8_t *bytes, const VtmSections *sec, uint64_t n_nodes,

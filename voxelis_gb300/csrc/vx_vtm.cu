@@ -14,11 +14,14 @@
 // 48 bytes) one lane parses the section's records from segment start + o while they start inside the
 // segment, giving table T0[seg][o] = records << 8 | exit offset into the next segment (or dead, when
 // a record fails to parse). Tables of 32 consecutive segments compose into T1, those of 32 T1 into T2
-// (S is chosen so that a section has at most 32^3 segments). One CTA then walks T2 from entry 0 and
-// walks down, giving every segment its true entry offset and the number of records before it; one
-// thread per segment re-parses its records from there, validates each against the reference's
-// assertions, records its offset by rank, and the thread that parses the section's last record reads
-// the next section's header. Sections run one after another (each start is the previous one's end).
+// (S is chosen so that a section has at most 32^3 segments). Walking T2 from entry 0, then T1, then T0
+// gives every segment its true entry offset and the number of records before it; one thread per segment
+// re-parses its records from there, validates each against the reference's assertions, records its
+// offset by rank, and the thread that parses the section's last record reads the next section's header.
+// Sections run one after another (each start is the previous one's end).
+// Three launches a section, a CTA for each group of 32 segments in the first and last: the group's bytes
+// and tables are in shared memory, so that the dependent steps (byte after byte, table after table) are
+// shared-memory reads.
 //
 // Placement. With L, B and C known the host creates C trees; then one kernel writes every leaf and
 // the BlockId of every branch (types = which children are leaves), and a second writes the branch
@@ -138,21 +141,39 @@ __device__ __forceinline__ uint64_t vtm_step(uint64_t e, const uint64_t *T) {
     return (((e >> 8) + (t >> 8)) << 8) | (t & 0xFFu);
 }
 
-__global__ void __launch_bounds__(kThreads) vtm_table_kernel(const uint8_t *b, uint64_t n, const VtmSections *sec,
-                                                             int kind, int vb, uint32_t S, uint64_t *T0) {
+// The segment tables of one group of kFan segments (T0), and their composition (T1). Small segments: the
+// length of the record at every byte of the group is found once (a thread a byte), and the tables hop
+// from record to record; larger ones are parsed from every entry.
+constexpr int kTableThreads = 512;
+constexpr uint32_t kStageSeg = 64;
+constexpr uint32_t kStageBytes = kFan * kStageSeg;
+
+__global__ void __launch_bounds__(kTableThreads) vtm_table_kernel(const uint8_t *b, uint64_t n, const VtmSections *sec,
+                                                                  int kind, int vb, uint32_t S, uint64_t *T0, uint64_t *T1) {
+    __shared__ uint64_t tab[kFan * kEntries];
+    __shared__ uint8_t bytes[kStageBytes + 64];  // a record that starts in the last segment reads 47 bytes past it
+    __shared__ uint8_t lens[kStageBytes];
     if (sec->count[kind] == 0) return;
     const Geometry g = vtm_geometry(sec, kind, n, S);
-    const unsigned lane = threadIdx.x & 31u;
-    const uint32_t warps = gridDim.x * (blockDim.x / 32);
-    for (uint32_t seg = (blockIdx.x * blockDim.x + threadIdx.x) / 32; seg < g.n0; seg += warps) {
-        const uint64_t s0 = g.start + (uint64_t)seg * S;
-        const uint64_t end = s0 + S < n ? s0 + S : n;
-        for (int h = 0; h < kEntries / 32; ++h) {
-            const uint32_t o = lane + 32u * h;
-            uint64_t pos = s0 + o, cnt = 0;
+    for (uint32_t group = blockIdx.x; group < g.n1; group += gridDim.x) {
+        const uint64_t g0 = g.start + (uint64_t)group * kFan * S, left = n - g0;  // positions below are from g0
+        const bool staged = S <= kStageSeg;
+        if (staged) {
+            const uint32_t m = (uint32_t)(left < kStageBytes + 64 ? left : kStageBytes + 64);
+            for (uint32_t k = threadIdx.x; k < m; k += kTableThreads) bytes[k] = b[g0 + k];
+            __syncthreads();
+            const uint32_t starts = m < kStageBytes ? m : kStageBytes;
+            for (uint32_t k = threadIdx.x; k < starts; k += kTableThreads)
+                lens[k] = (uint8_t)vtm_record_len(kind, bytes, k, left, vb);
+            __syncthreads();
+        }
+        const uint32_t segs = g.n0 - group * kFan < kFan ? g.n0 - group * kFan : kFan;
+        for (uint32_t k = threadIdx.x; k < segs * kEntries; k += kTableThreads) {
+            const uint64_t s0 = (uint64_t)(k / kEntries) * S, end = s0 + S < left ? s0 + S : left;
+            uint64_t pos = s0 + k % kEntries, cnt = 0;
             bool ok = true;
             while (pos < end) {
-                const uint32_t l = vtm_record_len(kind, b, pos, n, vb);
+                const uint32_t l = staged ? lens[pos] : vtm_record_len(kind, b + g0, pos, left, vb);
                 if (!l) {
                     ok = false;
                     break;
@@ -160,58 +181,35 @@ __global__ void __launch_bounds__(kThreads) vtm_table_kernel(const uint8_t *b, u
                 pos += l;
                 ++cnt;
             }
-            T0[(uint64_t)seg * kEntries + o] = ok ? (cnt << 8) | (pos - end) : kDead;
+            const uint64_t t = ok ? (cnt << 8) | (pos - end) : kDead;
+            tab[k] = t;
+            T0[(uint64_t)group * kFan * kEntries + k] = t;
         }
+        __syncthreads();
+        if (threadIdx.x < kEntries) {
+            uint64_t e = threadIdx.x;
+            for (uint32_t j = 0; j < segs; ++j) e = vtm_step(e, tab + j * kEntries);
+            T1[(uint64_t)group * kEntries + threadIdx.x] = e;
+        }
+        __syncthreads();  // the shared arrays are reused by the next group
     }
 }
 
-// U[g][o] = the kFan child tables of group g applied in turn from entry o (one warp per group).
+// T2[g] = the kFan T1 tables of group g applied in turn from every entry (one CTA per group).
 __global__ void __launch_bounds__(kThreads) vtm_compose_kernel(uint64_t n, const VtmSections *sec, int kind, uint32_t S,
-                                                               int level, const uint64_t *T, uint64_t *U) {
+                                                               const uint64_t *T1, uint64_t *T2) {
+    __shared__ uint64_t tab[kFan * kEntries];
     if (sec->count[kind] == 0) return;
     const Geometry geo = vtm_geometry(sec, kind, n, S);
-    const uint32_t n_child = level == 1 ? geo.n0 : geo.n1, n_group = level == 1 ? geo.n1 : geo.n2;
-    const unsigned lane = threadIdx.x & 31u;
-    const uint32_t warps = gridDim.x * (blockDim.x / 32);
-    for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / 32; g < n_group; g += warps) {
-        for (int h = 0; h < kEntries / 32; ++h) {
-            const uint32_t o = lane + 32u * h;
-            uint64_t e = o;
-            for (uint32_t j = 0; j < (uint32_t)kFan && (uint64_t)g * kFan + j < n_child; ++j)
-                e = vtm_step(e, T + ((uint64_t)g * kFan + j) * kEntries);
-            U[(uint64_t)g * kEntries + o] = e;
-        }
-    }
-}
-
-// One CTA of 1024 threads: the true entry state of every T2 group, T1 group and segment.
-__global__ void __launch_bounds__(1024) vtm_down_kernel(uint64_t n, const VtmSections *sec, int kind, uint32_t S,
-                                                        const uint64_t *T0, const uint64_t *T1, const uint64_t *T2,
-                                                        uint64_t *E0, uint64_t *E1, uint64_t *E2) {
-    if (sec->count[kind] == 0) return;
-    const Geometry g = vtm_geometry(sec, kind, n, S);
-    if (threadIdx.x == 0) {
-        uint64_t e = 0;
-        for (uint32_t k = 0; k < g.n2; ++k) {
-            E2[k] = e;
-            e = vtm_step(e, T2 + (uint64_t)k * kEntries);
-        }
-    }
+    const uint32_t g = blockIdx.x;
+    if (g >= geo.n2) return;
+    const uint32_t m = geo.n1 - g * kFan < kFan ? geo.n1 - g * kFan : kFan;
+    for (uint32_t k = threadIdx.x; k < m * kEntries; k += kThreads) tab[k] = T1[(uint64_t)g * kFan * kEntries + k];
     __syncthreads();
-    if (threadIdx.x < g.n2) {
-        uint64_t e = E2[threadIdx.x];
-        for (uint32_t j = 0; j < (uint32_t)kFan && threadIdx.x * kFan + j < g.n1; ++j) {
-            E1[threadIdx.x * kFan + j] = e;
-            e = vtm_step(e, T1 + ((uint64_t)threadIdx.x * kFan + j) * kEntries);
-        }
-    }
-    __syncthreads();
-    for (uint32_t h = threadIdx.x; h < g.n1; h += blockDim.x) {
-        uint64_t e = E1[h];
-        for (uint32_t j = 0; j < (uint32_t)kFan && (uint64_t)h * kFan + j < g.n0; ++j) {
-            E0[(uint64_t)h * kFan + j] = e;
-            e = vtm_step(e, T0 + ((uint64_t)h * kFan + j) * kEntries);
-        }
+    if (threadIdx.x < kEntries) {
+        uint64_t e = threadIdx.x;
+        for (uint32_t j = 0; j < m; ++j) e = vtm_step(e, tab + j * kEntries);
+        T2[(uint64_t)g * kEntries + threadIdx.x] = e;
     }
 }
 
@@ -231,23 +229,49 @@ __device__ void vtm_close(const DevInterner &I, const uint8_t *b, uint64_t n, Vt
     sec->done[kind] = 1;
 }
 
+// One group of kFan segments: their true entry states (the T2 tables before the group's, the T1 tables before
+// it in its T2 group, then its own T0 tables), then a thread a segment parses and checks its records.
 __global__ void __launch_bounds__(kThreads) vtm_emit_kernel(DevInterner I, const uint8_t *b, uint64_t n,
                                                             VtmSections *sec, int kind, int vb, uint32_t S,
-                                                            const uint64_t *E0, uint32_t *off, uint64_t cap) {
+                                                            const uint64_t *T0, const uint64_t *T1, const uint64_t *T2,
+                                                            uint32_t *off, uint64_t cap) {
+    __shared__ uint64_t tab[kFan * kEntries];
+    __shared__ uint64_t entry[kFan], at_s;
     const uint64_t count = sec->count[kind];
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t group = blockIdx.x;
     if (sec->start[kind] > n) return;  // an earlier section failed (its error bit is set)
     if (count == 0) {
-        if (t == 0) vtm_close(I, b, n, sec, kind, sec->start[kind]);
+        if (group == 0 && threadIdx.x == 0) vtm_close(I, b, n, sec, kind, sec->start[kind]);
         return;
     }
     const Geometry g = vtm_geometry(sec, kind, n, S);
     if (g.n0 == 0) {
-        if (t == 0) set_error(I, ERR_REF_PANIC, 43 + kind);  // records announced past the end
+        if (group == 0 && threadIdx.x == 0) set_error(I, ERR_REF_PANIC, 43 + kind);  // records announced past the end
         return;
     }
-    if (t >= g.n0) return;
-    const uint64_t e = E0[t];
+    if (group >= g.n1) return;
+    // three walks: T2 up to this group's, T1 up to this group, T0 of this group
+    for (int level = 2; level >= 0; --level) {
+        const uint32_t in = level == 2 ? group / kFan : (level == 1 ? group % kFan : 0u);  // tables to apply
+        const uint32_t m = level ? in : (g.n0 - group * kFan < kFan ? g.n0 - group * kFan : kFan);
+        const uint64_t *src = level == 2 ? T2
+                              : level == 1 ? T1 + (uint64_t)(group / kFan) * kFan * kEntries
+                                           : T0 + (uint64_t)group * kFan * kEntries;
+        for (uint32_t k = threadIdx.x; k < m * kEntries; k += kThreads) tab[k] = src[k];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint64_t e = level == 2 ? 0 : at_s;
+            for (uint32_t j = 0; j < m; ++j) {
+                if (level == 0) entry[j] = e;
+                e = vtm_step(e, tab + j * kEntries);
+            }
+            at_s = e;
+        }
+        __syncthreads();
+    }
+    const uint32_t t = group * kFan + threadIdx.x;
+    if (threadIdx.x >= kFan || t >= g.n0) return;
+    const uint64_t e = entry[threadIdx.x];
     if (e == kDead) return;
     uint64_t rank = e >> 8;
     if (rank >= count) return;
@@ -403,7 +427,7 @@ __global__ void vtm_finish_kernel(DevInterner I, const VtmSections *sec) {
 uint32_t vtm_segment_bytes(uint64_t n) {
     uint64_t s = (n + 32767) / 32768;  // at most 32^3 segments a section
     s = (s + 63) & ~63ull;
-    return (uint32_t)(s < 256 ? 256 : s);
+    return (uint32_t)(s < 64 ? 64 : s);
 }
 
 VtmScratchSizes vtm_scratch_sizes(uint64_t n) {
@@ -414,7 +438,6 @@ VtmScratchSizes vtm_scratch_sizes(uint64_t n) {
     z.n1 = (z.n0 + kFan - 1) / kFan + 1;
     z.n2 = (z.n1 + kFan - 1) / kFan + 1;
     z.table_words = (z.n0 + z.n1 + z.n2) * kEntries;
-    z.entry_words = z.n0 + z.n1 + z.n2;
     z.leaf_cap = n / 2 + 1;     // a leaf record holds at least 2 bytes
     z.branch_cap = n / 3 + 1;   // a branch record at least 3
     z.chunk_cap = n / 25 + 1;   // a chunk record at least 25
@@ -422,27 +445,22 @@ VtmScratchSizes vtm_scratch_sizes(uint64_t n) {
 }
 
 cudaError_t launch_vtm_parse(const DevInterner &I, const uint8_t *bytes, uint64_t n, VtmSections *sec,
-                             uint64_t *tables, uint64_t *entries, uint32_t *leaf_off, uint32_t *branch_off,
-                             uint32_t *chunk_off, int num_sms, cudaStream_t s) {
+                             uint64_t *tables, uint32_t *leaf_off, uint32_t *branch_off, uint32_t *chunk_off,
+                             int num_sms, cudaStream_t s) {
     const VtmScratchSizes z = vtm_scratch_sizes(n);
     const int vb = I.vbits / 8;
     uint64_t *T0 = tables, *T1 = T0 + z.n0 * kEntries, *T2 = T1 + z.n1 * kEntries;
-    uint64_t *E0 = entries, *E1 = E0 + z.n0, *E2 = E1 + z.n1;
     uint32_t *offs[3] = {leaf_off, branch_off, chunk_off};
     const uint64_t caps[3] = {z.leaf_cap, z.branch_cap, z.chunk_cap};
-    auto blocks_for = [&](uint64_t items, int per_block) {
-        uint64_t g = (items + per_block - 1) / per_block;
-        const uint64_t cap = (uint64_t)num_sms * 16;
-        return (unsigned)(g < 1 ? 1 : (g > cap ? cap : g));
-    };
+    const uint64_t cap = (uint64_t)num_sms * 16;
+    const unsigned groups = (unsigned)z.n1;  // at most 32^2 and one
     for (int kind = 0; kind < 3; ++kind) {
-        count_launches(5);
-        vtm_table_kernel<<<blocks_for(z.n0, kThreads / 32), kThreads, 0, s>>>(bytes, n, sec, kind, vb, z.seg_bytes, T0);
-        vtm_compose_kernel<<<blocks_for(z.n1, kThreads / 32), kThreads, 0, s>>>(n, sec, kind, z.seg_bytes, 1, T0, T1);
-        vtm_compose_kernel<<<blocks_for(z.n2, kThreads / 32), kThreads, 0, s>>>(n, sec, kind, z.seg_bytes, 2, T1, T2);
-        vtm_down_kernel<<<1, 1024, 0, s>>>(n, sec, kind, z.seg_bytes, T0, T1, T2, E0, E1, E2);
-        vtm_emit_kernel<<<(unsigned)((z.n0 + kThreads - 1) / kThreads), kThreads, 0, s>>>(
-            I, bytes, n, sec, kind, vb, z.seg_bytes, E0, offs[kind], caps[kind]);
+        count_launches(3);
+        vtm_table_kernel<<<groups < cap ? groups : (unsigned)cap, kTableThreads, 0, s>>>(
+            bytes, n, sec, kind, vb, z.seg_bytes, T0, T1);
+        vtm_compose_kernel<<<(unsigned)z.n2, kThreads, 0, s>>>(n, sec, kind, z.seg_bytes, T1, T2);
+        vtm_emit_kernel<<<groups, kThreads, 0, s>>>(I, bytes, n, sec, kind, vb, z.seg_bytes, T0, T1, T2, offs[kind],
+                                                    caps[kind]);
     }
     return cudaGetLastError();
 }
