@@ -38,6 +38,8 @@
 //      7 - c references: + (7 - 2c).
 //   Q7 (voxtree.rs:742-758): the fill leaf's Phase-0 reference is never released when the batch
 //      also has patches: + 1.
+#include <algorithm>
+
 #include "vx_launch.h"
 
 namespace vxg {
@@ -962,9 +964,12 @@ __global__ void __launch_bounds__(512, VX_APPLY_MIN_BLOCKS) apply_single_kernel(
         // round r reads set r % 3 and writes set (r + 1) % 3; set (r + 2) % 3 was read by round r - 1
         // and is written by round r + 1, so it is cleared now
         uint32_t *fr[2] = {frontier_a, frontier_b};
+        extern __shared__ uint32_t leaf_smem[];
+        const LeafDrops D = leaf_drops_init(I, leaf_smem);  // the leaf counts were flushed before the last barrier
         for (int r = 0; r < rounds; ++r) {
+            if (*(volatile unsigned long long *)&ctr->rel_count[r % 3] == 0) break;  // the same answer in every CTA
             if (t0) ctr->rel_count[(r + 2) % 3] = 0;
-            release_round_range(I, fr[r & 1], fr[(r + 1) & 1], &ctr->rel_count[r % 3], &ctr->rel_count[(r + 1) % 3],
+            release_round_range(I, D, fr[r & 1], fr[(r + 1) & 1], &ctr->rel_count[r % 3], &ctr->rel_count[(r + 1) % 3],
                                 cta_base, stride);
             if (!grid_sync(I)) return;
         }
@@ -1110,7 +1115,7 @@ size_t apply_single_scan_words(int num_sms) { return (size_t)num_sms * 32 + 64; 
 cudaError_t launch_apply_single(const DevInterner &I, const ApplyArgs &a, bool check_depths, bool clear_pass,
                                 uint32_t *frontier_a, uint32_t *frontier_b, int rounds, int num_sms, cudaStream_t s) {
     const int bt = a.threads > 0 ? a.threads : kThreads;
-    const size_t smem = leaf_refs_smem(I);
+    const size_t smem = std::max(leaf_refs_smem(I), release_smem(I.vbits));
     static int per_sm_cache[2][17] = {};  // [vbits == 16][threads / 32]
     int &per_sm = per_sm_cache[I.vbits == 16][bt / 32];
     if (per_sm == 0) {

@@ -483,23 +483,26 @@ __device__ __forceinline__ uint64_t intern_leaf(const DevInterner &I, uint32_t v
     return EMPTY_ID;
 }
 
-// Removes a dead node from its table, clears the record, bumps the generation and pushes the slot
-// on the free list (recycle, interner/mod.rs:566-625). `free_pos` is the free-list position.
-__device__ __forceinline__ void recycle_node(const DevInterner &I, uint32_t idx, unsigned long long free_pos) {
-    uint64_t id = I.ids[idx];
+// Removes a dead node (id: its BlockId, h: its fingerprint, gen: its generation) from its table, clears the
+// record, bumps the generation and puts the slot on the free list at `free_pos` (recycle,
+// interner/mod.rs:566-625). A branch's table slot always becomes a tombstone: freeing it where the next
+// slot is EMPTY leaves fewer of them, but the ones that stay then sit in runs that end in a live key,
+// every insert that hashes into a run lengthens it, and the rebuild that would end it comes late (edits of
+// a 512^3 tree: 1.4 ms an apply growing to 6 ms over 150 applies).
+__device__ __forceinline__ void recycle_node(const DevInterner &I, uint32_t idx, uint64_t id, uint64_t h, uint32_t gen,
+                                             unsigned long long free_pos) {
     if (id_is_leaf(id)) {
         uint32_t v = node_value(I, idx);
         atomicCAS((unsigned long long *)(I.leaf_table + v), id, 0ull);
     } else {
-        uint64_t h = I.hash[idx];
-        uint32_t tag = slot_tag(h);
+        const uint64_t slot = make_slot(slot_tag(h), idx);
         uint64_t pos = h & I.table_mask;
         bool removed = false;
         for (uint32_t p = 0; p <= I.max_probes; ++p) {
-            uint64_t s = ld_volatile(I.table + pos);
+            const uint64_t s = ld_volatile(I.table + pos);
             if (s == SLOT_EMPTY) break;
-            if (s == make_slot(tag, idx)) {
-                atomicExch((unsigned long long *)(I.table + pos), SLOT_TOMB);
+            if (s == slot) {  // nothing else writes a published slot while nodes are released
+                *(volatile uint64_t *)(I.table + pos) = SLOT_TOMB;
                 removed = true;
                 break;
             }
@@ -513,9 +516,7 @@ __device__ __forceinline__ void recycle_node(const DevInterner &I, uint32_t idx,
     I.hash[idx] = 0;
     I.refcount[idx] = 0;
     I.ids[idx] = 0;
-    uint32_t g = (uint32_t)I.generation[idx] + 1u;
-    if (g >= MAX_GENERATION) g = 0;
-    I.generation[idx] = (uint16_t)g;
+    I.generation[idx] = (uint16_t)(gen + 1u >= MAX_GENERATION ? 0u : gen + 1u);
     I.free_list[free_pos] = idx;
 }
 
@@ -604,36 +605,111 @@ __device__ __forceinline__ void release_roots_range(const DevInterner &I, const 
     }
 }
 
+// Per-CTA counts of the references that leaves lose in a release round (shared memory,
+// release_smem bytes): direct-mapped by node index with the owner as a tag; a leaf whose slot another
+// one owns goes straight to its global count. A few leaves are children of most bottom groups: one
+// returning atomic for each of their references serialised at those few addresses (4.5 ms for the
+// release of 3.2 M nodes with their 25 M child references).
+struct LeafDrops {
+    uint32_t *key;  // node index + 1, 0 = free
+    uint32_t *cnt;
+    uint32_t slots;  // power of two
+};
+inline __host__ __device__ uint32_t release_slots(int vbits) { return vbits == 8 ? 512u : 4096u; }
+inline __host__ __device__ size_t release_smem(int vbits) { return (size_t)release_slots(vbits) * 8; }
+
+// Every thread of the CTA calls it; mem: release_smem bytes no thread still uses.
+__device__ __forceinline__ LeafDrops leaf_drops_init(const DevInterner &I, uint32_t *mem) {
+    LeafDrops D;
+    D.slots = release_slots(I.vbits);
+    D.key = mem;
+    D.cnt = mem + D.slots;
+    for (uint32_t k = threadIdx.x; k < 2 * D.slots; k += blockDim.x) mem[k] = 0;
+    __syncthreads();
+    return D;
+}
+
+// Counts n lost references of leaf idx; false when its slot is taken (the caller goes to the global count).
+__device__ __forceinline__ bool leaf_drop(const LeafDrops &D, uint32_t idx, uint32_t n) {
+    const uint32_t s = (idx * 0x9E3779B1u) >> 8 & (D.slots - 1u), key = idx + 1u;
+    uint32_t t = *(volatile uint32_t *)(D.key + s);
+    if (t == 0) {
+        t = atomicCAS(D.key + s, 0u, key);
+        if (t == 0) t = key;
+    }
+    if (t != key) return false;
+    atomicAdd(D.cnt + s, n);
+    return true;
+}
+
+// Takes n references from node idx; true when none is left. More than it has is the reference's
+// underflow: the count stays at zero and the error is recorded.
+__device__ __forceinline__ bool drop_refs(const DevInterner &I, uint32_t idx, uint32_t n, uint32_t old) {
+    if (old < n) {
+        atomicAdd(I.refcount + idx, n - old);
+        set_error(I, ERR_REF_UB, 61);
+    }
+    return old == n;
+}
+
 // Retires the *n_in dying nodes of `in`: their children lose one reference each (children reaching
-// zero are the next dying set, appended to `out` and counted in *n_out) and the nodes are recycled.
-__device__ __forceinline__ void release_round_range(const DevInterner &I, const uint32_t *in, uint32_t *out,
-                                                    const unsigned long long *n_in, unsigned long long *n_out,
-                                                    uint64_t cta_base, uint64_t stride) {
+// zero are the next dying set, appended to `out` and counted in *n_out) and the nodes are recycled. A thread
+// takes a node; the counts of its branch children are decremented together, those of leaves in D, which
+// the CTA flushes at the end. The whole CTA calls it.
+__device__ __forceinline__ void release_round_range(const DevInterner &I, const LeafDrops &D, const uint32_t *in,
+                                                    uint32_t *out, const unsigned long long *n_in,
+                                                    unsigned long long *n_out, uint64_t cta_base, uint64_t stride) {
     const uint64_t n = *n_in;
     const unsigned lane = threadIdx.x & 31u;
+    if (cta_base >= n) return;
     for (uint64_t base = cta_base; base < n; base += stride) {
         const uint64_t j = base + threadIdx.x;
         const bool in_range = j < n;
         const uint32_t idx = in_range ? in[j] : 0u;
         const uint64_t id = in_range ? I.ids[idx] : 0ull;
-        const bool branch = in_range && id != 0 && id_is_branch(id);
-        for (int k = 0; k < 8; ++k) {
-            bool dies = false;
-            uint32_t cidx = 0;
-            if (branch) {
-                const uint64_t c = I.children[8ull * idx + k];
-                if (c != EMPTY_ID) {
-                    cidx = id_index(c);
-                    const unsigned old = atomicSub(I.refcount + cidx, 1u);
-                    if (old == 0) {
-                        atomicAdd(I.refcount + cidx, 1u);
-                        set_error(I, ERR_REF_UB, 61);
-                    } else {
-                        dies = old == 1;
-                    }
-                }
+        const uint64_t h = in_range ? I.hash[idx] : 0ull;
+        const uint32_t gen = in_range ? I.generation[idx] : 0u;
+        uint64_t c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (id != 0 && id_is_branch(id)) {
+            const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(I.children + 8ull * idx);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const ulonglong2 w = src[k];
+                c[2 * k] = w.x;
+                c[2 * k + 1] = w.y;
             }
-            push_dying(out, n_out, dies, cidx);
+        }
+        uint32_t old[8], cnt[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {  // cnt: references to take now; equal children are taken together
+            cnt[k] = c[k] != EMPTY_ID ? 1u : 0u;
+            old[k] = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (i < k && c[i] == c[k]) cnt[k] = 0;
+                if (i > k && c[i] == c[k] && cnt[k]) ++cnt[k];
+            }
+            if (cnt[k] && id_is_leaf(c[k]) && leaf_drop(D, id_index(c[k]), cnt[k])) cnt[k] = 0;
+            if (cnt[k]) old[k] = atomicSub(I.refcount + id_index(c[k]), cnt[k]);
+        }
+        uint32_t dies = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (cnt[k] && drop_refs(I, id_index(c[k]), cnt[k], old[k])) dies |= 1u << k;
+        if (__any_sync(0xFFFFFFFFu, dies != 0)) {  // one range of the next dying set for the warp
+            const uint32_t mine = __popc(dies);
+            uint32_t incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= (unsigned)o) incl += y;
+            }
+            unsigned long long at = 0;
+            if (lane == 31) at = atomicAdd(n_out, (unsigned long long)incl);
+            at = __shfl_sync(0xFFFFFFFFu, at, 31) + (incl - mine);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if ((dies >> k) & 1u) out[at++] = id_index(c[k]);
         }
         const bool rec = in_range && id != 0;
         if (in_range && id == 0) set_error(I, ERR_INTERNAL, 62);
@@ -644,10 +720,24 @@ __device__ __forceinline__ void release_round_range(const DevInterner &I, const 
             if ((int)lane == leader) fbase = atomicAdd(&I.ctr->free_count, (unsigned long long)__popc(m));
             fbase = __shfl_sync(0xFFFFFFFFu, fbase, leader);
         }
-        const unsigned tomb = __ballot_sync(0xFFFFFFFFu, rec && branch);
+        const unsigned tomb = __ballot_sync(0xFFFFFFFFu, rec && id_is_branch(id));
         if (lane == 0 && tomb) atomicAdd(&I.ctr->tombstones, (unsigned long long)__popc(tomb));
-        if (rec) recycle_node(I, idx, fbase + __popc(m & ((1u << lane) - 1u)));
+        if (rec) recycle_node(I, idx, id, h, gen, fbase + __popc(m & ((1u << lane) - 1u)));
     }
+    __syncthreads();
+    for (uint32_t s = threadIdx.x; s < D.slots; s += blockDim.x) {  // slots: a multiple of the CTA's warps
+        const uint32_t n_ref = D.cnt[s];
+        bool dies = false;
+        uint32_t idx = 0;
+        if (n_ref) {
+            idx = D.key[s] - 1u;
+            dies = drop_refs(I, idx, n_ref, atomicSub(I.refcount + idx, n_ref));
+            D.key[s] = 0;
+            D.cnt[s] = 0;
+        }
+        push_dying(out, n_out, dies, idx);
+    }
+    __syncthreads();
 }
 
 }  // namespace vxg

@@ -79,9 +79,11 @@ __global__ void __launch_bounds__(kThreads) release_roots_kernel(DevInterner I, 
 }
 
 __global__ void __launch_bounds__(kThreads) release_round_kernel(DevInterner I, const uint32_t *in, uint32_t *out) {
+    extern __shared__ uint32_t release_mem[];
+    const LeafDrops D = leaf_drops_init(I, release_mem);
     pdl_wait();
     pdl_release();
-    release_round_range(I, in, out, &I.ctr->scratch[SC_REL_IN], &I.ctr->scratch[SC_REL_OUT],
+    release_round_range(I, D, in, out, &I.ctr->scratch[SC_REL_IN], &I.ctr->scratch[SC_REL_OUT],
                         (uint64_t)blockIdx.x * blockDim.x, (uint64_t)gridDim.x * blockDim.x);
     if (grid_last_cta(&I.ctr->scratch[SC_DONE])) release_advance(I);
 }
@@ -113,10 +115,10 @@ __device__ uint32_t seq_alloc(Seq &S) {
 }
 
 __device__ void seq_recycle(Seq &S, uint32_t idx) {
-    const bool branch = id_is_branch(S.I.ids[idx]);
-    recycle_node(S.I, idx, S.I.ctr->free_count);
+    const uint64_t id = S.I.ids[idx];
+    recycle_node(S.I, idx, id, S.I.hash[idx], S.I.generation[idx], S.I.ctr->free_count);
     S.I.ctr->free_count += 1;
-    if (branch) S.I.ctr->tombstones += 1;
+    if (id_is_branch(id)) S.I.ctr->tombstones += 1;
 }
 
 __device__ bool seq_valid(Seq &S, uint64_t id) {
@@ -1622,7 +1624,7 @@ cudaError_t launch_release(const DevInterner &I, uint64_t *list, uint32_t *front
     uint32_t *in = frontier_a, *out = frontier_b;
     for (int r = 0; r < rounds; ++r) {  // each kernel's last CTA advances the dying set
         count_launches(1);
-        (void)launch_pdl(release_round_kernel, dim3(g), dim3(kThreads), 0, s, I, in, out);
+        (void)launch_pdl(release_round_kernel, dim3(g), dim3(kThreads), release_smem(I.vbits), s, I, in, out);
         uint32_t *t = in;
         in = out;
         out = t;
