@@ -2188,7 +2188,7 @@ __global__ void __launch_bounds__(kThreads) epoch_refcount_kernel(DevInterner I)
     else
         for (unsigned k = threadIdx.x; k < kLeafTab; k += blockDim.x) tab_key[k] = 0, tab_cnt[k] = 0;
     __syncthreads();
-    const unsigned long long n = I.ctr->alloc_count;
+    const unsigned long long n = I.ctr->alloc_count & kTicketMask;
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
     for (unsigned long long t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += stride) {
         const uint32_t idx = node_for_ticket(I, t);

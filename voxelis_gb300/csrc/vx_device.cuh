@@ -55,10 +55,15 @@ constexpr uint8_t TREE_UNUSED = 0xFF;  // depth marker of a free tree slot
 constexpr uint32_t SPIN_LIMIT = 1u << 22;   // bounded waits (~tens of ms with nanosleep)
 constexpr uint32_t ROUND_LIMIT = 1u << 20;  // bounded warp-intern rounds
 
+// DevCounters::alloc_count: the epoch's tickets in the low bits, in the others the tombstones its inserts
+// took, so that counting those costs an insert no second atomic on the line every insert goes to.
+constexpr int kTicketBits = 33;  // more than the largest capacity (32 bits) twice over
+constexpr unsigned long long kTicketMask = (1ull << kTicketBits) - 1ull;
+
 struct DevCounters {
     unsigned long long next_index;   // bump pointer
     unsigned long long free_count;   // free-list length
-    unsigned long long alloc_count;  // allocations in the current epoch
+    unsigned long long alloc_count;  // allocations in the current epoch (kTicketBits), reused tombstones above
     unsigned long long tombstones;   // deleted branch-table slots
     unsigned int error;              // sticky ERR_* bits
     unsigned int error_info;         // first error detail
@@ -281,7 +286,8 @@ __device__ __forceinline__ uint32_t node_for_ticket(const DevInterner &I, unsign
 // fresh indices its tickets took become allocated.
 __device__ __forceinline__ void epoch_finalize_body(const DevInterner &I) {
     DevCounters *c = I.ctr;
-    const unsigned long long alloc = c->alloc_count, fc = c->free_count;
+    const unsigned long long alloc = c->alloc_count & kTicketMask, fc = c->free_count;
+    c->tombstones -= c->alloc_count >> kTicketBits;
     const unsigned long long used_free = alloc < fc ? alloc : fc;
     c->free_count = fc - used_free;
     unsigned long long ni = c->next_index + (alloc - used_free);
@@ -342,6 +348,12 @@ __device__ __forceinline__ bool key_equal(const DevInterner &I, uint32_t idx, co
 // one non-blocking probe step; lanes that claimed an empty slot receive node indices from a single
 // warp-aggregated ticket range, write their node and publish it. A lane that meets a slot still being
 // written retries it next round, so no lane ever waits inside a divergent branch.
+// A new key takes the first tombstone of its probe sequence, once the sequence has reached an EMPTY slot
+// without meeting the key. Slots only go from EMPTY or tombstone to a key while nodes are created, so two
+// lanes with one key agree on the slot or one of them loses the compare-and-swap, and a loser goes on from
+// the slot it lost. Edits that come and go recreate the same keys (the bottom groups of a fill and its
+// undo): without reuse each left one more tombstone for its next insert to walk over, and 4096 edits of a
+// 512^3 tree and their undo grew from 1.9 to 8.0 ms a pass before the table was rebuilt.
 // Returns the BlockId; *created tells whether this lane inserted the node. On failure (probe limit,
 // round limit, out of nodes: a sticky error bit is set) the lane gets EMPTY_ID, which every consumer
 // handles without dereferencing it, so a failed call leaves wrong but memory-safe results until
@@ -358,6 +370,7 @@ __device__ __forceinline__ uint64_t warp_intern_branch_inl(const DevInterner &I,
     uint32_t tag = 0;
     uint64_t pos = 0;
     uint32_t probes = 0;
+    uint32_t tomb = 0;  // 1 + probes before the first tombstone met, 0: none
     bool done = !active;
     uint64_t result = EMPTY_ID;
     *created = false;
@@ -373,12 +386,20 @@ __device__ __forceinline__ uint64_t warp_intern_branch_inl(const DevInterner &I,
         bool waiting = false;
         if (!done) {
             uint64_t s = ld_probe(I.table + pos);
+            if (s == SLOT_TOMB && tomb == 0) tomb = probes + 1;
             if (s == SLOT_EMPTY) {
-                uint64_t prev = atomicCAS((unsigned long long *)(I.table + pos), SLOT_EMPTY, make_slot(tag, IDX_BUSY));
-                if (prev == SLOT_EMPTY)
+                if (tomb) {
+                    probes = tomb - 1;
+                    pos = (h + probes) & I.table_mask;
+                }
+                const uint64_t free_slot = tomb ? SLOT_TOMB : SLOT_EMPTY;
+                uint64_t prev = atomicCAS((unsigned long long *)(I.table + pos), free_slot, make_slot(tag, IDX_BUSY));
+                if (prev == free_slot) {
                     claimed = true;
-                else
+                } else {
                     s = prev;
+                    tomb = 0;
+                }
             }
             if (!claimed) {
                 if ((uint32_t)(s >> 32) == tag && s != SLOT_TOMB) {
@@ -407,14 +428,18 @@ __device__ __forceinline__ uint64_t warp_intern_branch_inl(const DevInterner &I,
         if (cm) {
             unsigned long long base = 0;
             const int leader = __ffs(cm) - 1;
-            if ((int)lane == leader) base = atomicAdd(&I.ctr->alloc_count, (unsigned long long)__popc(cm));
-            base = __shfl_sync(0xFFFFFFFFu, base, leader);
+            const unsigned reused = __ballot_sync(0xFFFFFFFFu, claimed && tomb != 0);
+            if ((int)lane == leader)
+                base = atomicAdd(&I.ctr->alloc_count,
+                                 (unsigned long long)__popc(cm) | ((unsigned long long)__popc(reused) << kTicketBits));
+            base = __shfl_sync(0xFFFFFFFFu, base & kTicketMask, leader);
             if (claimed) {
                 const unsigned rank = __popc(cm & ((1u << lane) - 1u));
                 const uint32_t idx = node_for_ticket(I, base + rank, fc, ni);
                 if (idx == NO_NODE) {
                     set_error(I, ERR_OOM, 1);
                     atomicExch((unsigned long long *)(I.table + pos), SLOT_TOMB);
+                    if (tomb) atomicAdd(&I.ctr->tombstones, 1ull);
                 } else {
                     result = write_branch(I, idx, c, types, mask, h, lod, base + rank >= fc);
                     publish_release((unsigned long long *)(I.table + pos), make_slot(tag, idx));
@@ -457,7 +482,7 @@ __device__ __forceinline__ uint64_t intern_leaf(const DevInterner &I, uint32_t v
         if (s == 0) {  // free (or its creator ran out of memory and backed off): claim it
             const uint64_t prev = atomicCAS(slot, 0ull, LEAF_BUSY);
             if (prev == 0) {
-                const unsigned long long t = atomicAdd(&I.ctr->alloc_count, 1ull);
+                const unsigned long long t = atomicAdd(&I.ctr->alloc_count, 1ull) & kTicketMask;
                 const uint32_t idx = node_for_ticket(I, t, fc, ni);
                 if (idx == NO_NODE) {
                     set_error(I, ERR_OOM, 2);

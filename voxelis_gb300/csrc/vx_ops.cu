@@ -160,12 +160,17 @@ __device__ uint64_t seq_branch(Seq &S, const uint64_t c[8], uint32_t types, uint
     const DevInterner &I = S.I;
     const uint64_t h = branch_fingerprint(c, (types << 8) | mask);
     const uint32_t tag = slot_tag(h);
-    uint64_t pos = h & I.table_mask;
+    uint64_t pos = h & I.table_mask, tomb = ~0ull;  // the first tombstone met takes a new key
     for (uint32_t p = 0; p <= I.max_probes; ++p, pos = (pos + 1) & I.table_mask) {
         const uint64_t s = I.table[pos];
+        if (s == SLOT_TOMB && tomb == ~0ull) tomb = pos;
         if (s == SLOT_EMPTY) {
             const uint32_t idx = seq_alloc(S);
             if (idx == NO_NODE) return INVALID_ID;
+            if (tomb != ~0ull) {
+                pos = tomb;
+                I.ctr->tombstones -= 1;
+            }
             uint32_t cv[8];
             for (int k = 0; k < 8; ++k) cv[k] = node_value(I, id_index(c[k]));
             const uint64_t id = write_branch(I, idx, c, types, mask, h, calc_average8(cv));
