@@ -1,19 +1,24 @@
 // Batched VoxTree::apply_batch over many trees sharing one interner, level-synchronous on the GPU.
 //
 // Restates set_batch_at_depth_iterative (spatial/voxtree.rs:724-1118) for n trees at once:
+//   plan     the levels' structure from the sorted records alone. A record heads a sibling run at step s
+//            (the parents s levels above the bottom groups) when its group differs from the one before it
+//            above the 3 s low bits, or it starts an item; counting the records that head each step
+//            gives every parent of every level its number, its first child and its first record at once.
 //   prep     Phase 0 fill (voxtree.rs:742-758): the fill leaf replaces the old root as the
 //            starting node; without patches it is the new root.
 //   bottom   Phase 1 (voxtree.rs:770-897), one thread per touched bottom group: descend the old
 //            tree to depth d-1, collapse a full uniform group to a leaf, otherwise merge the set
 //            voxels into the existing children (or into 8 copies of an ancestor leaf) and
-//            hash-cons the branch. Groups that change nothing drop out, as in the reference.
-//   levels   Phase 2 (voxtree.rs:905-1106), one step per level for all trees together: entries
-//            are kept sorted by (tree, path), so the siblings of one parent form a run; run heads
-//            are found by comparing sibling prefixes (PATH_MASKS), numbered by a prefix scan,
-//            and each parent gathers its run, clones the untouched children of the old parent or
-//            replicates an ancestor leaf, collapses 8 equal leaves, and hash-conses the result.
-//   finish   apply_batch (voxtree.rs:303-328): commit the new root, queue the old root for
-//            release, report assert_ne!(new_root, old_root) as a reference panic.
+//            hash-cons the branch. The record that heads a parent passes the old node at the parent's
+//            place on its descent and leaves it there for the level passes. Groups that change nothing
+//            are marked, as the reference drops them.
+//   levels   Phase 2 (voxtree.rs:905-1106), one step per level for all trees together: each parent
+//            gathers its run's changed children, clones the untouched children of the old parent or
+//            replicates an ancestor leaf, collapses 8 equal leaves, and hash-conses the result; a parent
+//            none of whose children changed is marked unchanged.
+//   finish   apply_batch (voxtree.rs:303-328), by the thread that makes an item's root: commit it,
+//            queue the old root for release, report assert_ne!(new_root, old_root) as a reference panic.
 // Clear pass (P4). The reference ignores Batch clear bits (voxtree.rs:779). With P4 they are
 // honoured as VoxTree::set(pos, 0) for every cleared voxel after the set phase (remove_at_depth,
 // voxtree.rs:542-706). Those removals commute, so the same level-synchronous machinery applies them
@@ -23,14 +28,14 @@
 // EMPTY from its mask, and becomes EMPTY itself when its mask empties. Nothing collapses. The
 // removal path is refcount-exact, so no correction applies.
 // Trees are processed deepest first, so the trees whose root is produced at a step are the tail
-// of that step's list and the next list is a prefix of the parents.
+// of that step's list, and a parent's number at a step is its number among the records that head it.
 //
 // Refcounts. After the build every count is the in-degree from newly created nodes plus tree roots,
 // plus the corrections below. The lane that creates a branch adds its children's references right
 // away, from the key it still holds in registers (no re-read of the node): branch children by a
 // global reduction, leaf children into a per-CTA table indexed by leaf value that the CTA flushes
-// once (leaves are the hot spots: a few values are named by most bottom groups). The last CTA of
-// the root-commit kernel closes the allocation epoch. The corrections reproduce where the
+// once (leaves are the hot spots: a few values are named by most bottom groups). The allocation epoch is
+// closed once the last level is done. The corrections reproduce where the
 // reference's increments differ from the references its nodes hold:
 //   Q5 (voxtree.rs:835-839, 846-868): an ancestor leaf is charged 8 - |set| references, but only
 //      8 - |modified| slots keep it: + (|modified| - |set|), or + (8 - |set|) when nothing changed.
@@ -51,9 +56,6 @@ constexpr int kThreads = 256;
 #ifndef VX_APPLY_MIN_BLOCKS
 #define VX_APPLY_MIN_BLOCKS 2
 #endif
-constexpr int kScanPer = 8;
-constexpr int kScanBlock = kThreads * kScanPer;
-
 __device__ __forceinline__ void add_ref_delta(const DevInterner &I, uint64_t id, int delta) {
     if (delta != 0 && id != EMPTY_ID) atomicAdd(I.refcount + id_index(id), (unsigned)delta);
 }
@@ -135,18 +137,39 @@ __device__ __forceinline__ void leaf_refs_flush(const DevInterner &I, const Leaf
     }
 }
 
-__device__ __forceinline__ void prep_item(const DevInterner &I, const ApplyArgs &a, int mode, uint32_t i) {
+// ---- items ---------------------------------------------------------------------------------------
+// Depth of item i: given by the host, or (check_depths) read from the tree table with the checks of a
+// device-resident call, an item that fails them counting as a tree of depth 2.
+__device__ __forceinline__ int item_depth_of(const DevInterner &I, const ApplyArgs &a, uint32_t i, bool check_depths,
+                                             bool *bad = nullptr) {
+    if (!check_depths) return a.it_depth[i];
     const uint32_t t = a.it_tree[i];
-    const uint64_t old = I.roots[t];
+    const int d = t < I.tree_cap ? I.depths[t] : TREE_UNUSED;
+    int prev = 0xFF;
+    if (i > 0) {
+        const uint32_t tp = a.it_tree[i - 1];
+        prev = tp < I.tree_cap ? I.depths[tp] : TREE_UNUSED;
+    }
+    if (d == TREE_UNUSED || d > a.max_depth || d < 2 || (i > 0 && d > prev)) {
+        if (bad) *bad = true;
+        return 2;
+    }
+    return d;
+}
+
+__device__ __forceinline__ uint64_t item_root(const DevInterner &I, const ApplyArgs &a, uint32_t i) {
+    const uint32_t t = a.it_tree[i];
+    return t < I.tree_cap ? I.roots[t] : EMPTY_ID;
+}
+
+// Phase 0 of item i (set phase).
+__device__ __forceinline__ void prep_item(const DevInterner &I, const ApplyArgs &a, uint32_t i) {
+    const uint64_t old = item_root(I, a, i);
     const uint8_t f = a.it_flags[i];
     uint64_t init = old;
     a.it_old[i] = old;
-    if (mode == 1) {  // the clear pass starts from the root the set phase left
-        a.it_init[i] = old;
-        a.it_new[i] = INVALID_ID;
-        return;
-    }
     a.it_panic[i] = 0;
+    a.it_changed[i] = 0;
     if (f & 1) {
         bool created;
         const uint64_t fill = intern_leaf(I, a.it_fill[i], &created);
@@ -154,53 +177,199 @@ __device__ __forceinline__ void prep_item(const DevInterner &I, const ApplyArgs 
         if (f & 2) add_ref_delta(I, fill, 1);  // Q7
     }
     a.it_init[i] = init;
-    a.it_new[i] = (f & 2) ? INVALID_ID : init;
 }
 
-__global__ void prep_items_kernel(DevInterner I, ApplyArgs a) {
-    pdl_wait();
-    pdl_release();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < a.n_items) prep_item(I, a, a.mode, i);
+// The root of item i is nw (mode 0: the set phase, voxtree.rs:303-328; mode 1: the clear pass).
+__device__ __forceinline__ void finish_item(const DevInterner &I, const ApplyArgs &a, int mode, uint32_t i, uint64_t nw) {
+    const uint32_t t = a.it_tree[i];
+    if (t >= I.tree_cap) return;
+    uint64_t old;
+    if (mode == 1) {
+        old = I.roots[t];
+        if (nw != EMPTY_ID) atomicAdd(I.refcount + id_index(nw), 1u);
+    } else {
+        if (a.it_panic[i]) return;
+        old = a.it_old[i];
+        if ((a.it_flags[i] & 3) && nw != EMPTY_ID) atomicAdd(I.refcount + id_index(nw), 1u);  // the tree's root reference
+        if (old != EMPTY_ID && nw == old && !(I.flags & (1u << 4))) {  // assert_ne!(new_root_id, self.root_id) (voxtree.rs:311)
+            set_error(I, ERR_REF_PANIC, 41);
+            return;
+        }
+    }
+    if (old != EMPTY_ID) {
+        const unsigned long long e = atomicAdd(&I.ctr->scratch[SC_RELEASE], 1ull);
+        a.release_list[e] = old;
+    }
+    I.roots[t] = nw;
+    a.it_changed[i] = 1;
 }
 
-// Phase 1 for records cta_base + threadIdx.x, + stride, ... (a CTA-uniform loop: whole warps take
-// part in the warp-cooperative interning).
-__device__ __forceinline__ void bottom_range(const DevInterner &I, const ApplyArgs &a, int mode, const LeafRefs &L,
-                                             uint64_t cta_base, uint64_t stride) {
-    for (uint64_t base = cta_base; base < a.n_records; base += stride) {
-        const uint64_t r = base + threadIdx.x;
-        bool active = r < a.n_records;
-        uint32_t i = 0, set = 0, changed = 0;
-        int d = 0;
+// ---- the plan of the levels ------------------------------------------------------------------------
+// Records are taken in tiles of 32 (one warp). The CTAs of the grid own contiguous ranges of tiles, their
+// warps contiguous parts of a range. Word 0 of a count is the records with clear bits, word s the records
+// that head step s; lane s of a warp keeps word s.
+struct Tiles {
+    uint32_t lo, hi;  // this warp's tiles
+    uint32_t woff;    // its place in ApplyArgs::warp_off
+};
+__device__ __forceinline__ Tiles warp_tiles(const ApplyArgs &a) {
+    const uint32_t nw = blockDim.x >> 5, warp = threadIdx.x >> 5;
+    const uint32_t total = (uint32_t)(((uint64_t)a.n_records + 31) / 32);
+    const uint32_t per_cta = (total + gridDim.x - 1) / gridDim.x, per_warp = (per_cta + nw - 1) / nw;
+    const uint64_t c0 = (uint64_t)blockIdx.x * per_cta, c1 = c0 + per_cta < total ? c0 + per_cta : total;
+    const uint64_t w0 = c0 + (uint64_t)warp * per_warp, w1 = w0 + per_warp < c1 ? w0 + per_warp : c1;
+    Tiles t;
+    t.lo = (uint32_t)(w0 < w1 ? w0 : 0);
+    t.hi = (uint32_t)(w0 < w1 ? w1 : 0);
+    t.woff = (blockIdx.x * nw + warp) * kPlanWords;
+    return t;
+}
+
+// Steps that record r (of item i and group g, depth d) heads: 1 .. the result. Whole warp, lanes in order.
+__device__ __forceinline__ uint32_t head_steps(const ApplyArgs &a, uint64_t r, bool in, uint32_t i, uint32_t g, int d) {
+    uint32_t ip = __shfl_up_sync(0xFFFFFFFFu, i, 1), gp = __shfl_up_sync(0xFFFFFFFFu, g, 1);
+    if (!in) return 0;
+    const uint32_t top = (uint32_t)d - 1u;
+    if (r == 0) return top;
+    if ((threadIdx.x & 31u) == 0) {
+        ip = a.rec_item[r - 1];
+        gp = a.rec_group[r - 1];
+    }
+    if (ip != i) return top;
+    const uint32_t x = g ^ gp, s = x ? (31u - __clz(x)) / 3u : 0u;
+    return s < top ? s : top;
+}
+
+// Counts of this CTA's range (all threads of the CTA call it; cnt_s: kPlanWords words a warp).
+__device__ __forceinline__ void plan_count(const DevInterner &I, const ApplyArgs &a, bool check_depths,
+                                           uint32_t (*cnt_s)[kPlanWords]) {
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const Tiles t = warp_tiles(a);
+    uint32_t acc = 0;  // word `lane`, over this warp's tiles so far
+    for (uint32_t tile = t.lo; tile < t.hi; ++tile) {
+        const uint64_t r = 32ull * tile + lane;
+        const bool in = r < a.n_records;
+        const uint32_t i = in ? a.rec_item[r] : 0u, g = in ? a.rec_group[r] : 0u;
+        const int d = in ? item_depth_of(I, a, i, check_depths) : 2;
+        const uint32_t hs = head_steps(a, r, in, i, g, d);
+        if (lane < kPlanWords) a.tile_base[(uint64_t)tile * kPlanWords + lane] = acc;
+        const unsigned cl = __ballot_sync(0xFFFFFFFFu, in && a.rec_clear[r] != 0);
+        if (lane == 0) acc += __popc(cl);
+        const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, hs);
+        for (uint32_t s = 1; s <= top; ++s) {
+            const unsigned b = __ballot_sync(0xFFFFFFFFu, hs >= s);
+            if (lane == s) acc += __popc(b);
+        }
+    }
+    if (lane < kPlanWords) cnt_s[warp][lane] = acc;
+    __syncthreads();
+    if (threadIdx.x < kPlanWords) {  // the warps' places in the range, and its sums
+        uint32_t run = 0;
+        for (uint32_t w = 0; w < nw; ++w) {
+            a.warp_off[(blockIdx.x * nw + w) * kPlanWords + threadIdx.x] = run;
+            run += cnt_s[w][threadIdx.x];
+        }
+        a.part[threadIdx.x * gridDim.x + blockIdx.x] = run;
+    }
+    __syncthreads();
+}
+
+struct Plan {
+    uint32_t base[kPlanWords];   // counts of the ranges before this CTA's
+    uint32_t total[kPlanWords];  // counts of all ranges, no more than a step's room
+};
+
+// After every CTA's plan_count. All threads of the CTA call it.
+__device__ __forceinline__ void plan_totals(const ApplyArgs &a, Plan &P) {
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (uint32_t s = warp; s < kPlanWords; s += nw) {
+        uint32_t before = 0, all = 0;
+        for (uint32_t c = lane; c < gridDim.x; c += 32) {
+            const uint32_t v = a.part[s * gridDim.x + c];
+            all += v;
+            if (c < blockIdx.x) before += v;
+        }
+        before = __reduce_add_sync(0xFFFFFFFFu, before);
+        all = __reduce_add_sync(0xFFFFFFFFu, all);
+        if (lane == 0) {
+            P.base[s] = before;
+            P.total[s] = s > 0 && all > a.p_cap[s] ? a.p_cap[s] : all;
+        }
+    }
+    __syncthreads();
+}
+
+// ---- Phase 1 -----------------------------------------------------------------------------------------
+// An entry's value word: LOD value, the slot among its siblings, and whether it changed.
+constexpr uint32_t kChanged = 1u << 31;
+__device__ __forceinline__ uint32_t entry_word(uint32_t value, uint32_t path, bool changed) {
+    return value | ((path & 7u) << 16) | (changed ? kChanged : 0u);
+}
+
+// The records of this warp's tiles. In the set phase it also writes the parents' first children and
+// records; in both the old node at each parent's place.
+__device__ __forceinline__ void bottom_records(const DevInterner &I, const ApplyArgs &a, int mode, const LeafRefs &L,
+                                               const Plan &P) {
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned lt = (1u << lane) - 1u;
+    const Tiles tiles = warp_tiles(a);
+    const uint32_t at_warp = (lane < kPlanWords && tiles.lo < tiles.hi) ? P.base[lane] + a.warp_off[tiles.woff + lane] : 0u;
+    for (uint32_t tile = tiles.lo; tile < tiles.hi; ++tile) {
+        const uint64_t r = 32ull * tile + lane;
+        const bool in = r < a.n_records;
+        const uint32_t i = in ? a.rec_item[r] : 0u, g = in ? a.rec_group[r] : 0u;
+        const int d = in ? a.it_depth[i] : 2;
+        const uint32_t hs = head_steps(a, r, in, i, g, d);
+        const uint32_t at = lane < kPlanWords ? at_warp + a.tile_base[(uint64_t)tile * kPlanWords + lane] : 0u;
+        bool active = in;
+        uint32_t set = 0, changed = 0;
         uint64_t cur = EMPTY_ID, anc = EMPTY_ID, out = EMPTY_ID;
         uint32_t v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         uint64_t c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         uint32_t cv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         uint32_t types = 0, mask = 0, lod = 0;
         bool want_branch = false;
-        if (active) {
-            i = a.rec_item[r];
-            d = a.it_depth[i];
+        if (in) {
             set = mode ? a.rec_clear[r] : a.rec_set[r];
             if (set == 0 || a.it_panic[i]) active = false;
         }
-        bool uniform = false;
-        if (active) {
-            const uint32_t path = a.rec_group[r] << 3;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = a.rec_vals[8 * r + k];
-            // descend to depth d-1 (voxtree.rs:792-822)
-            cur = a.it_init[i];
-            for (int cd = 0; cd < d - 1; ++cd) {
+        if (active || hs) cur = mode ? item_root(I, a, i) : a.it_init[i];
+        // descend to depth d-1 (voxtree.rs:792-822); at step s the node is the old one of the parent there
+        const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, in ? (uint32_t)d - 1u : 0u);
+        uint32_t above = 0;  // this record's number at step s + 1, when it heads it
+        for (uint32_t s = top; s >= 1; --s) {
+            const unsigned b = __ballot_sync(0xFFFFFFFFu, hs >= s);
+            const uint32_t p = __shfl_sync(0xFFFFFFFFu, at, s) + __popc(b & lt);
+            if (hs > s && mode == 0 && above < a.p_cap[s + 1]) a.p_start[s + 1][above] = p;
+            if (hs >= s) {
+                if (p < a.p_cap[s]) {
+                    a.p_old[s][p] = anc != EMPTY_ID ? anc : cur;
+                    if (mode == 0) a.p_rec[s][p] = (uint32_t)r;
+                } else {
+                    set_error(I, ERR_INVALID, 47);  // records that are not sorted by (item, group)
+                }
+                above = p;
+            }
+            if (s < (uint32_t)d && cur != EMPTY_ID) {
                 if (id_is_branch(cur)) {
-                    const uint32_t idx = (path >> (3 * (d - cd - 1))) & 7u;
-                    cur = I.children[8ull * id_index(cur) + idx];
+                    cur = I.children[8ull * id_index(cur) + ((g >> (3 * (s - 1))) & 7u)];
                 } else {
                     anc = cur;
                     cur = EMPTY_ID;
                 }
-                if (cur == EMPTY_ID) break;
+            }
+        }
+        if (hs && mode == 0 && above < a.p_cap[1]) a.p_start[1][above] = (uint32_t)r;
+        bool uniform = false;
+        if (active) {
+            if ((reinterpret_cast<uintptr_t>(a.rec_vals) & 15u) == 0) {
+                const uint4 w = reinterpret_cast<const uint4 *>(a.rec_vals)[r];
+                const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = (ws[k >> 1] >> (16 * (k & 1))) & 0xFFFFu;
+            } else {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = a.rec_vals[8 * r + k];
             }
             uniform = set == 0xFF;
 #pragma unroll
@@ -312,351 +481,62 @@ __device__ __forceinline__ void bottom_range(const DevInterner &I, const ApplyAr
         const uint64_t id = warp_intern_branch_inl(I, want_branch, c, types, mask, lod, &created);
         if (created) add_child_refs(I, L, c, cv);
         if (want_branch) out = id;
-        if (r < a.n_records) {
-            a.flags[r] = changed;
+        if (in) {
             a.rec_id[r] = out;
-            a.rec_val[r] = lod;
+            a.rec_val[r] = entry_word(lod, g, changed != 0);
         }
     }
 }
 
-__global__ void __launch_bounds__(512, VX_APPLY_MIN_BLOCKS) bottom_kernel(DevInterner I, ApplyArgs a) {
-    pdl_wait();
-    pdl_release();
-    const LeafRefs L = leaf_refs_init(I);
-    bottom_range(I, a, a.mode, L, (uint64_t)blockIdx.x * blockDim.x, (uint64_t)gridDim.x * blockDim.x);
-    leaf_refs_flush(I, L);
-}
-
-// Exclusive scan of n flags: per-block scan, scan of block sums, add-back. pos[n] = total.
-__global__ void __launch_bounds__(kThreads) scan_blocks_kernel(const uint32_t *in, uint32_t *out, uint32_t *sums,
-                                                              uint32_t n) {
-    pdl_wait();
-    pdl_release();
-    __shared__ uint32_t warp_tot[kThreads / 32];
-    const uint32_t base = blockIdx.x * kScanBlock + threadIdx.x * kScanPer;
-    uint32_t x[kScanPer];
-    uint32_t local = 0;
-#pragma unroll
-    for (int k = 0; k < kScanPer; ++k) {
-        x[k] = (base + k < n) ? in[base + k] : 0u;
-        local += x[k];
-    }
-    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t incl = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= (unsigned)o) incl += y;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < kThreads / 32 ? warp_tot[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xFFFFFFFFu, w, o);
-            if (lane >= (unsigned)o) w += y;
-        }
-        if (lane < kThreads / 32) warp_tot[lane] = w;
-    }
-    __syncthreads();
-    uint32_t run = incl - local + (warp ? warp_tot[warp - 1] : 0);
-#pragma unroll
-    for (int k = 0; k < kScanPer; ++k) {
-        if (base + k < n) out[base + k] = run;
-        run += x[k];
-    }
-    if (threadIdx.x == kThreads - 1) sums[blockIdx.x] = warp_tot[kThreads / 32 - 1];
-}
-
-// Variants reading the element count from device memory (entries of a level pass); blocks past the
-// count only record an empty block sum.
-__global__ void __launch_bounds__(kThreads) scan_blocks_dev_kernel(const uint32_t *in, uint32_t *out, uint32_t *sums,
-                                                                  const unsigned long long *n_dev) {
-    pdl_wait();
-    pdl_release();
-    const uint32_t n = (uint32_t)*n_dev;
-    if (blockIdx.x * kScanBlock >= n) {
-        if (threadIdx.x == 0) sums[blockIdx.x] = 0;
-        return;
-    }
-    __shared__ uint32_t warp_tot[kThreads / 32];
-    const uint32_t base = blockIdx.x * kScanBlock + threadIdx.x * kScanPer;
-    uint32_t x[kScanPer];
-    uint32_t local = 0;
-#pragma unroll
-    for (int k = 0; k < kScanPer; ++k) {
-        x[k] = (base + k < n) ? in[base + k] : 0u;
-        local += x[k];
-    }
-    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t incl = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= (unsigned)o) incl += y;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < kThreads / 32 ? warp_tot[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xFFFFFFFFu, w, o);
-            if (lane >= (unsigned)o) w += y;
-        }
-        if (lane < kThreads / 32) warp_tot[lane] = w;
-    }
-    __syncthreads();
-    uint32_t run = incl - local + (warp ? warp_tot[warp - 1] : 0);
-#pragma unroll
-    for (int k = 0; k < kScanPer; ++k) {
-        if (base + k < n) out[base + k] = run;
-        run += x[k];
-    }
-    if (threadIdx.x == kThreads - 1) sums[blockIdx.x] = warp_tot[kThreads / 32 - 1];
-}
-
-// One-pass exclusive scan of the first n = *n_dev flags (decoupled look-back): out[i] = sum of
-// in[0..i), out[n] = the total. CTAs take tiles of kScanBlock elements in launch order from a ticket
-// counter, publish their tile sum (state 1) at once and their inclusive prefix (state 2) as soon as
-// they know it; a tile's prefix is found by walking back over earlier tiles' status words until one
-// holds an inclusive prefix. A CTA only waits on tiles whose tickets were taken earlier, by CTAs
-// that are therefore running or done, and the walk is bounded (ERR_TIMEOUT). Every scan starts with
-// all status words at state 0: the last CTA to finish (all look-back walks are over by then) clears
-// the words this scan used, so the state lives on the device alone and a scan replayed from a CUDA
-// graph behaves as one launched directly. The CTA with the last ticket resets the ticket counter.
-__global__ void __launch_bounds__(kThreads) scan_onepass_dev_kernel(DevInterner I, const uint32_t *in, uint32_t *out,
-                                                                   unsigned long long *status,
-                                                                   const unsigned long long *n_dev) {
-    pdl_wait();
-    pdl_release();
-    __shared__ uint32_t tile_s, prefix_s;
-    __shared__ uint32_t warp_tot[kThreads / 32];
-    unsigned long long *ticket = &I.ctr->scratch[SC_SCAN_TICKET];
-    if (threadIdx.x == 0) {
-        tile_s = (uint32_t)atomicAdd(ticket, 1ull);
-        if (tile_s == gridDim.x - 1) *ticket = 0;  // every ticket is taken: ready for the next scan
-    }
-    __syncthreads();
-    const uint32_t tile = tile_s;
-    const uint32_t n = (uint32_t)*n_dev;
-    const uint32_t base = tile * kScanBlock + threadIdx.x * kScanPer;
-    uint32_t x[kScanPer];
-    uint32_t local = 0;
-#pragma unroll
-    for (int k = 0; k < kScanPer; ++k) {
-        x[k] = (base + k < n) ? in[base + k] : 0u;
-        local += x[k];
-    }
-    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t incl = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= (unsigned)o) incl += y;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < kThreads / 32 ? warp_tot[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xFFFFFFFFu, w, o);
-            if (lane >= (unsigned)o) w += y;
-        }
-        if (lane < kThreads / 32) warp_tot[lane] = w;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t agg = warp_tot[kThreads / 32 - 1];
-        uint32_t excl = 0;
-        if (tile > 0) {
-            st_release_u64(status + tile, (1ull << 32) | agg);
-            uint32_t j = tile - 1;
-            for (uint32_t spin = 0;; ++spin) {
-                if (spin >= I.spin_limit) {
-                    set_error(I, ERR_TIMEOUT, 40);
-                    break;
-                }
-                const unsigned long long w = ld_acquire(reinterpret_cast<const uint64_t *>(status + j));
-                const unsigned long long state = (w >> 32) & 3ull;
-                if (state == 0) continue;  // tile j has not published yet
-                excl += (uint32_t)w;
-                if (state == 2ull || j == 0) break;  // an inclusive prefix ends the walk
-                --j;
-            }
-        }
-        st_release_u64(status + tile, (2ull << 32) | (excl + agg));
-        prefix_s = excl;
-    }
-    __syncthreads();
-    uint32_t run = prefix_s + incl - local + (warp ? warp_tot[warp - 1] : 0);
-#pragma unroll
-    for (int k = 0; k < kScanPer; ++k) {
-        if (base + k < n) out[base + k] = run;
-        run += x[k];
-        if (base + k + 1 == n) out[n] = run;  // the total after the last element
-    }
-    if (n == 0 && tile == 0 && threadIdx.x == 0) out[0] = 0;
-    if (grid_last_cta(&I.ctr->scratch[SC_SCAN_DONE]))  // no walk reads a status word any more
-        for (uint32_t t = 0; t < gridDim.x; ++t) status[t] = 0;
-}
-
-__global__ void scan_add_dev_kernel(uint32_t *out, const uint32_t *sums, const unsigned long long *n_dev) {
-    pdl_wait();
-    pdl_release();
-    const uint32_t n = (uint32_t)*n_dev;
-    const uint32_t b = blockIdx.x;
-    if (b == 0 || b * kScanBlock >= n) return;
-    const uint32_t add = sums[b];
-    const uint32_t base = b * kScanBlock;
-    for (uint32_t k = threadIdx.x; k < kScanBlock; k += blockDim.x)
-        if (base + k < n) out[base + k] += add;
-}
-
-__global__ void scan_total_dev_kernel(const uint32_t *in, uint32_t *out, const unsigned long long *n_dev) {
-    pdl_wait();
-    pdl_release();
-    const uint32_t n = (uint32_t)*n_dev;
-    out[n] = n ? out[n - 1] + in[n - 1] : 0u;
-}
-
-__global__ void scan_add_kernel(uint32_t *out, const uint32_t *sums, uint32_t n) {
-    pdl_wait();
-    pdl_release();
-    const uint32_t b = blockIdx.x;
-    if (b == 0) return;
-    const uint32_t add = sums[b];
-    const uint32_t base = b * kScanBlock;
-    for (uint32_t k = threadIdx.x; k < kScanBlock; k += blockDim.x)
-        if (base + k < n) out[base + k] += add;
-}
-
-__global__ void scan_total_kernel(const uint32_t *in, uint32_t *out, uint32_t n) {
-    pdl_wait();
-    pdl_release();
-    out[n] = n ? out[n - 1] + in[n - 1] : 0u;
-}
-
-__device__ __forceinline__ void scatter_record(const ApplyArgs &a, uint32_t r) {
-    if (!a.flags[r]) return;
-    const uint32_t e = a.pos[r];
-    a.e_item[0][e] = a.rec_item[r];
-    a.e_path[0][e] = a.rec_group[r] << 3;
-    a.e_id[0][e] = a.rec_id[r];
-    a.e_val[0][e] = a.rec_val[r];
-}
-
-__global__ void scatter_bottom_kernel(DevInterner I, ApplyArgs a) {
-    pdl_wait();
-    pdl_release();
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r == 0) I.ctr->scratch[SC_ENTRIES] = a.pos[a.n_records];
-    if (r < a.n_records) scatter_record(a, r);
-}
-
-__device__ __forceinline__ uint32_t parent_key_path(uint32_t path, int d, int t) {
-    return t == 1 ? 0u : (path & path_mask(d, t - 2));
-}
-
-// Run heads of a level step: entry j starts a sibling run unless entry j-1 has the same parent.
-__device__ __forceinline__ void head_flag(const ApplyArgs &a, int step, int buf, uint32_t j) {
-    const uint32_t i = a.e_item[buf][j];
-    const int d = a.it_depth[i];
-    const int t = d - step;
-    uint32_t head = 1;
-    if (j > 0) {
-        const uint32_t ip = a.e_item[buf][j - 1];
-        if (ip == i && parent_key_path(a.e_path[buf][j - 1], d, t) == parent_key_path(a.e_path[buf][j], d, t))
-            head = 0;
-    }
-    a.flags[j] = head;
-}
-
-__global__ void heads_kernel(DevInterner I, ApplyArgs a, int step, int buf) {
-    pdl_wait();
-    pdl_release();
-    const uint32_t count = (uint32_t)I.ctr->scratch[SC_ENTRIES];
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x)
-        head_flag(a, step, buf, j);
-}
-
-// After the scan of the head flags: the number of parents and where each one's run starts.
-__device__ __forceinline__ void starts_head(const DevInterner &I, const ApplyArgs &a, uint32_t count) {
-    const uint32_t np = a.pos[count];
-    a.p_start[np] = count;
-    I.ctr->scratch[SC_PARENTS] = np;
-    I.ctr->scratch[SC_ROOTS] = 0;
-}
-
-__global__ void starts_kernel(DevInterner I, ApplyArgs a) {
-    pdl_wait();
-    pdl_release();
-    const uint32_t count = (uint32_t)I.ctr->scratch[SC_ENTRIES];
-    if (blockIdx.x == 0 && threadIdx.x == 0) starts_head(I, a, count);
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x)
-        if (a.flags[j]) a.p_start[a.pos[j]] = j;
-}
-
-// Entries of the next level pass: the parents just reduced that are not tree roots.
-__device__ __forceinline__ void next_count(const DevInterner &I) {
-    I.ctr->scratch[SC_ENTRIES] = I.ctr->scratch[SC_PARENTS] - I.ctr->scratch[SC_ROOTS];
-}
-
-// Phase 2 for one level: parents cta_base + threadIdx.x, + stride, ... of the n_par run heads
-// (a CTA-uniform loop, as in bottom_range).
+// ---- Phase 2 -----------------------------------------------------------------------------------------
+// Parents cta_base + threadIdx.x, + stride, ... of step s (n_par of them, their children are the n_child
+// entries of step s - 1). A CTA-uniform loop: whole warps take part in the warp-cooperative interning.
 __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyArgs &a, int mode, const LeafRefs &L,
-                                              int step, int buf, uint32_t n_par, uint64_t cta_base, uint64_t stride) {
-    const int nb = buf ^ 1;
+                                              uint32_t s, uint32_t n_par, uint32_t n_child, uint64_t cta_base, uint64_t stride) {
+    const uint64_t *in_id = s == 1 ? a.rec_id : a.e_id[(s - 1) & 1];
+    const uint32_t *in_val = s == 1 ? a.rec_val : a.e_val[(s - 1) & 1];
     for (uint64_t base = cta_base; base < n_par; base += stride) {
         const uint64_t p = base + threadIdx.x;
         const bool in = p < n_par;
         uint64_t c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         uint32_t cv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         uint32_t types = 0, mask = 0, lod = 0;
-        uint32_t i = 0, path0 = 0;
-        int d = 0, t = 0;
-        bool want_branch = false;
+        uint32_t i = 0, r0 = 0;
+        bool want_branch = false, changed = false;
         uint64_t out = EMPTY_ID;
         uint32_t out_val = 0;
         if (in) {
-            const uint32_t b = a.p_start[p], e = a.p_start[p + 1];
-            i = a.e_item[buf][b];
-            d = a.it_depth[i];
-            t = d - step;
-            path0 = a.e_path[buf][b];
-            // the old node at the parent's place (voxtree.rs:934-952)
-            uint64_t eq = a.it_init[i], leaf = EMPTY_ID;
-            for (int cd = 0; cd + 1 < t; ++cd) {
-                if (id_is_leaf(eq)) {
-                    leaf = eq;
-                    eq = EMPTY_ID;
-                    break;
-                }
-                const uint32_t idx = (path0 >> (3 * (d - cd - 1))) & 7u;
-                eq = I.children[8ull * id_index(eq) + idx];
-                if (eq == EMPTY_ID) break;
-            }
-            if (id_is_leaf(eq)) {
-                leaf = eq;
-                eq = EMPTY_ID;
-            }
-            // gather the run of new children (voxtree.rs:959-1000); slots by select, so that the
+            r0 = a.p_rec[s][p];
+            i = a.rec_item[r0];
+            const uint32_t b = a.p_start[s][p];
+            uint32_t e = p + 1 < n_par ? a.p_start[s][p + 1] : n_child;
+            if (e > n_child) e = n_child;
+            const bool last = p + 1 == n_par;  // its run ends where its item's entries do
+            // gather the run of changed children (voxtree.rs:959-1000); slots by select, so that the
             // arrays stay in registers
             for (uint32_t j = b; j < e; ++j) {
-                const uint32_t ti = (a.e_path[buf][j] >> (3 * (d - t))) & 7u;
-                const uint64_t id = a.e_id[buf][j];
-                const uint32_t ev = a.e_val[buf][j];
+                if (last && a.rec_item[s == 1 ? j : a.p_rec[s - 1][j]] != i) break;
+                const uint32_t ev = in_val[j];
+                if (!(ev & kChanged)) continue;
+                const uint32_t ti = (ev >> 16) & 7u;
+                const uint64_t id = in_id[j];
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
                     if ((uint32_t)k == ti) {
                         c[k] = id;
-                        cv[k] = ev;
+                        cv[k] = ev & 0xFFFFu;
                     }
                 types |= (id_is_leaf(id) ? 1u : 0u) << ti;
                 mask |= 1u << ti;
+            }
+            changed = mask != 0;
+        }
+        if (changed) {
+            // the old node at the parent's place (voxtree.rs:934-952): a branch, or a leaf at or above it
+            uint64_t eq = a.p_old[s][p], leaf = EMPTY_ID;
+            if (id_is_leaf(eq)) {
+                leaf = eq;
+                eq = EMPTY_ID;
             }
             if (mode == 1) {  // remove_at_depth_branch / _leaf one level up (voxtree.rs:559-706)
                 const uint32_t ch = mask;
@@ -703,9 +583,6 @@ __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyA
                 if (mask) {
                     want_branch = true;
                     lod = calc_average8(cv);
-                } else {
-                    out = EMPTY_ID;
-                    out_val = 0;
                 }
             } else {
                 const uint32_t existing_mask = eq != EMPTY_ID ? id_mask(eq) : 0u;
@@ -714,7 +591,7 @@ __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyA
                 if (mask != 0xFF) {
                     if (cloned) {  // voxtree.rs:1017-1031
                         const uint64_t *src = I.children + 8ull * id_index(eq);
-    #pragma unroll
+#pragma unroll
                         for (int k = 0; k < 8; ++k) {
                             if (!((cloned >> k) & 1)) continue;
                             c[k] = src[k];
@@ -724,7 +601,7 @@ __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyA
                         }
                     } else if (leaf != EMPTY_ID) {  // voxtree.rs:1032-1047
                         const uint32_t lv = node_value(I, id_index(leaf));
-    #pragma unroll
+#pragma unroll
                         for (int k = 0; k < 8; ++k)
                             if ((inv >> k) & 1) {
                                 c[k] = leaf;
@@ -735,7 +612,7 @@ __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyA
                     }
                 }
                 bool same = types == 0xFF;
-    #pragma unroll
+#pragma unroll
                 for (int k = 1; k < 8; ++k) same = same && c[k] == c[0];
                 if (same) {  // voxtree.rs:1062-1075
                     out = c[0];
@@ -746,7 +623,7 @@ __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyA
                     lod = calc_average8(cv);
                 }
             }
-            }
+        }
         bool created;
         const uint64_t id = warp_intern_branch_inl(I, want_branch, c, types, mask, lod, &created);
         if (created) add_child_refs(I, L, c, cv);
@@ -755,341 +632,195 @@ __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyA
             out = id;
             out_val = lod;
         }
-        if (t == 1) {
-            a.it_new[i] = out;
-            atomicAdd(&I.ctr->scratch[SC_ROOTS], 1ull);
+        if ((uint32_t)a.it_depth[i] - 1u == s) {
+            if (changed) finish_item(I, a, mode, i, out);
         } else {
-            a.e_item[nb][p] = i;
-            a.e_path[nb][p] = path0 & path_mask(d, t - 2);
-            a.e_id[nb][p] = out;
-            a.e_val[nb][p] = out_val;
+            a.e_id[s & 1][p] = out;
+            a.e_val[s & 1][p] = entry_word(out_val, a.rec_group[r0] >> (3 * s), changed);
         }
     }
 }
 
-__global__ void __launch_bounds__(512, VX_APPLY_MIN_BLOCKS) parents_kernel(DevInterner I, ApplyArgs a, int step, int buf) {
+// ---- phases of an apply ------------------------------------------------------------------------------
+// Set phase: depths, Phase 0 and the counts of the plan. All threads of the grid.
+__device__ __forceinline__ void phase_plan(const DevInterner &I, const ApplyArgs &a, bool check_depths,
+                                           uint32_t (*cnt_s)[kPlanWords]) {
+    const uint64_t gt = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    if (gt == 0) I.ctr->scratch[SC_RELEASE] = 0;
+    for (uint64_t i = gt; i < a.n_items; i += stride) {
+        if (check_depths) {
+            bool bad = false;
+            const_cast<uint8_t *>(a.it_depth)[i] = (uint8_t)item_depth_of(I, a, (uint32_t)i, true, &bad);
+            if (bad) set_error(I, ERR_INVALID, 46);
+        }
+        prep_item(I, a, (uint32_t)i);
+    }
+    plan_count(I, a, check_depths, cnt_s);
+}
+
+// Phase 1, and the roots of the items that have none of it.
+__device__ __forceinline__ void phase_bottom(const DevInterner &I, const ApplyArgs &a, int mode, const LeafRefs &L,
+                                             const Plan &P) {
+    const uint64_t gt = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    if (mode == 0)
+        for (uint64_t i = gt; i < a.n_items; i += stride)
+            if (!(a.it_flags[i] & 2)) finish_item(I, a, 0, (uint32_t)i, a.it_init[i]);
+    bottom_records(I, a, mode, L, P);
+}
+
+constexpr int kMaxApplyWarps = 16;  // 512 threads
+
+// One launch per phase (tune_set_launch 0).
+__global__ void __launch_bounds__(512) apply_plan_kernel(DevInterner I, ApplyArgs a, int check_depths) {
     pdl_wait();
     pdl_release();
-    const LeafRefs L = leaf_refs_init(I);
-    parents_range(I, a, a.mode, L, step, buf, (uint32_t)I.ctr->scratch[SC_PARENTS],
-                  (uint64_t)blockIdx.x * blockDim.x, (uint64_t)gridDim.x * blockDim.x);
-    leaf_refs_flush(I, L);
-    if (grid_last_cta(&I.ctr->scratch[SC_DONE])) next_count(I);  // entries of the next step
+    __shared__ uint32_t cnt_s[kMaxApplyWarps][kPlanWords];
+    phase_plan(I, a, check_depths != 0, cnt_s);
 }
 
-
-
-__device__ __forceinline__ void finish_item(const DevInterner &I, const ApplyArgs &a, int mode, uint32_t i) {
-    if (mode == 1) {
-        const uint64_t nw = a.it_new[i], old = a.it_old[i];
-        if (nw == INVALID_ID) return;
-        if (nw != EMPTY_ID) atomicAdd(I.refcount + id_index(nw), 1u);
-        if (old != EMPTY_ID) {
-            const unsigned long long e = atomicAdd(&I.ctr->scratch[SC_RELEASE], 1ull);
-            a.release_list[e] = old;
-        }
-        I.roots[a.it_tree[i]] = nw;
-        a.it_changed[i] = 1;
-        return;
-    }
-    a.it_changed[i] = 0;
-    if (a.it_panic[i]) return;
-    const uint64_t nw = a.it_new[i], old = a.it_old[i];
-    if (nw == INVALID_ID) return;
-    const uint8_t f = a.it_flags[i];
-    if ((f & 3) && nw != EMPTY_ID) atomicAdd(I.refcount + id_index(nw), 1u);  // the tree's root reference
-    if (old != EMPTY_ID) {
-        if (nw == old && !(I.flags & (1u << 4))) {  // assert_ne!(new_root_id, self.root_id) (voxtree.rs:311)
-            set_error(I, ERR_REF_PANIC, 41);
-            return;
-        }
-        const unsigned long long e = atomicAdd(&I.ctr->scratch[SC_RELEASE], 1ull);
-        a.release_list[e] = old;
-    }
-    I.roots[a.it_tree[i]] = nw;
-    a.it_changed[i] = 1;
-}
-
-// Commits every item's root, then (last CTA) closes the allocation epoch: every node of this apply
-// pass has been created and has added its children's references by now.
-__global__ void finish_items_kernel(DevInterner I, ApplyArgs a) {
+__global__ void __launch_bounds__(512, VX_APPLY_MIN_BLOCKS) apply_bottom_kernel(DevInterner I, ApplyArgs a, int mode) {
     pdl_wait();
     pdl_release();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < a.n_items) finish_item(I, a, a.mode, i);
-    if (grid_last_cta(&I.ctr->scratch[SC_DONE])) epoch_finalize_body(I);
-}
-
-__global__ void zero_counter_kernel(DevInterner I, int slot) { pdl_wait(); pdl_release(); I.ctr->scratch[slot] = 0; }
-
-__device__ __forceinline__ void item_depth(const DevInterner &I, const ApplyArgs &a, uint32_t i) {
-    const uint32_t t = a.it_tree[i];
-    const int d = t < I.tree_cap ? I.depths[t] : TREE_UNUSED;
-    int prev = 0xFF;
-    if (i > 0) {
-        const uint32_t tp = a.it_tree[i - 1];
-        prev = tp < I.tree_cap ? I.depths[tp] : TREE_UNUSED;
-    }
-    if (d == TREE_UNUSED || d > a.max_depth || d < 2 || (i > 0 && d > prev)) {
-        set_error(I, ERR_INVALID, 46);
-        const_cast<uint8_t *>(a.it_depth)[i] = 2;
-        return;
-    }
-    const_cast<uint8_t *>(a.it_depth)[i] = (uint8_t)d;
-}
-
-__global__ void item_depths_kernel(DevInterner I, ApplyArgs a) {
-    pdl_wait();
-    pdl_release();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < a.n_items) item_depth(I, a, i);
-}
-
-// ---- the whole apply in one cooperative launch -------------------------------------------------------
-// Exclusive scan of one value per thread across the CTA (blockDim.x a multiple of 32, at most 1024);
-// *total receives the CTA's sum. Every thread of the CTA calls it.
-__device__ __forceinline__ uint32_t cta_exclusive_scan(uint32_t x, uint32_t *total) {
-    __shared__ uint32_t wsum[32];
-    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    uint32_t incl = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= (unsigned)o) incl += y;
-    }
-    if (lane == 31) wsum[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < nw ? wsum[lane] : 0u;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, w, o);
-            if (lane >= (unsigned)o) w += y;
-        }
-        if (lane < nw) wsum[lane] = w;
-    }
-    __syncthreads();
-    const uint32_t excl = incl - x + (warp ? wsum[warp - 1] : 0u);
-    *total = wsum[nw - 1];
-    __syncthreads();  // wsum is reused by the next call
-    return excl;
-}
-
-// Exclusive scan of in[0..n) into out (out[n] = the total) by the whole cooperative grid: each CTA
-// sums a contiguous range, the sums meet at a grid barrier, then each CTA scans its range from the
-// sum of the ranges before it. Ends with a grid barrier (out is read across CTAs afterwards).
-__device__ __forceinline__ bool grid_exclusive_scan(const DevInterner &I, const uint32_t *in, uint32_t *out,
-                                                    uint32_t n, uint32_t *partials) {
-    const uint32_t per = (n + gridDim.x - 1) / gridDim.x;
-    const uint32_t lo = min(n, blockIdx.x * per), hi = min(n, lo + per);
-    uint32_t s = 0, tot;
-    for (uint32_t k = lo + threadIdx.x; k < hi; k += blockDim.x) s += in[k];
-    cta_exclusive_scan(s, &tot);
-    if (threadIdx.x == 0) partials[blockIdx.x] = tot;
-    if (!grid_sync(I)) return false;
-    uint32_t before = 0;
-    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += blockDim.x) before += partials[b];
-    cta_exclusive_scan(before, &tot);
-    uint32_t carry = tot;
-    for (uint32_t base = lo; base < hi; base += blockDim.x) {
-        const uint32_t k = base + threadIdx.x;
-        const uint32_t x = k < hi ? in[k] : 0u;
-        const uint32_t e = cta_exclusive_scan(x, &tot);
-        if (k < hi) out[k] = carry + e;
-        carry += tot;
-    }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = carry;
-    return grid_sync(I);
-}
-
-// The set phase (mode 0) and, when `clear_pass`, the clear pass (mode 1) with their releases: the
-// launch sequence of launch_apply_bottom / launch_apply_levels / launch_release in one kernel whose
-// phases are separated by grid barriers. Counts stay in device memory and are read by every CTA
-// after the barrier that follows their last write.
-__global__ void __launch_bounds__(512, VX_APPLY_MIN_BLOCKS) apply_single_kernel(const DevInterner I, const ApplyArgs a,
-                                                                                   int check_depths, int clear_pass,
-                                                                                   uint32_t *frontier_a,
-                                                                                   uint32_t *frontier_b, int rounds) {
-    const uint64_t cta_base = (uint64_t)blockIdx.x * blockDim.x, stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t gt = cta_base + threadIdx.x;
-    const bool t0 = gt == 0;
-    DevCounters *ctr = I.ctr;
-    if (check_depths) {
-        for (uint64_t i = gt; i < a.n_items; i += stride) item_depth(I, a, (uint32_t)i);
-        if (!grid_sync(I)) return;
-    }
-    for (int mode = 0; mode <= clear_pass; ++mode) {
+    __shared__ Plan P;
+    plan_totals(a, P);
+    if (blockIdx.x == 0 && threadIdx.x < kPlanWords) a.level_n[threadIdx.x] = P.total[threadIdx.x];
+    if (mode == 1 && blockIdx.x == 0 && threadIdx.x == 0) I.ctr->scratch[SC_RELEASE] = 0;
+    if (mode == 0 || P.total[0]) {
         const LeafRefs L = leaf_refs_init(I);
-        for (uint64_t i = gt; i < a.n_items; i += stride) prep_item(I, a, mode, (uint32_t)i);
-        if (!grid_sync(I)) return;
-        // Phase 1, then the changed groups become the first level's entries
-        bottom_range(I, a, mode, L, cta_base, stride);
-        if (!grid_sync(I)) return;
-        if (!grid_exclusive_scan(I, a.flags, a.pos, a.n_records, a.scan_tmp)) return;
-        for (uint64_t r = gt; r < a.n_records; r += stride) scatter_record(a, (uint32_t)r);
-        uint32_t count = a.pos[a.n_records];
-        if (!grid_sync(I)) return;
-        // Phase 2, one level step at a time
-        int buf = 0;
-        for (int step = 1; step <= a.max_depth - 1; ++step) {
-            for (uint64_t j = gt; j < count; j += stride) head_flag(a, step, buf, (uint32_t)j);
-            if (!grid_sync(I)) return;
-            if (!grid_exclusive_scan(I, a.flags, a.pos, count, a.scan_tmp)) return;
-            const uint32_t np = a.pos[count];
-            if (t0) {
-                a.p_start[np] = count;
-                ctr->scratch[SC_ROOTS] = 0;
-            }
-            for (uint64_t j = gt; j < count; j += stride)
-                if (a.flags[j]) a.p_start[a.pos[j]] = (uint32_t)j;
-            if (!grid_sync(I)) return;
-            parents_range(I, a, mode, L, step, buf, np, cta_base, stride);
-            if (!grid_sync(I)) return;
-            count = np - (uint32_t)ctr->scratch[SC_ROOTS];  // parents that are not tree roots
-            buf ^= 1;
-        }
-        // roots, the epoch, the release of the replaced roots
-        if (t0) ctr->scratch[SC_RELEASE] = 0;
-        if (!grid_sync(I)) return;
-        for (uint64_t i = gt; i < a.n_items; i += stride) finish_item(I, a, mode, (uint32_t)i);
+        phase_bottom(I, a, mode, L, P);
         leaf_refs_flush(I, L);
-        if (t0) {
-            ctr->rel_count[0] = 0;
-            ctr->rel_count[1] = 0;
+    }
+    // without records no level pass follows that would close the epoch
+    if (a.n_records == 0 && grid_last_cta(&I.ctr->scratch[SC_DONE])) epoch_finalize_body(I);
+}
+
+__global__ void __launch_bounds__(512, VX_APPLY_MIN_BLOCKS) apply_parents_kernel(DevInterner I, ApplyArgs a, int mode, int s) {
+    pdl_wait();
+    pdl_release();
+    if (mode == 0 || a.level_n[0]) {
+        const LeafRefs L = leaf_refs_init(I);
+        parents_range(I, a, mode, L, s, a.level_n[s], s == 1 ? a.n_records : a.level_n[s - 1],
+                      (uint64_t)blockIdx.x * blockDim.x, (uint64_t)gridDim.x * blockDim.x);
+        leaf_refs_flush(I, L);
+    }
+    if (s == a.max_depth - 1 && grid_last_cta(&I.ctr->scratch[SC_DONE])) epoch_finalize_body(I);
+}
+
+// ---- the whole apply in one launch ---------------------------------------------------------------------
+// Barrier of all threads of the launch; writes before it are visible to all after it. sync() returns
+// false when its bounded wait gave up (ERR_TIMEOUT recorded).
+// Grid: a cooperative launch (every CTA resident). Thread 0 of each CTA adds one to a counter that only
+// grows and waits for it to reach the barrier's number of arrivals: one round trip after the last arrival.
+// The counter's value at the start of a launch is kept beside it, and moved by the first CTA as it leaves
+// (every CTA has read it by then).
+struct GridBarrier {
+    const DevInterner &I;
+    unsigned long long target;
+    __device__ explicit GridBarrier(const DevInterner &i) : I(i), target(*(volatile unsigned long long *)&i.ctr->bar_gen) {}
+    // After a barrier that gave up the arrivals are out of step until the interner is reset.
+    __device__ bool usable() { return !(*reinterpret_cast<volatile unsigned int *>(&I.ctr->error) & ERR_TIMEOUT); }
+    __device__ bool sync() {
+        __shared__ int ok_s;
+        target += gridDim.x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int ok = 1;
+            __threadfence();
+            atomicAdd(&I.ctr->bar_count, 1ull);
+            for (uint32_t spin = 0; (long long)(ld_acquire(reinterpret_cast<const uint64_t *>(&I.ctr->bar_count)) - target) < 0;) {
+                // a CTA that gave up at an earlier barrier never arrives: stop waiting at once
+                const bool gave_up = (spin & 1023u) == 1023u &&
+                                     (*reinterpret_cast<volatile unsigned int *>(&I.ctr->error) & ERR_TIMEOUT);
+                if (++spin >= I.spin_limit || gave_up) {
+                    set_error(I, ERR_TIMEOUT, 49);
+                    ok = 0;
+                    break;
+                }
+                __nanosleep(20);
+            }
+            __threadfence();
+            ok_s = ok;
         }
-        if (!grid_sync(I)) return;
+        __syncthreads();
+        return ok_s != 0;
+    }
+    __device__ void leave() {
+        if (blockIdx.x == 0 && threadIdx.x == 0) I.ctr->bar_gen = target;
+    }
+};
+
+// One cluster: its hardware barrier.
+struct ClusterBarrier {
+    __device__ explicit ClusterBarrier(const DevInterner &) {}
+    __device__ bool usable() { return true; }
+    __device__ bool sync() {
+        asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        return true;
+    }
+    __device__ void leave() {}
+};
+
+// The set phase (mode 0) and, when `clear_pass` and some record has clear bits, the clear pass (mode 1), each
+// with its release: the phases of the separate launches with a barrier after each. Barriers: two, one a
+// level, one for the roots and one a release round that has nodes.
+template <class Barrier>
+__device__ __forceinline__ void apply_single(const DevInterner &I, const ApplyArgs &a, int check_depths, int clear_pass,
+                                             uint32_t *frontier_a, uint32_t *frontier_b, int rounds) {
+    extern __shared__ uint32_t leaf_smem[];
+    __shared__ uint32_t cnt_s[kMaxApplyWarps][kPlanWords];
+    __shared__ Plan P;
+    const uint64_t cta_base = (uint64_t)blockIdx.x * blockDim.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    const bool t0 = cta_base + threadIdx.x == 0;
+    DevCounters *ctr = I.ctr;
+    Barrier bar(I);
+    if (!bar.usable()) return;
+    phase_plan(I, a, check_depths != 0, cnt_s);
+    if (!bar.sync()) return;
+    plan_totals(a, P);
+    for (int mode = 0; mode <= clear_pass && (mode == 0 || P.total[0]); ++mode) {
+        const LeafRefs L = leaf_refs_init(I);
+        if (t0) {
+            ctr->rel_count[0] = ctr->rel_count[1] = ctr->rel_count[2] = 0;
+            if (mode == 1) ctr->scratch[SC_RELEASE] = 0;
+        }
+        phase_bottom(I, a, mode, L, P);
+        if (!bar.sync()) return;
+        for (int s = 1; s <= a.max_depth - 1 && a.n_records; ++s) {
+            parents_range(I, a, mode, L, s, P.total[s], s == 1 ? a.n_records : P.total[s - 1], cta_base, stride);
+            if (s == a.max_depth - 1) leaf_refs_flush(I, L);
+            if (!bar.sync()) return;
+        }
         if (t0) epoch_finalize_body(I);
         release_roots_range(I, a.release_list, frontier_a, &ctr->rel_count[0], cta_base, stride);
-        if (!grid_sync(I)) return;
+        const LeafDrops D = leaf_drops_init(I, leaf_smem);  // the leaf counts were flushed before the last barrier
+        if (!bar.sync()) return;
         // round r reads set r % 3 and writes set (r + 1) % 3; set (r + 2) % 3 was read by round r - 1
         // and is written by round r + 1, so it is cleared now
         uint32_t *fr[2] = {frontier_a, frontier_b};
-        extern __shared__ uint32_t leaf_smem[];
-        const LeafDrops D = leaf_drops_init(I, leaf_smem);  // the leaf counts were flushed before the last barrier
         for (int r = 0; r < rounds; ++r) {
             if (*(volatile unsigned long long *)&ctr->rel_count[r % 3] == 0) break;  // the same answer in every CTA
             if (t0) ctr->rel_count[(r + 2) % 3] = 0;
             release_round_range(I, D, fr[r & 1], fr[(r + 1) & 1], &ctr->rel_count[r % 3], &ctr->rel_count[(r + 1) % 3],
                                 cta_base, stride);
-            if (!grid_sync(I)) return;
+            if (!bar.sync()) return;
         }
     }
+    bar.leave();
 }
 
-}  // namespace
-
-size_t scan_tmp_words(uint32_t n) { return (size_t)(n + kScanBlock - 1) / kScanBlock + 32; }
-
-// Dynamic shared memory of the kernels that create branches (their LeafRefs table).
-static size_t leaf_refs_smem(const DevInterner &I) { return I.vbits == 8 ? 256 * 4 : 2 * kLeafSlots * 4; }
-
-// Scan of the first *n_dev of n_max flags (count in device memory): one launch with the look-back
-// status words for up to kScanStatusTiles tiles (a serving wave's records: 4 fewer launches per
-// level), else block sums, their scan and an add (large batches: the single-thread look-back walk
-// measured 12% slower than the three launches on 45 M edits).
-static cudaError_t launch_scan_dev(const DevInterner &I, const uint32_t *flags, uint32_t *pos, uint32_t *tmp,
-                                   uint32_t n_max, const unsigned long long *n_dev, unsigned long long *status,
-                                   cudaStream_t s) {
-    const uint32_t nb = (n_max + kScanBlock - 1) / kScanBlock;
-    if (nb == 0) return cudaSuccess;
-    if (status && nb <= kScanStatusTiles) {
-        count_launches(1);
-        (void)launch_pdl(scan_onepass_dev_kernel, dim3(nb), dim3(kThreads), 0, s, I, flags, pos, status, n_dev);
-        return cudaGetLastError();
-    }
-    count_launches(1);
-    (void)launch_pdl(scan_blocks_dev_kernel, dim3(nb), dim3(kThreads), 0, s, flags, pos, tmp, n_dev);
-    if (nb > 1) {
-        uint32_t *tmp2 = tmp + nb;
-        cudaError_t e = launch_scan(tmp, tmp2, tmp2 + nb + 1 + 32, nb, s);
-        if (e != cudaSuccess) return e;
-        count_launches(1);
-        (void)launch_pdl(scan_add_dev_kernel, dim3(nb), dim3(kThreads), 0, s, pos, tmp2, n_dev);
-    }
-    count_launches(1);
-    (void)launch_pdl(scan_total_dev_kernel, dim3(1), dim3(1), 0, s, flags, pos, n_dev);
-    return cudaGetLastError();
+__global__ void __launch_bounds__(512, VX_APPLY_MIN_BLOCKS) apply_grid_kernel(const DevInterner I, const ApplyArgs a,
+                                                                              int check_depths, int clear_pass,
+                                                                              uint32_t *frontier_a, uint32_t *frontier_b,
+                                                                              int rounds) {
+    apply_single<GridBarrier>(I, a, check_depths, clear_pass, frontier_a, frontier_b, rounds);
 }
 
-cudaError_t launch_scan(const uint32_t *flags, uint32_t *pos, uint32_t *tmp, uint32_t n, cudaStream_t s) {
-    const uint32_t nb = (n + kScanBlock - 1) / kScanBlock;
-    if (nb == 0) {
-        count_launches(1);
-        (void)launch_pdl(scan_total_kernel, dim3(1), dim3(1), 0, s, flags, pos, 0);
-        return cudaGetLastError();
-    }
-    count_launches(1);
-    (void)launch_pdl(scan_blocks_kernel, dim3(nb), dim3(kThreads), 0, s, flags, pos, tmp, n);
-    if (nb > 1) {
-        uint32_t *tmp2 = tmp + nb;  // scan of the block sums (recursive)
-        cudaError_t e = launch_scan(tmp, tmp2, tmp2 + nb + 1 + 32, nb, s);
-        if (e != cudaSuccess) return e;
-        count_launches(1);
-        (void)launch_pdl(scan_add_kernel, dim3(nb), dim3(kThreads), 0, s, pos, tmp2, n);
-    }
-    count_launches(1);
-    (void)launch_pdl(scan_total_kernel, dim3(1), dim3(1), 0, s, flags, pos, n);
-    return cudaGetLastError();
+__global__ void __launch_bounds__(512, 1) apply_cluster_kernel(const DevInterner I, const ApplyArgs a, int check_depths,
+                                                               int clear_pass, uint32_t *frontier_a, uint32_t *frontier_b,
+                                                               int rounds) {
+    apply_single<ClusterBarrier>(I, a, check_depths, clear_pass, frontier_a, frontier_b, rounds);
 }
 
-cudaError_t launch_item_depths(const DevInterner &I, const ApplyArgs &a, cudaStream_t s) {
-    if (a.n_items == 0) return cudaSuccess;
-    count_launches(1);
-    (void)launch_pdl(item_depths_kernel, dim3((a.n_items + kThreads - 1) / kThreads), dim3(kThreads), 0, s, I, a);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_apply_bottom(const DevInterner &I, const ApplyArgs &a, int num_sms, cudaStream_t s) {
-    const unsigned ib = (a.n_items + kThreads - 1) / kThreads;
-    count_launches(1);
-    (void)launch_pdl(prep_items_kernel, dim3(ib), dim3(kThreads), 0, s, I, a);
-    const uint32_t R = a.n_records;
-    if (R) {
-        const int bt = a.threads > 0 ? a.threads : kThreads;
-        const unsigned cap = (unsigned)num_sms * (unsigned)(a.blocks_per_sm > 0 ? a.blocks_per_sm : 8);
-        const unsigned need = (R + bt - 1) / bt;
-        const unsigned g = need < cap ? need : cap;
-        count_launches(1);
-        (void)launch_pdl(bottom_kernel, dim3(g), dim3(bt), leaf_refs_smem(I), s, I, a);
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_apply_levels(const DevInterner &I, const ApplyArgs &a, int num_sms, cudaStream_t s) {
-    const unsigned ib = (a.n_items + kThreads - 1) / kThreads;
-    const uint32_t R = a.n_records;
-    const unsigned rb = (R + kThreads - 1) / kThreads;
-    if (R) {
-        const int bt = a.threads > 0 ? a.threads : kThreads;
-        const unsigned cap = (unsigned)num_sms * (unsigned)(a.blocks_per_sm > 0 ? a.blocks_per_sm : 8);
-        const unsigned need = (R + bt - 1) / bt;
-        const unsigned g = need < cap ? need : cap;
-        cudaError_t e = launch_scan(a.flags, a.pos, a.scan_tmp, R, s);
-        if (e != cudaSuccess) return e;
-        count_launches(1);
-        (void)launch_pdl(scatter_bottom_kernel, dim3(rb), dim3(kThreads), 0, s, I, a);
-        int buf = 0;
-        const unsigned sb = rb < (unsigned)num_sms * 16 ? rb : (unsigned)num_sms * 16;
-        for (int step = 1; step <= a.max_depth - 1; ++step) {
-            count_launches(1);
-            (void)launch_pdl(heads_kernel, dim3(sb), dim3(kThreads), 0, s, I, a, step, buf);
-            e = launch_scan_dev(I, a.flags, a.pos, a.scan_tmp, R, &I.ctr->scratch[SC_ENTRIES], a.scan_status, s);
-            if (e != cudaSuccess) return e;
-            count_launches(1);
-            (void)launch_pdl(starts_kernel, dim3(sb), dim3(kThreads), 0, s, I, a);
-            count_launches(1);
-            (void)launch_pdl(parents_kernel, dim3(g), dim3(bt), leaf_refs_smem(I), s, I, a, step, buf);  // its last CTA sets the next entry count
-            buf ^= 1;
-        }
-    }
-    count_launches(1);
-    (void)launch_pdl(zero_counter_kernel, dim3(1), dim3(1), 0, s, I, SC_RELEASE);
-    count_launches(1);
-    (void)launch_pdl(finish_items_kernel, dim3(ib), dim3(kThreads), 0, s, I, a);  // its last CTA closes the epoch
-    return cudaGetLastError();
-}
-
-namespace {
 // rec_item[r] = i for every record r of item i (records of item i: [first[i], first[i+1])), one CTA
 // per item with coalesced stores.
 __global__ void __launch_bounds__(kThreads) expand_items_kernel(const uint32_t *first, uint32_t n,
@@ -1099,7 +830,44 @@ __global__ void __launch_bounds__(kThreads) expand_items_kernel(const uint32_t *
         for (uint32_t r = first[i] + threadIdx.x; r < r1; r += blockDim.x) rec_item[r] = i;
     }
 }
+
 }  // namespace
+
+// Dynamic shared memory of the kernels that create branches (their LeafRefs table), and of the single
+// launch, whose release rounds use it in turn.
+static size_t leaf_refs_smem(const DevInterner &I) { return I.vbits == 8 ? 256 * 4 : 2 * kLeafSlots * 4; }
+
+static int apply_threads_of(const ApplyArgs &a) { return a.threads > 0 ? a.threads : kThreads; }
+
+uint32_t apply_max_ctas(int num_sms, int blocks_per_sm) {
+    const uint32_t g = (uint32_t)num_sms * (uint32_t)(blocks_per_sm > 0 ? blocks_per_sm : 8);
+    return g < kApplyCluster ? kApplyCluster : g;
+}
+
+cudaError_t launch_apply(const DevInterner &I, const ApplyArgs &a, int mode, bool check_depths, int num_sms, cudaStream_t s,
+                         void (*levels_begin)(void *), void *levels_ctx) {
+    const int bt = apply_threads_of(a);
+    const uint64_t items = a.n_records > a.n_items ? a.n_records : a.n_items;
+    const uint64_t cap = (uint64_t)num_sms * (uint64_t)(a.blocks_per_sm > 0 ? a.blocks_per_sm : 8);
+    uint64_t g = (items + bt - 1) / bt;
+    if (g > cap) g = cap;
+    if (g < 1) g = 1;
+    if (mode == 0) {
+        count_launches(1);
+        cudaError_t e = launch_pdl(apply_plan_kernel, dim3((unsigned)g), dim3(bt), 0, s, I, a, check_depths ? 1 : 0);
+        if (e != cudaSuccess) return e;
+    }
+    count_launches(1);
+    cudaError_t e = launch_pdl(apply_bottom_kernel, dim3((unsigned)g), dim3(bt), leaf_refs_smem(I), s, I, a, mode);
+    if (levels_begin) (*levels_begin)(levels_ctx);
+    for (int step = 1; step <= a.max_depth - 1 && a.n_records && e == cudaSuccess; ++step) {
+        uint64_t gp = ((uint64_t)a.p_cap[step] + bt - 1) / bt;
+        if (gp > cap) gp = cap;
+        count_launches(1);
+        e = launch_pdl(apply_parents_kernel, dim3((unsigned)gp), dim3(bt), leaf_refs_smem(I), s, I, a, mode, step);
+    }
+    return e;
+}
 
 cudaError_t launch_expand_items(const uint32_t *first, uint32_t n, uint32_t *rec_item, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
@@ -1108,43 +876,53 @@ cudaError_t launch_expand_items(const uint32_t *first, uint32_t n, uint32_t *rec
     return cudaGetLastError();
 }
 
-size_t apply_single_scan_words(int num_sms) { return (size_t)num_sms * 32 + 64; }
-
-// The whole apply sequence in one cooperative launch: as many CTAs as can be resident at once (the
-// grid barrier needs every CTA running).
+#ifndef VX_CLUSTER_RECORDS
+#define VX_CLUSTER_RECORDS 4096
+#endif
+// The whole apply sequence in one launch: a small apply as one cluster, whose barrier is in hardware; else
+// as many CTAs as can be resident at once (the grid barrier needs every CTA running).
 cudaError_t launch_apply_single(const DevInterner &I, const ApplyArgs &a, bool check_depths, bool clear_pass,
                                 uint32_t *frontier_a, uint32_t *frontier_b, int rounds, int num_sms, cudaStream_t s) {
-    const int bt = a.threads > 0 ? a.threads : kThreads;
     const size_t smem = std::max(leaf_refs_smem(I), release_smem(I.vbits));
+    const uint64_t items = a.n_records > a.n_items ? a.n_records : a.n_items;
+    int cd = check_depths ? 1 : 0, cp = clear_pass ? 1 : 0;
+    if (items <= VX_CLUSTER_RECORDS) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kApplyCluster);
+        cfg.blockDim = dim3(512);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kApplyCluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        count_launches(1);
+        return cudaLaunchKernelEx(&cfg, apply_cluster_kernel, I, a, cd, cp, frontier_a, frontier_b, rounds);
+    }
+    const int bt = apply_threads_of(a);
     static int per_sm_cache[2][17] = {};  // [vbits == 16][threads / 32]
     int &per_sm = per_sm_cache[I.vbits == 16][bt / 32];
     if (per_sm == 0) {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, apply_single_kernel, bt, smem);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, apply_grid_kernel, bt, smem);
         if (e != cudaSuccess) return e;
         if (per_sm < 1) return cudaErrorInvalidConfiguration;
     }
     int want = a.blocks_per_sm > 0 ? a.blocks_per_sm : per_sm;
     if (want > per_sm) want = per_sm;
-    if ((size_t)num_sms * want > apply_single_scan_words(num_sms) - 64) want = 32;  // partials of the grid scan
-    // a small apply (a serving wave) runs on as few CTAs as its records fill, no fewer than a quarter
-    // of the SMs: every grid barrier costs one arrival per CTA
+    // a small apply runs on as few CTAs as its records fill, no fewer than a quarter of the SMs: every
+    // grid barrier costs one arrival per CTA
     uint64_t grid = (uint64_t)num_sms * want;
-    const uint64_t fill = ((uint64_t)(a.n_records > a.n_items ? a.n_records : a.n_items) + bt - 1) / bt;
+    const uint64_t fill = (items + bt - 1) / bt;
     const uint64_t floor_ctas = (uint64_t)(num_sms + 3) / 4;
     if (fill < grid) grid = fill > floor_ctas ? fill : floor_ctas;
     DevInterner Ic = I;
     ApplyArgs ac = a;
-    int cd = check_depths ? 1 : 0, cp = clear_pass ? 1 : 0;
     void *args[] = {&Ic, &ac, &cd, &cp, &frontier_a, &frontier_b, &rounds};
     count_launches(1);
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(apply_single_kernel), dim3((unsigned)grid), dim3(bt), args,
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(apply_grid_kernel), dim3((unsigned)grid), dim3(bt), args,
                                        smem, s);
-}
-
-cudaError_t launch_apply(const DevInterner &I, const ApplyArgs &a, int num_sms, cudaStream_t s) {
-    cudaError_t e = launch_apply_bottom(I, a, num_sms, s);
-    if (e != cudaSuccess) return e;
-    return launch_apply_levels(I, a, num_sms, s);
 }
 
 }  // namespace vxg

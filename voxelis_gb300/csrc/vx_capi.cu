@@ -216,7 +216,6 @@ struct vx_interner {
     uint64_t seq_queue_cap = 0;
     unsigned long long *d_live = nullptr;
     int *d_status = nullptr;
-    unsigned long long *scan_status = nullptr;  // kScanStatusTiles look-back words, zero between scans
     // pinned staging
     DevCounters *h_ctr = nullptr;
     int *h_status = nullptr;
@@ -415,64 +414,62 @@ struct Item {
     uint32_t caller_index;
 };
 
-// Words of scan scratch an apply over Rp = R + 1 flags needs (block sums of the per-phase scans, or
-// the per-CTA partial sums of the single-launch path).
-size_t scan_words(vx_interner *it, size_t Rp) {
-    return std::max(scan_tmp_words((uint32_t)Rp) * 4, apply_single_scan_words(it->num_sms));
-}
-
 // Device scratch of one batched apply over n items and R touched groups. With `own_inputs` the
 // item and record input arrays are carved from the workspace too (host-staging path).
-int carve_apply(vx_interner *it, uint32_t n, uint64_t R, bool own_inputs, ApplyArgs &a) {
-    const size_t Rp = R + 1;
-    const size_t in_items = own_inputs ? 1 : 0, in_recs = own_inputs ? 1 : 0;
-    const size_t need = Carve::need({n * 4 * in_items, n, n * in_items, n * 4 * in_items, n * 8, n * 8, n * 8, n,
-                                     n, R * 4 * in_recs, R * 4 * in_recs, R * in_recs, R * in_recs, R * 16 * in_recs,
-                                     Rp * 4, Rp * 4, scan_words(it, Rp) * 4, R * 4, R * 4, R * 4,
-                                     R * 4, R * 8, R * 8, R * 4, R * 4, Rp * 4, R * 8, R * 4, n * 8,
-                                     (n + 1) * 4 * in_items});
-    VX_CUDA(it->ws.reserve(need));
-    Carve c(it->ws.p);
-    a.mode = 0;
-    a.n_items = n;
-    a.n_records = (uint32_t)R;
-    a.threads = it->apply_threads;
-    a.blocks_per_sm = it->apply_blocks_per_sm;
-    if (own_inputs) a.it_tree = c.take<uint32_t>(n);
-    a.it_depth = c.take<uint8_t>(n);
-    if (own_inputs) {
-        a.it_flags = c.take<uint8_t>(n);
-        a.it_fill = c.take<uint32_t>(n);
+int carve_apply(vx_interner *it, uint32_t n, uint64_t R, int max_depth, bool own_inputs, ApplyArgs &a) {
+    // parents of step s: at most one a record, and one a node of the step's level in each tree
+    uint64_t cap[kPlanWords] = {};
+    for (int s = 1; s <= max_depth - 1 && s < kPlanWords; ++s) {
+        const int bits = 3 * (max_depth - 1 - s);
+        cap[s] = R;
+        if (((uint64_t)n << bits) < R) cap[s] = (uint64_t)n << bits;
     }
-    a.it_init = c.take<uint64_t>(n);
-    a.it_old = c.take<uint64_t>(n);
-    a.it_new = c.take<uint64_t>(n);
-    a.it_panic = c.take<uint8_t>(n);
-    a.it_changed = c.take<uint8_t>(n);
-    if (own_inputs) {
-        a.rec_item = c.take<uint32_t>(R);
-        a.rec_group = c.take<uint32_t>(R);
-        a.rec_set = c.take<uint8_t>(R);
-        a.rec_clear = c.take<uint8_t>(R);
-        a.rec_vals = c.take<uint16_t>(R * 8);
-    }
-    a.flags = c.take<uint32_t>(Rp);
-    a.pos = c.take<uint32_t>(Rp);
-    a.scan_tmp = c.take<uint32_t>(scan_words(it, Rp));
-    a.scan_status = it->scan_status;
-    a.e_item[0] = c.take<uint32_t>(R);
-    a.e_item[1] = c.take<uint32_t>(R);
-    a.e_path[0] = c.take<uint32_t>(R);
-    a.e_path[1] = c.take<uint32_t>(R);
-    a.e_id[0] = c.take<uint64_t>(R);
-    a.e_id[1] = c.take<uint64_t>(R);
-    a.e_val[0] = c.take<uint32_t>(R);
-    a.e_val[1] = c.take<uint32_t>(R);
-    a.p_start = c.take<uint32_t>(Rp);
-    a.rec_id = c.take<uint64_t>(R);
-    a.rec_val = c.take<uint32_t>(R);
-    a.release_list = c.take<uint64_t>(n);
-    if (own_inputs) a.it_first = c.take<uint32_t>((size_t)n + 1);
+    const uint32_t ctas = apply_max_ctas(it->num_sms, it->apply_blocks_per_sm);
+    const size_t tiles = (size_t)((R + 31) / 32);
+    auto layout = [&](void *base) {
+        Carve c(base);
+        a.n_items = n;
+        a.n_records = (uint32_t)R;
+        a.max_depth = max_depth;
+        a.threads = it->apply_threads;
+        a.blocks_per_sm = it->apply_blocks_per_sm;
+        a.it_depth = c.take<uint8_t>(n);
+        a.it_init = c.take<uint64_t>(n);
+        a.it_old = c.take<uint64_t>(n);
+        a.it_panic = c.take<uint8_t>(n);
+        a.it_changed = c.take<uint8_t>(n);
+        a.release_list = c.take<uint64_t>(n);
+        if (own_inputs) {
+            a.it_tree = c.take<uint32_t>(n);
+            a.it_flags = c.take<uint8_t>(n);
+            a.it_fill = c.take<uint32_t>(n);
+            a.rec_item = c.take<uint32_t>(R);
+            a.rec_group = c.take<uint32_t>(R);
+            a.rec_set = c.take<uint8_t>(R);
+            a.rec_clear = c.take<uint8_t>(R);
+            a.rec_vals = c.take<uint16_t>(R * 8);
+            a.it_first = c.take<uint32_t>((size_t)n + 1);
+        }
+        a.part = c.take<uint32_t>((size_t)kPlanWords * ctas);
+        a.warp_off = c.take<uint32_t>((size_t)kPlanWords * ctas * 16);
+        a.level_n = c.take<uint32_t>(kPlanWords);
+        a.tile_base = c.take<uint32_t>(tiles * kPlanWords);
+        for (int s = 1; s < kPlanWords; ++s) {
+            a.p_cap[s] = (uint32_t)cap[s];
+            a.p_rec[s] = c.take<uint32_t>(cap[s]);
+            a.p_start[s] = c.take<uint32_t>(cap[s]);
+            a.p_old[s] = c.take<uint64_t>(cap[s]);
+        }
+        a.rec_id = c.take<uint64_t>(R);
+        a.rec_val = c.take<uint32_t>(R);
+        for (int k = 0; k < 2; ++k) {  // entries of odd steps, of even ones
+            a.e_id[k] = c.take<uint64_t>(cap[k ? 1 : 2]);
+            a.e_val[k] = c.take<uint32_t>(cap[k ? 1 : 2]);
+        }
+        return c.off;
+    };
+    VX_CUDA(it->ws.reserve(layout(nullptr) + 256));
+    layout(it->ws.p);
     return VX_OK;
 }
 
@@ -489,16 +486,10 @@ int apply_sequence(vx_interner *it, ApplyArgs &a, bool clear_pass, bool check_de
                                     rounds, it->num_sms, s));
         return VX_OK;
     }
-    if (check_depths) VX_CUDA(launch_item_depths(it->dev, a, s));
     for (int mode = 0; mode < (clear_pass ? 2 : 1); ++mode) {
-        a.mode = mode;
         {
-            Phase ph(it, VX_PROF_BOTTOM);
-            VX_CUDA(launch_apply_bottom(it->dev, a, it->num_sms, s));
-        }
-        {
-            Phase ph(it, VX_PROF_APPLY);
-            VX_CUDA(launch_apply_levels(it->dev, a, it->num_sms, s));
+            PhaseSwitch ps(it, VX_PROF_BOTTOM, VX_PROF_APPLY);
+            VX_CUDA(launch_apply(it->dev, a, mode, check_depths, it->num_sms, s, &PhaseSwitch::next, &ps));
         }
         {
             Phase ph(it, VX_PROF_RELEASE);
@@ -618,9 +609,8 @@ int run_apply(vx_interner *it, std::vector<Item> items, uint8_t *changed_out) {
     };
 
     ApplyArgs a{};
-    int st0 = carve_apply(it, n, R, true, a);
+    int st0 = carve_apply(it, n, R, max_depth, true, a);
     if (st0 != VX_OK) return st0;
-    a.max_depth = max_depth;
     cudaStream_t s = it->stream;
     VX_CUDA(cudaMemcpyAsync((void *)a.it_tree, it_tree, n * 4, cudaMemcpyHostToDevice, s));
     VX_CUDA(cudaMemcpyAsync((void *)a.it_depth, it_depth, n, cudaMemcpyHostToDevice, s));
@@ -833,8 +823,6 @@ int vx_interner_create(uint64_t budget_bytes, int voxel_bits, uint32_t patch_fla
     alloc((void **)&it->frontier, 2 * cap * 4 + 64);
     alloc((void **)&it->d_live, 2 * sizeof(unsigned long long));
     alloc((void **)&it->d_status, sizeof(int) * 4);
-    alloc((void **)&it->scan_status, (size_t)kScanStatusTiles * 8);
-    if (ok && cudaMemset(it->scan_status, 0, (size_t)kScanStatusTiles * 8) != cudaSuccess) ok = false;
     if (patch_flags & VX_PATCH_P3) {
         it->seq_queue_cap = std::max<uint64_t>(cap + 1, 32768);
         alloc((void **)&it->seq_queue, it->seq_queue_cap * 8);
@@ -876,8 +864,7 @@ int vx_interner_destroy(vx_interner *it) {
     if (it->stream) cudaStreamSynchronize(it->stream);
     DevInterner &D = it->dev;
     void *ptrs[] = {D.children, D.values, D.refcount, D.generation, D.hash, D.ids, D.free_list, D.ctr, D.table,
-                    D.leaf_table, D.roots, D.depths, it->frontier, it->seq_queue, it->d_live, it->d_status,
-                    it->scan_status};
+                    D.leaf_table, D.roots, D.depths, it->frontier, it->seq_queue, it->d_live, it->d_status};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     it->ws.release();
@@ -1297,7 +1284,7 @@ int vx_apply_groups_async(vx_interner *it, uint32_t n_items, const vx_tree *tree
     it->all_trees_unknown = true;
     if (n_items == 0) return VX_OK;
     ApplyArgs a{};
-    int st = carve_apply(it, n_items, n_records, false, a);
+    int st = carve_apply(it, n_items, n_records, max_depth, false, a);
     if (st != VX_OK) return st;
     a.it_tree = trees_dev;
     a.it_flags = item_flags_dev;
@@ -1307,7 +1294,6 @@ int vx_apply_groups_async(vx_interner *it, uint32_t n_items, const vx_tree *tree
     a.rec_set = rec_set_dev;
     a.rec_clear = rec_clear_dev;
     a.rec_vals = rec_values_dev;
-    a.max_depth = max_depth;
     st = apply_sequence(it, a, (it->flags & VX_PATCH_P4) != 0, true);
     if (st != VX_OK) return st;
     if (changed_dev) VX_CUDA(cudaMemcpyAsync(changed_dev, a.it_changed, n_items, cudaMemcpyDeviceToDevice, it->stream));

@@ -69,8 +69,8 @@ struct DevCounters {
     unsigned int error_info;         // first error detail
     unsigned long long scratch[10];  // per-launch counters used by the kernels
     unsigned long long created;      // nodes allocated since the interner was created or reset
-    unsigned long long bar_count;    // grid barrier of single-launch kernels: CTAs arrived
-    unsigned long long bar_gen;      //   and the barrier's generation
+    unsigned long long bar_count;    // grid barrier of single-launch kernels: arrivals, only growing
+    unsigned long long bar_gen;      //   and their number when the next launch starts
     unsigned long long rel_count[3]; // dying-set sizes of single-launch release rounds (rotating)
 };
 
@@ -543,42 +543,6 @@ __device__ __forceinline__ void recycle_node(const DevInterner &I, uint32_t idx,
     I.ids[idx] = 0;
     I.generation[idx] = (uint16_t)(gen + 1u >= MAX_GENERATION ? 0u : gen + 1u);
     I.free_list[free_pos] = idx;
-}
-
-// ---- grid barrier of single-launch (cooperative) kernels -------------------------------------------
-// Every CTA of the grid must call it (all CTAs are resident: cooperative launch). Thread 0 arrives
-// with a fence and waits, bounded, for the generation to move; the last to arrive resets the count
-// and moves the generation with release semantics. Writes before the barrier are visible to every
-// thread of the grid after it. Returns false if the wait gave up (ERR_TIMEOUT recorded).
-__device__ __forceinline__ bool grid_sync(const DevInterner &I) {
-    __shared__ int ok_s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        const unsigned long long gen = ld_acquire(reinterpret_cast<const uint64_t *>(&I.ctr->bar_gen));
-        __threadfence();
-        if (atomicAdd(&I.ctr->bar_count, 1ull) == gridDim.x - 1) {
-            I.ctr->bar_count = 0;
-            st_release_u64(&I.ctr->bar_gen, gen + 1);
-        } else {
-            uint32_t spin = 0;
-            while (ld_acquire(reinterpret_cast<const uint64_t *>(&I.ctr->bar_gen)) == gen) {
-                // a CTA that gave up at an earlier barrier never arrives: stop waiting at once
-                const bool gave_up = (spin & 1023u) == 1023u &&
-                                     (*reinterpret_cast<volatile unsigned int *>(&I.ctr->error) & ERR_TIMEOUT);
-                if (++spin >= I.spin_limit || gave_up) {
-                    set_error(I, ERR_TIMEOUT, 49);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(32);
-            }
-        }
-        __threadfence();
-        ok_s = ok;
-    }
-    __syncthreads();
-    return ok_s != 0;
 }
 
 // ---- release (dec_ref_recursive, interner/mod.rs:419-534, breadth first) ------------------------

@@ -82,9 +82,10 @@ cudaError_t launch_expand_items(const uint32_t *first, uint32_t n, uint32_t *rec
 
 
 // ---- general batch apply (vx_apply.cu) ---------------------------------------------------------
+constexpr int kPlanWords = 12;        // counts of the plan: records with clear bits, then one per step (1 .. 11)
+constexpr uint32_t kApplyCluster = 8;  // CTAs of a small apply, which runs as one cluster
 struct ApplyArgs {
-    int mode;                    // 0: set phase (set_batch_at_depth_iterative); 1: clear pass (P4)
-    int threads;                 // launch shape of the bottom/parents kernels
+    int threads;                 // launch shape of the kernels
     int blocks_per_sm;
     uint32_t n_items;
     uint32_t n_records;
@@ -96,7 +97,6 @@ struct ApplyArgs {
     const uint32_t *it_fill;
     uint64_t *it_init;           // scratch
     uint64_t *it_old;
-    uint64_t *it_new;
     uint8_t *it_panic;
     uint8_t *it_changed;         // result
     // records sorted by (item, group)
@@ -105,48 +105,39 @@ struct ApplyArgs {
     const uint8_t *rec_set;
     const uint8_t *rec_clear;
     const uint16_t *rec_vals;    // [n_records * 8]
-    // scratch
-    uint32_t *flags;             // [n_records + 1]
-    uint32_t *pos;               // [n_records + 1]
-    uint32_t *scan_tmp;          // block sums
-    unsigned long long *scan_status;  // [kScanStatusTiles] look-back words of one-pass scans (all 0 between scans)
-    uint32_t *e_item[2];
-    uint32_t *e_path[2];
-    uint64_t *e_id[2];
-    uint32_t *e_val[2];
-    uint32_t *p_start;           // [n_records + 1]
-    uint32_t *it_first;           // [n_items + 1] first record of each item (host staging of an apply)
+    // scratch: the plan
+    uint32_t *part;              // [kPlanWords][CTAs] counts of the CTAs' ranges
+    uint32_t *warp_off;          // [CTAs * warps][kPlanWords] counts before a warp's tiles in its range
+    uint32_t *tile_base;         // [tiles of 32 records][kPlanWords] counts before a tile in its warp's
+    uint32_t *level_n;           // [kPlanWords] totals (separate launches)
+    // parents of step s, the nodes s levels above the bottom groups: room for p_cap[s] of them
+    uint32_t p_cap[kPlanWords];
+    uint32_t *p_rec[kPlanWords];    // first record under it
+    uint32_t *p_start[kPlanWords];  // its first child among the entries of step s - 1 (records for s = 1)
+    uint64_t *p_old[kPlanWords];    // the old tree's node at its place
+    // results: of the records, and of the parents of the last two steps
     uint64_t *rec_id;
     uint32_t *rec_val;
+    uint64_t *e_id[2];
+    uint32_t *e_val[2];
+    uint32_t *it_first;          // [n_items + 1] first record of each item (host staging of an apply)
     uint64_t *release_list;      // [n_items]
 };
-cudaError_t launch_apply(const DevInterner &I, const ApplyArgs &a, int num_sms, cudaStream_t s);
-// The same sequence (with the item depth check when check_depths, the clear pass when clear_pass and
-// the release of the replaced roots in `rounds` rounds) as one cooperative launch: every CTA
-// resident, phases separated by grid barriers. a.scan_tmp must hold apply_single_scan_words words.
+// Most CTAs of a launch (sizes part and warp_off).
+uint32_t apply_max_ctas(int num_sms, int blocks_per_sm);
+// The set phase (mode 0, with the item depth check when check_depths) or the clear pass (mode 1) in one
+// launch per phase; the caller releases the replaced roots. levels_begin(levels_ctx), when given, runs on
+// the host between the bottom groups' launch and the levels' (the profiler marks its phases there).
+cudaError_t launch_apply(const DevInterner &I, const ApplyArgs &a, int mode, bool check_depths, int num_sms, cudaStream_t s,
+                         void (*levels_begin)(void *) = nullptr, void *levels_ctx = nullptr);
+// The same sequence (with the clear pass when clear_pass and the release of the replaced roots in `rounds`
+// rounds) as one launch whose phases are separated by barriers.
 cudaError_t launch_apply_single(const DevInterner &I, const ApplyArgs &a, bool check_depths, bool clear_pass,
                                 uint32_t *frontier_a, uint32_t *frontier_b, int rounds, int num_sms, cudaStream_t s);
-size_t apply_single_scan_words(int num_sms);
-// The same sequence in two parts: items + bottom groups, then the level passes and the commit.
-cudaError_t launch_apply_bottom(const DevInterner &I, const ApplyArgs &a, int num_sms, cudaStream_t s);
-cudaError_t launch_apply_levels(const DevInterner &I, const ApplyArgs &a, int num_sms, cudaStream_t s);
-// Fills it_depth from the tree table and checks the deepest-first order (device-resident inputs).
-cudaError_t launch_item_depths(const DevInterner &I, const ApplyArgs &a, cudaStream_t s);
-// Counter slots used by launch_apply (DevCounters::scratch indices).
-enum : int {
-    SC_ENTRIES = 0, SC_PARENTS = 1, SC_ROOTS = 2, SC_RELEASE = 3, SC_REL_IN = 4, SC_REL_OUT = 5, SC_REF_DONE = 6,
-    SC_DONE = 7, SC_SCAN_TICKET = 8, SC_SCAN_DONE = 9
-};
+// Counter slots (DevCounters::scratch indices).
+enum : int { SC_RELEASE = 3, SC_REL_IN = 4, SC_REL_OUT = 5, SC_REF_DONE = 6, SC_DONE = 7 };
 static_assert(SC_RELEASE == kScRelease && SC_REL_IN == kScRelIn && SC_REL_OUT == kScRelOut,
               "release slots shared with vx_device.cuh");
-// Tiles of a one-pass device scan with a status word each (ApplyArgs::scan_status, zero between
-// scans: the scan's last CTA clears them); larger scans take the three-launch path.
-constexpr uint32_t kScanStatusTiles = 64;
-
-// Inclusive-to-exclusive scan of n u32 flags (n from the host) into pos; pos[n] = total.
-cudaError_t launch_scan(const uint32_t *flags, uint32_t *pos, uint32_t *tmp, uint32_t n, cudaStream_t s);
-// Block sums of one scan level; `tmp` must hold 4 x scan_tmp_words(n) words for the recursion.
-size_t scan_tmp_words(uint32_t n);
 
 // ---- reads, releases, single-voxel operations, maintenance (vx_ops.cu) -------------------------
 cudaError_t launch_get_many(const DevInterner &I, uint64_t n, const uint32_t *trees, const int32_t *xyz,
