@@ -207,7 +207,7 @@ __device__ __forceinline__ void finish_item(const DevInterner &I, const ApplyArg
 // ---- the plan of the levels ------------------------------------------------------------------------
 // Records are taken in tiles of 32 (one warp). The CTAs of the grid own contiguous ranges of tiles, their
 // warps contiguous parts of a range. Word 0 of a count is the records with clear bits, word s the records
-// that head step s; lane s of a warp keeps word s.
+// that head step s, word kRootWord + s the items whose root is made at step s; lane s of a warp keeps word s.
 struct Tiles {
     uint32_t lo, hi;  // this warp's tiles
     uint32_t woff;    // its place in ApplyArgs::warp_off
@@ -226,23 +226,26 @@ __device__ __forceinline__ Tiles warp_tiles(const ApplyArgs &a) {
 }
 
 // Steps that record r (of item i and group g, depth d) heads: 1 .. the result. Whole warp, lanes in order.
-__device__ __forceinline__ uint32_t head_steps(const ApplyArgs &a, uint64_t r, bool in, uint32_t i, uint32_t g, int d) {
+__device__ __forceinline__ uint32_t head_steps(const ApplyArgs &a, uint64_t r, bool in, uint32_t i, uint32_t g, int d,
+                                               bool *first = nullptr) {
     uint32_t ip = __shfl_up_sync(0xFFFFFFFFu, i, 1), gp = __shfl_up_sync(0xFFFFFFFFu, g, 1);
     if (!in) return 0;
     const uint32_t top = (uint32_t)d - 1u;
-    if (r == 0) return top;
-    if ((threadIdx.x & 31u) == 0) {
+    if ((threadIdx.x & 31u) == 0 && r > 0) {
         ip = a.rec_item[r - 1];
         gp = a.rec_group[r - 1];
     }
-    if (ip != i) return top;
+    if (r == 0 || ip != i) {
+        if (first) *first = true;
+        return top;
+    }
     const uint32_t x = g ^ gp, s = x ? (31u - __clz(x)) / 3u : 0u;
     return s < top ? s : top;
 }
 
-// Counts of this CTA's range (all threads of the CTA call it; cnt_s: kPlanWords words a warp).
+// Counts of this CTA's range (all threads of the CTA call it; cnt_s: kPartWords words a warp).
 __device__ __forceinline__ void plan_count(const DevInterner &I, const ApplyArgs &a, bool check_depths,
-                                           uint32_t (*cnt_s)[kPlanWords]) {
+                                           uint32_t (*cnt_s)[kPartWords]) {
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const Tiles t = warp_tiles(a);
     uint32_t acc = 0;  // word `lane`, over this warp's tiles so far
@@ -251,8 +254,14 @@ __device__ __forceinline__ void plan_count(const DevInterner &I, const ApplyArgs
         const bool in = r < a.n_records;
         const uint32_t i = in ? a.rec_item[r] : 0u, g = in ? a.rec_group[r] : 0u;
         const int d = in ? item_depth_of(I, a, i, check_depths) : 2;
-        const uint32_t hs = head_steps(a, r, in, i, g, d);
+        bool first = false;
+        const uint32_t hs = head_steps(a, r, in, i, g, d, &first);
         if (lane < kPlanWords) a.tile_base[(uint64_t)tile * kPlanWords + lane] = acc;
+        // the first record of an item heads every step up to its root's
+        for (unsigned h = __ballot_sync(0xFFFFFFFFu, first); h; h &= h - 1) {
+            const uint32_t root_step = __shfl_sync(0xFFFFFFFFu, hs, __ffs(h) - 1);
+            if (lane == kRootWord + root_step) ++acc;
+        }
         const unsigned cl = __ballot_sync(0xFFFFFFFFu, in && a.rec_clear[r] != 0);
         if (lane == 0) acc += __popc(cl);
         const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, hs);
@@ -261,12 +270,12 @@ __device__ __forceinline__ void plan_count(const DevInterner &I, const ApplyArgs
             if (lane == s) acc += __popc(b);
         }
     }
-    if (lane < kPlanWords) cnt_s[warp][lane] = acc;
+    if (lane < kPartWords) cnt_s[warp][lane] = acc;
     __syncthreads();
-    if (threadIdx.x < kPlanWords) {  // the warps' places in the range, and its sums
+    if (threadIdx.x < kPartWords) {  // the warps' places in the range, and its sums
         uint32_t run = 0;
         for (uint32_t w = 0; w < nw; ++w) {
-            a.warp_off[(blockIdx.x * nw + w) * kPlanWords + threadIdx.x] = run;
+            if (threadIdx.x < kPlanWords) a.warp_off[(blockIdx.x * nw + w) * kPlanWords + threadIdx.x] = run;
             run += cnt_s[w][threadIdx.x];
         }
         a.part[threadIdx.x * gridDim.x + blockIdx.x] = run;
@@ -276,13 +285,21 @@ __device__ __forceinline__ void plan_count(const DevInterner &I, const ApplyArgs
 
 struct Plan {
     uint32_t base[kPlanWords];   // counts of the ranges before this CTA's
-    uint32_t total[kPlanWords];  // counts of all ranges, no more than a step's room
+    uint32_t total[kPartWords];  // counts of all ranges, no more than a step's room
 };
+
+// Entries of step s - 1 (records for s = 1) that have a parent at step s: all but the roots, which are the
+// tail of the list.
+__device__ __forceinline__ uint32_t plan_children(const ApplyArgs &a, const uint32_t *total, uint32_t s) {
+    if (s == 1) return a.n_records;
+    const uint32_t n = total[s - 1], roots = total[kRootWord + s - 1];
+    return n > roots ? n - roots : 0;
+}
 
 // After every CTA's plan_count. All threads of the CTA call it.
 __device__ __forceinline__ void plan_totals(const ApplyArgs &a, Plan &P) {
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (uint32_t s = warp; s < kPlanWords; s += nw) {
+    for (uint32_t s = warp; s < kPartWords; s += nw) {
         uint32_t before = 0, all = 0;
         for (uint32_t c = lane; c < gridDim.x; c += 32) {
             const uint32_t v = a.part[s * gridDim.x + c];
@@ -292,8 +309,8 @@ __device__ __forceinline__ void plan_totals(const ApplyArgs &a, Plan &P) {
         before = __reduce_add_sync(0xFFFFFFFFu, before);
         all = __reduce_add_sync(0xFFFFFFFFu, all);
         if (lane == 0) {
-            P.base[s] = before;
-            P.total[s] = s > 0 && all > a.p_cap[s] ? a.p_cap[s] : all;
+            if (s < kPlanWords) P.base[s] = before;
+            P.total[s] = s > 0 && s < kPlanWords && all > a.p_cap[s] ? a.p_cap[s] : all;
         }
     }
     __syncthreads();
@@ -489,7 +506,7 @@ __device__ __forceinline__ void bottom_records(const DevInterner &I, const Apply
 }
 
 // ---- Phase 2 -----------------------------------------------------------------------------------------
-// Parents cta_base + threadIdx.x, + stride, ... of step s (n_par of them, their children are the n_child
+// Parents cta_base + threadIdx.x, + stride, ... of step s (n_par of them, their children are the first n_child
 // entries of step s - 1). A CTA-uniform loop: whole warps take part in the warp-cooperative interning.
 __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyArgs &a, int mode, const LeafRefs &L,
                                               uint32_t s, uint32_t n_par, uint32_t n_child, uint64_t cta_base, uint64_t stride) {
@@ -511,23 +528,29 @@ __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyA
             const uint32_t b = a.p_start[s][p];
             uint32_t e = p + 1 < n_par ? a.p_start[s][p + 1] : n_child;
             if (e > n_child) e = n_child;
-            const bool last = p + 1 == n_par;  // its run ends where its item's entries do
-            // gather the run of changed children (voxtree.rs:959-1000); slots by select, so that the
-            // arrays stay in registers
-            for (uint32_t j = b; j < e; ++j) {
-                if (last && a.rec_item[s == 1 ? j : a.p_rec[s - 1][j]] != i) break;
-                const uint32_t ev = in_val[j];
-                if (!(ev & kChanged)) continue;
-                const uint32_t ti = (ev >> 16) & 7u;
-                const uint64_t id = in_id[j];
+            // gather the run of changed children (voxtree.rs:959-1000), four loads in flight; slots by
+            // select, so that the arrays stay in registers
+            for (uint32_t j0 = b; j0 < e; j0 += 4) {
+                uint32_t ev[4];
+                uint64_t id[4];
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    if ((uint32_t)k == ti) {
-                        c[k] = id;
-                        cv[k] = ev & 0xFFFFu;
-                    }
-                types |= (id_is_leaf(id) ? 1u : 0u) << ti;
-                mask |= 1u << ti;
+                for (int q = 0; q < 4; ++q) {
+                    ev[q] = j0 + q < e ? in_val[j0 + q] : 0u;
+                    id[q] = j0 + q < e ? in_id[j0 + q] : 0ull;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (!(ev[q] & kChanged)) continue;
+                    const uint32_t ti = (ev[q] >> 16) & 7u;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        if ((uint32_t)k == ti) {
+                            c[k] = id[q];
+                            cv[k] = ev[q] & 0xFFFFu;
+                        }
+                    types |= (id_is_leaf(id[q]) ? 1u : 0u) << ti;
+                    mask |= 1u << ti;
+                }
             }
             changed = mask != 0;
         }
@@ -644,7 +667,7 @@ __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyA
 // ---- phases of an apply ------------------------------------------------------------------------------
 // Set phase: depths, Phase 0 and the counts of the plan. All threads of the grid.
 __device__ __forceinline__ void phase_plan(const DevInterner &I, const ApplyArgs &a, bool check_depths,
-                                           uint32_t (*cnt_s)[kPlanWords]) {
+                                           uint32_t (*cnt_s)[kPartWords]) {
     const uint64_t gt = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
     if (gt == 0) I.ctr->scratch[SC_RELEASE] = 0;
     for (uint64_t i = gt; i < a.n_items; i += stride) {
@@ -674,7 +697,7 @@ constexpr int kMaxApplyWarps = 16;  // 512 threads
 __global__ void __launch_bounds__(512) apply_plan_kernel(DevInterner I, ApplyArgs a, int check_depths) {
     pdl_wait();
     pdl_release();
-    __shared__ uint32_t cnt_s[kMaxApplyWarps][kPlanWords];
+    __shared__ uint32_t cnt_s[kMaxApplyWarps][kPartWords];
     phase_plan(I, a, check_depths != 0, cnt_s);
 }
 
@@ -683,7 +706,7 @@ __global__ void __launch_bounds__(512, VX_APPLY_MIN_BLOCKS) apply_bottom_kernel(
     pdl_release();
     __shared__ Plan P;
     plan_totals(a, P);
-    if (blockIdx.x == 0 && threadIdx.x < kPlanWords) a.level_n[threadIdx.x] = P.total[threadIdx.x];
+    if (blockIdx.x == 0 && threadIdx.x < kPartWords) a.level_n[threadIdx.x] = P.total[threadIdx.x];
     if (mode == 1 && blockIdx.x == 0 && threadIdx.x == 0) I.ctr->scratch[SC_RELEASE] = 0;
     if (mode == 0 || P.total[0]) {
         const LeafRefs L = leaf_refs_init(I);
@@ -699,7 +722,7 @@ __global__ void __launch_bounds__(512, VX_APPLY_MIN_BLOCKS) apply_parents_kernel
     pdl_release();
     if (mode == 0 || a.level_n[0]) {
         const LeafRefs L = leaf_refs_init(I);
-        parents_range(I, a, mode, L, s, a.level_n[s], s == 1 ? a.n_records : a.level_n[s - 1],
+        parents_range(I, a, mode, L, s, a.level_n[s], plan_children(a, a.level_n, s),
                       (uint64_t)blockIdx.x * blockDim.x, (uint64_t)gridDim.x * blockDim.x);
         leaf_refs_flush(I, L);
     }
@@ -767,7 +790,7 @@ template <class Barrier>
 __device__ __forceinline__ void apply_single(const DevInterner &I, const ApplyArgs &a, int check_depths, int clear_pass,
                                              uint32_t *frontier_a, uint32_t *frontier_b, int rounds) {
     extern __shared__ uint32_t leaf_smem[];
-    __shared__ uint32_t cnt_s[kMaxApplyWarps][kPlanWords];
+    __shared__ uint32_t cnt_s[kMaxApplyWarps][kPartWords];
     __shared__ Plan P;
     const uint64_t cta_base = (uint64_t)blockIdx.x * blockDim.x, stride = (uint64_t)gridDim.x * blockDim.x;
     const bool t0 = cta_base + threadIdx.x == 0;
@@ -786,7 +809,7 @@ __device__ __forceinline__ void apply_single(const DevInterner &I, const ApplyAr
         phase_bottom(I, a, mode, L, P);
         if (!bar.sync()) return;
         for (int s = 1; s <= a.max_depth - 1 && a.n_records; ++s) {
-            parents_range(I, a, mode, L, s, P.total[s], s == 1 ? a.n_records : P.total[s - 1], cta_base, stride);
+            parents_range(I, a, mode, L, s, P.total[s], plan_children(a, P.total, s), cta_base, stride);
             if (s == a.max_depth - 1) leaf_refs_flush(I, L);
             if (!bar.sync()) return;
         }

@@ -450,9 +450,9 @@ int carve_apply(vx_interner *it, uint32_t n, uint64_t R, int max_depth, bool own
             a.rec_vals = c.take<uint16_t>(R * 8);
             a.it_first = c.take<uint32_t>((size_t)n + 1);
         }
-        a.part = c.take<uint32_t>((size_t)kPlanWords * ctas);
+        a.part = c.take<uint32_t>((size_t)kPartWords * ctas);
         a.warp_off = c.take<uint32_t>((size_t)kPlanWords * ctas * 16);
-        a.level_n = c.take<uint32_t>(kPlanWords);
+        a.level_n = c.take<uint32_t>(kPartWords);
         a.tile_base = c.take<uint32_t>(tiles * kPlanWords);
         for (int s = 1; s < kPlanWords; ++s) {
             a.p_cap[s] = (uint32_t)cap[s];

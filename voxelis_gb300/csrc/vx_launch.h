@@ -82,7 +82,8 @@ cudaError_t launch_expand_items(const uint32_t *first, uint32_t n, uint32_t *rec
 
 
 // ---- general batch apply (vx_apply.cu) ---------------------------------------------------------
-constexpr int kPlanWords = 12;        // counts of the plan: records with clear bits, then one per step (1 .. 11)
+constexpr int kPlanWords = 12;        // counts of the plan: records with clear bits, then parents per step (1 .. 11)
+constexpr int kRootWord = 12, kPartWords = 24;  // and after them the roots per step
 constexpr uint32_t kApplyCluster = 8;  // CTAs of a small apply, which runs as one cluster
 struct ApplyArgs {
     int threads;                 // launch shape of the kernels
@@ -106,10 +107,10 @@ struct ApplyArgs {
     const uint8_t *rec_clear;
     const uint16_t *rec_vals;    // [n_records * 8]
     // scratch: the plan
-    uint32_t *part;              // [kPlanWords][CTAs] counts of the CTAs' ranges
+    uint32_t *part;              // [kPartWords][CTAs] counts of the CTAs' ranges
     uint32_t *warp_off;          // [CTAs * warps][kPlanWords] counts before a warp's tiles in its range
     uint32_t *tile_base;         // [tiles of 32 records][kPlanWords] counts before a tile in its warp's
-    uint32_t *level_n;           // [kPlanWords] totals (separate launches)
+    uint32_t *level_n;           // [kPartWords] totals (separate launches)
     // parents of step s, the nodes s levels above the bottom groups: room for p_cap[s] of them
     uint32_t p_cap[kPlanWords];
     uint32_t *p_rec[kPlanWords];    // first record under it
