@@ -730,48 +730,6 @@ __global__ void __launch_bounds__(512, VX_APPLY_MIN_BLOCKS) apply_parents_kernel
 }
 
 // ---- the whole apply in one launch ---------------------------------------------------------------------
-// Barrier of all threads of the launch; writes before it are visible to all after it. sync() returns
-// false when its bounded wait gave up (ERR_TIMEOUT recorded).
-// Grid: a cooperative launch (every CTA resident). Thread 0 of each CTA adds one to a counter that only
-// grows and waits for it to reach the barrier's number of arrivals: one round trip after the last arrival.
-// The counter's value at the start of a launch is kept beside it, and moved by the first CTA as it leaves
-// (every CTA has read it by then).
-struct GridBarrier {
-    const DevInterner &I;
-    unsigned long long target;
-    __device__ explicit GridBarrier(const DevInterner &i) : I(i), target(*(volatile unsigned long long *)&i.ctr->bar_gen) {}
-    // After a barrier that gave up the arrivals are out of step until the interner is reset.
-    __device__ bool usable() { return !(*reinterpret_cast<volatile unsigned int *>(&I.ctr->error) & ERR_TIMEOUT); }
-    __device__ bool sync() {
-        __shared__ int ok_s;
-        target += gridDim.x;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int ok = 1;
-            __threadfence();
-            atomicAdd(&I.ctr->bar_count, 1ull);
-            for (uint32_t spin = 0; (long long)(ld_acquire(reinterpret_cast<const uint64_t *>(&I.ctr->bar_count)) - target) < 0;) {
-                // a CTA that gave up at an earlier barrier never arrives: stop waiting at once
-                const bool gave_up = (spin & 1023u) == 1023u &&
-                                     (*reinterpret_cast<volatile unsigned int *>(&I.ctr->error) & ERR_TIMEOUT);
-                if (++spin >= I.spin_limit || gave_up) {
-                    set_error(I, ERR_TIMEOUT, 49);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(20);
-            }
-            __threadfence();
-            ok_s = ok;
-        }
-        __syncthreads();
-        return ok_s != 0;
-    }
-    __device__ void leave() {
-        if (blockIdx.x == 0 && threadIdx.x == 0) I.ctr->bar_gen = target;
-    }
-};
-
 // One cluster: its hardware barrier.
 struct ClusterBarrier {
     __device__ explicit ClusterBarrier(const DevInterner &) {}
@@ -802,7 +760,7 @@ __device__ __forceinline__ void apply_single(const DevInterner &I, const ApplyAr
     plan_totals(a, P);
     for (int mode = 0; mode <= clear_pass && (mode == 0 || P.total[0]); ++mode) {
         const LeafRefs L = leaf_refs_init(I);
-        if (t0) {
+        if (t0) {  // (nothing reads them before the barrier after the last level)
             ctr->rel_count[0] = ctr->rel_count[1] = ctr->rel_count[2] = 0;
             if (mode == 1) ctr->scratch[SC_RELEASE] = 0;
         }
@@ -828,6 +786,7 @@ __device__ __forceinline__ void apply_single(const DevInterner &I, const ApplyAr
             if (!bar.sync()) return;
         }
     }
+    if (t0) ctr->rel_count[0] = ctr->rel_count[1] = ctr->rel_count[2] = 0;  // as the release launches expect
     bar.leave();
 }
 

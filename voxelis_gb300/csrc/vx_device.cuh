@@ -71,7 +71,7 @@ struct DevCounters {
     unsigned long long created;      // nodes allocated since the interner was created or reset
     unsigned long long bar_count;    // grid barrier of single-launch kernels: arrivals, only growing
     unsigned long long bar_gen;      //   and their number when the next launch starts
-    unsigned long long rel_count[3]; // dying-set sizes of single-launch release rounds (rotating)
+    unsigned long long rel_count[3]; // dying-set sizes of release rounds (rotating; zero between launches)
 };
 
 struct DevInterner {
@@ -545,16 +545,53 @@ __device__ __forceinline__ void recycle_node(const DevInterner &I, uint32_t idx,
     I.free_list[free_pos] = idx;
 }
 
-// ---- release (dec_ref_recursive, interner/mod.rs:419-534, breadth first) ------------------------
-// Counter slots of the release rounds in DevCounters::scratch (the batched-apply launcher's table
-// lists every slot).
-constexpr int kScRelease = 3, kScRelIn = 4, kScRelOut = 5;
+// ---- barriers of kernels that run in phases ------------------------------------------------------------
+// Barrier of all threads of the launch; writes before it are visible to all after it. sync() returns
+// false when its bounded wait gave up (ERR_TIMEOUT recorded).
+// Grid: a cooperative launch (every CTA resident). Thread 0 of each CTA adds one to a counter that only
+// grows and waits for it to reach the barrier's number of arrivals: one round trip after the last arrival.
+// The counter's value at the start of a launch is kept beside it, and moved by the first CTA as it leaves
+// (every CTA has read it by then).
+struct GridBarrier {
+    const DevInterner &I;
+    unsigned long long target;
+    __device__ explicit GridBarrier(const DevInterner &i) : I(i), target(*(volatile unsigned long long *)&i.ctr->bar_gen) {}
+    // After a barrier that gave up the arrivals are out of step until the interner is reset.
+    __device__ bool usable() { return !(*reinterpret_cast<volatile unsigned int *>(&I.ctr->error) & ERR_TIMEOUT); }
+    __device__ bool sync() {
+        __shared__ int ok_s;
+        target += gridDim.x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int ok = 1;
+            __threadfence();
+            atomicAdd(&I.ctr->bar_count, 1ull);
+            for (uint32_t spin = 0; (long long)(ld_acquire(reinterpret_cast<const uint64_t *>(&I.ctr->bar_count)) - target) < 0;) {
+                // a CTA that gave up at an earlier barrier never arrives: stop waiting at once
+                const bool gave_up = (spin & 1023u) == 1023u &&
+                                     (*reinterpret_cast<volatile unsigned int *>(&I.ctr->error) & ERR_TIMEOUT);
+                if (++spin >= I.spin_limit || gave_up) {
+                    set_error(I, ERR_TIMEOUT, 49);
+                    ok = 0;
+                    break;
+                }
+                __nanosleep(20);
+            }
+            __threadfence();
+            ok_s = ok;
+        }
+        __syncthreads();
+        return ok_s != 0;
+    }
+    __device__ void leave() {
+        if (blockIdx.x == 0 && threadIdx.x == 0) I.ctr->bar_gen = target;
+    }
+};
 
-// The dying set just produced becomes the input of the next round.
-__device__ __forceinline__ void release_advance(const DevInterner &I) {
-    I.ctr->scratch[kScRelIn] = I.ctr->scratch[kScRelOut];
-    I.ctr->scratch[kScRelOut] = 0;
-}
+// ---- release (dec_ref_recursive, interner/mod.rs:419-534, breadth first) ------------------------
+// Counter slot of the listed roots' number in DevCounters::scratch (the batched-apply launcher's table
+// lists every slot).
+constexpr int kScRelease = 3;
 
 __device__ __forceinline__ void push_dying(uint32_t *list, unsigned long long *count, bool push, uint32_t idx) {
     const unsigned m = __ballot_sync(0xFFFFFFFFu, push);

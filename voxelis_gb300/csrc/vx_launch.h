@@ -136,9 +136,8 @@ cudaError_t launch_apply(const DevInterner &I, const ApplyArgs &a, int mode, boo
 cudaError_t launch_apply_single(const DevInterner &I, const ApplyArgs &a, bool check_depths, bool clear_pass,
                                 uint32_t *frontier_a, uint32_t *frontier_b, int rounds, int num_sms, cudaStream_t s);
 // Counter slots (DevCounters::scratch indices).
-enum : int { SC_RELEASE = 3, SC_REL_IN = 4, SC_REL_OUT = 5, SC_REF_DONE = 6, SC_DONE = 7 };
-static_assert(SC_RELEASE == kScRelease && SC_REL_IN == kScRelIn && SC_REL_OUT == kScRelOut,
-              "release slots shared with vx_device.cuh");
+enum : int { SC_RELEASE = 3, SC_REF_DONE = 6, SC_DONE = 7 };
+static_assert(SC_RELEASE == kScRelease, "release slot shared with vx_device.cuh");
 
 // ---- reads, releases, single-voxel operations, maintenance (vx_ops.cu) -------------------------
 cudaError_t launch_get_many(const DevInterner &I, uint64_t n, const uint32_t *trees, const int32_t *xyz,

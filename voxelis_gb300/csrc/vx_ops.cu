@@ -69,26 +69,36 @@ __global__ void __launch_bounds__(kThreads) get_kernel(DevInterner I, uint64_t n
 }
 
 // ---- release (bodies in vx_device.cuh, shared with the single-launch apply) ------------------------
-__global__ void __launch_bounds__(kThreads) release_roots_kernel(DevInterner I, const uint64_t *list,
-                                                                uint32_t *out) {
-    pdl_wait();
-    pdl_release();
-    release_roots_range(I, list, out, &I.ctr->scratch[SC_REL_OUT], (uint64_t)blockIdx.x * blockDim.x,
-                        (uint64_t)gridDim.x * blockDim.x);
-    if (grid_last_cta(&I.ctr->scratch[SC_DONE])) release_advance(I);
-}
-
-__global__ void __launch_bounds__(kThreads) release_round_kernel(DevInterner I, const uint32_t *in, uint32_t *out) {
+// The listed roots and then rounds until no node dies, one cooperative launch with a grid barrier after each
+// (a launch per round, empty ones too, took 18 us a round on the few hundred nodes of a served wave).
+__global__ void __launch_bounds__(kThreads) release_kernel(DevInterner I, const uint64_t *list, uint32_t *frontier_a,
+                                                           uint32_t *frontier_b, int rounds) {
     extern __shared__ uint32_t release_mem[];
+    const uint64_t cta_base = (uint64_t)blockIdx.x * blockDim.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    const bool t0 = cta_base + threadIdx.x == 0;
+    DevCounters *ctr = I.ctr;
+    GridBarrier bar(I);
+    if (!bar.usable()) return;
     const LeafDrops D = leaf_drops_init(I, release_mem);
-    pdl_wait();
-    pdl_release();
-    release_round_range(I, D, in, out, &I.ctr->scratch[SC_REL_IN], &I.ctr->scratch[SC_REL_OUT],
-                        (uint64_t)blockIdx.x * blockDim.x, (uint64_t)gridDim.x * blockDim.x);
-    if (grid_last_cta(&I.ctr->scratch[SC_DONE])) release_advance(I);
+    // the counts are zero between launches: the rounds clear them, and the last one read is empty
+    release_roots_range(I, list, frontier_a, &ctr->rel_count[0], cta_base, stride);
+    if (!bar.sync()) return;
+    uint32_t *fr[2] = {frontier_a, frontier_b};
+    int r = 0;
+    for (; r < rounds; ++r) {
+        if (*(volatile unsigned long long *)&ctr->rel_count[r % 3] == 0) break;  // the same answer in every CTA
+        if (t0) ctr->rel_count[(r + 2) % 3] = 0;
+        release_round_range(I, D, fr[r & 1], fr[(r + 1) & 1], &ctr->rel_count[r % 3], &ctr->rel_count[(r + 1) % 3],
+                            cta_base, stride);
+        if (!bar.sync()) return;
+    }
+    if (t0) {  // set r % 3 was read by every CTA before its last barrier, or is the empty one
+        ctr->rel_count[(r + 1) % 3] = 0;
+        ctr->rel_count[(r + 2) % 3] = 0;
+        if (r == rounds) ctr->rel_count[r % 3] = 0;
+    }
+    bar.leave();
 }
-
-__global__ void release_advance_kernel(DevInterner I) { pdl_wait(); pdl_release(); release_advance(I); }
 
 // ---- single-thread reference-order operations ---------------------------------------------------
 struct Seq {
@@ -496,174 +506,305 @@ __global__ void __launch_bounds__(kSeqThreads) tree_set_kernel(DevInterner I, ui
 // reference's set_at_depth_iterative / remove_at_depth (voxtree.rs:393-706) on the tree's current
 // root, so every node it creates, including the stale types bits of the set path (the old parent's
 // types ORed with the new child's leaf bit, voxtree.rs:513-514), is the node the reference creates.
-// All 32 lanes run the same sequence on the same values (loads of one address are one transaction);
-// lane 0 interns, through the concurrent leaf and branch inserts, and broadcasts. Refcounts are not
-// touched during the calls and nothing is released: every node stays valid until the call ends, and
-// a call that finds a node made by an earlier call gets the same node the reference would recreate.
+// Refcounts are not touched during the calls and nothing is released: every node stays valid until the call
+// ends, and a call that finds a node made by an earlier call gets the same node the reference would recreate.
 // Afterwards the epoch refcount kernel counts one reference per child slot of every created node,
 // the trees take their final roots (+1) and release their first ones, and created nodes that ended
 // unreferenced (the intermediate roots and paths) are released, which leaves the refcounts the
 // reference's per-call inc/dec bookkeeping gives.
-struct WSeq {
-    const DevInterner &I;
-    bool ok;
+//
+// Bound by a call's chain of dependent round trips, so lane L of the warp is level L of the path. The descent
+// leaves the path's rows of 8 children in the lanes; their values are loaded together. Going up, a level is
+// looked up alone until the first new node: every node above it has a child that no key can name yet, so
+// those are created together, a lane each, without comparing keys: one ticket range, and the slots, records
+// and publications side by side. 8192 calls on 64 trees of depth 5: 1610 us, 3070 us when each level was
+// looked up, allocated, written and published before the next.
+struct Level {  // lane L's level of the path
+    uint64_t c[8];   // children of the old node: a branch's, 8 copies of a leaf above it, or EMPTY
+    uint32_t cv[8];  // their values
+    uint64_t node, leaf;  // the branch at this level, or EMPTY and the leaf at or above it
+    uint32_t pi;          // the path's child slot
 };
 
-__device__ __forceinline__ uint64_t wchild(const DevInterner &I, uint64_t id, uint32_t k) {
-    return __ldcg((const unsigned long long *)(I.children + 8ull * id_index(id) + k));
-}
-
-__device__ uint64_t wleaf(WSeq &S, uint32_t v) {
-    uint64_t id = EMPTY_ID;
-    if ((threadIdx.x & 31u) == 0) {
-        bool created;
-        id = intern_leaf(S.I, v, &created);
+// Slot of a new key in the branch table, claimed (BUSY): the first tombstone of its sequence, else its EMPTY
+// slot. find: the key may be there or be created by another warp, whose node is then returned in *id;
+// otherwise no slot can hold it. False (and an error) when the limits end the search.
+__device__ __forceinline__ bool set_claim(const DevInterner &I, bool find, const uint64_t c[8], uint32_t types, uint32_t mask,
+                                          uint64_t h, uint64_t *pos_out, uint64_t *id, bool *reused) {
+    const uint32_t tag = slot_tag(h);
+    uint64_t pos = h & I.table_mask;
+    uint32_t probes = 0, tomb = 0, rounds = 0;
+    for (;;) {
+        uint64_t s = ld_probe(I.table + pos);
+        if (s == SLOT_TOMB && tomb == 0) tomb = probes + 1;
+        if (s == SLOT_EMPTY) {
+            if (tomb) {
+                probes = tomb - 1;
+                pos = (h + probes) & I.table_mask;
+            }
+            const uint64_t free_slot = tomb ? SLOT_TOMB : SLOT_EMPTY;
+            const uint64_t prev = atomicCAS((unsigned long long *)(I.table + pos), free_slot, make_slot(tag, IDX_BUSY));
+            if (prev == free_slot) {
+                *pos_out = pos;
+                *reused = tomb != 0;
+                return true;
+            }
+            s = prev;
+            tomb = 0;
+        }
+        if (find && (uint32_t)(s >> 32) == tag && s != SLOT_TOMB) {
+            if ((uint32_t)s == IDX_BUSY) {  // being written by a warp that waits for nobody
+                if (++rounds > I.round_limit) {
+                    set_error(I, ERR_TIMEOUT, 2);
+                    return false;
+                }
+                __nanosleep(32);
+                continue;
+            }
+            if (key_equal(I, (uint32_t)s, c, types, mask, id)) return true;
+        }
+        pos = (pos + 1) & I.table_mask;
+        if (++probes > I.max_probes) {
+            set_error(I, ERR_TABLE_FULL, 1);
+            return false;
+        }
     }
-    id = __shfl_sync(0xFFFFFFFFu, id, 0);
-    if (id == EMPTY_ID) S.ok = false;
-    return id;
 }
 
-__device__ uint64_t wbranch(WSeq &S, const uint64_t c[8], uint32_t types, uint32_t mask) {
-    uint32_t cv[8];
+// Types and mask of lane L's new node over child `cur` (set: voxtree.rs:500-539; remove: 559-705). Returns
+// false when no node is made: all 8 children are the same leaf (the child stands for it), or none is left
+// (*cur becomes EMPTY).
+__device__ __forceinline__ bool set_level(const Level &P, bool remove, uint64_t *cur, uint32_t *types, uint32_t *mask) {
+    const uint32_t bit = 1u << P.pi, lbit = id_is_leaf(*cur) ? bit : 0u;
+    if (remove) {
+        const uint32_t there = *cur == EMPTY_ID ? 0u : bit;
+        if (P.node == EMPTY_ID) {  // the leaf above, split
+            *types = 0xFFu & ~bit;
+            *mask = (0xFFu & ~bit) | there;
+            return true;
+        }
+        *types = id_types(P.node) & ~bit;
+        *mask = *cur == EMPTY_ID ? id_mask(P.node) & ~bit : id_mask(P.node);
+        if (*mask == 0) *cur = EMPTY_ID;
+        return *mask != 0;
+    }
+    if (P.node != EMPTY_ID) {
+        *types = id_types(P.node) | lbit;
+        *mask = id_mask(P.node) | bit;
+        bool same = *types == 0xFF;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) cv[k] = c[k] ? node_value_cg(S.I, id_index(c[k])) : 0u;
-    bool created;
-    uint64_t id = warp_intern_branch(S.I, (threadIdx.x & 31u) == 0, c, types & 0xFFu, mask & 0xFFu,
-                                     calc_average8(cv), &created);
-    id = __shfl_sync(0xFFFFFFFFu, id, 0);
-    if (id == EMPTY_ID) S.ok = false;
-    return id;
+        for (int k = 0; k < 8; ++k) same = same && ((uint32_t)k == P.pi || P.c[k] == *cur);
+        return !same;
+    }
+    *types = P.leaf == EMPTY_ID ? lbit : (0xFFu & ~bit) | lbit;
+    *mask = P.leaf == EMPTY_ID ? bit : 0xFFu;
+    return true;
 }
 
-// set_at_depth_iterative (voxtree.rs:393-540)
-__device__ uint64_t wset(WSeq &S, uint64_t root, int32_t x, int32_t y, int32_t z, int d, uint32_t voxel) {
-    const DevInterner &I = S.I;
-    uint64_t st_node[11], st_leaf[11];
-    uint32_t st_idx[11];
-    uint64_t cur = root, leaf = EMPTY_ID;
-    int depth = 0;
-    while (depth < d) {
-        const uint32_t index = cidx(x, y, z, depth, d);
-        if (id_is_branch(cur)) {
-            st_node[depth] = cur;
-            st_leaf[depth] = leaf;
-            cur = wchild(I, cur, index);
-        } else {
-            if (node_value_cg(I, id_index(cur)) == voxel) return INVALID_ID;
-            leaf = cur;
-            cur = EMPTY_ID;
-            st_node[depth] = cur;
-            st_leaf[depth] = leaf;
+__device__ __forceinline__ void put_child(Level &P, uint64_t id, uint32_t value) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if ((uint32_t)k == P.pi) {
+            P.c[k] = id;
+            P.cv[k] = value;
         }
-        st_idx[depth] = index;
-        ++depth;
-    }
-    if (id_is_leaf(cur) && node_value_cg(I, id_index(cur)) == voxel) return INVALID_ID;
-    cur = wleaf(S, voxel);
-    while (depth > 0 && S.ok) {
-        --depth;
-        const uint64_t pn = st_node[depth], pl = st_leaf[depth];
-        const uint32_t pi = st_idx[depth];
-        const uint32_t lbit = (id_is_leaf(cur) ? 1u : 0u) << pi;
-        uint64_t br[8];
-        if (pn != EMPTY_ID) {
-            const uint32_t types = id_types(pn) | lbit;
-            for (int k = 0; k < 8; ++k) br[k] = wchild(I, pn, k);
-            br[pi] = cur;
-            bool same = types == 0xFF;
-            for (int k = 0; k < 8; ++k) same = same && br[k] == cur;
-            if (!same) cur = wbranch(S, br, types, id_mask(pn) | (1u << pi));
-        } else if (pl == EMPTY_ID) {
-            for (int k = 0; k < 8; ++k) br[k] = EMPTY_ID;
-            br[pi] = cur;
-            cur = wbranch(S, br, lbit, 1u << pi);
-        } else {
-            for (int k = 0; k < 8; ++k) br[k] = pl;
-            br[pi] = cur;
-            cur = wbranch(S, br, ~(1u << pi) | lbit, 0xFFu);
-        }
-    }
-    return cur;
 }
 
-// remove_at_depth / _branch / _leaf (voxtree.rs:542-706)
-__device__ uint64_t wremove(WSeq &S, uint64_t root, int32_t x, int32_t y, int32_t z, int d) {
-    const DevInterner &I = S.I;
-    uint64_t frames[11];
-    int depth = 0;
-    uint64_t node = root, result = EMPTY_ID;
-    while (id_is_branch(node)) {
-        if (depth >= d) {
-            set_error(I, ERR_REF_PANIC, 80);  // "Branch node at max depth"
-            S.ok = false;
+// One call by one warp: the new root, INVALID_ID when nothing changes; *ok is cleared on an error.
+__device__ uint64_t warp_set(const DevInterner &I, unsigned long long fc, unsigned long long ni, uint64_t root, int32_t x,
+                             int32_t y, int32_t z, int d, uint32_t voxel, bool *ok) {
+    const unsigned lane = threadIdx.x & 31u;
+    const bool remove = voxel == 0;
+    constexpr unsigned kAll = 0xFFFFFFFFu;
+    uint64_t leaf_id = voxel ? ld_volatile(I.leaf_table + voxel) : EMPTY_ID;  // beside the descent's loads
+    Level P;
+    P.node = P.leaf = EMPTY_ID;
+    P.pi = (int)lane < d ? cidx(x, y, z, lane, d) : 0u;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) P.c[k] = EMPTY_ID;
+    uint64_t cur = root, above = EMPTY_ID;  // above: the leaf the path ran into
+    for (int L = 0; L < d; ++L) {
+        if (cur == EMPTY_ID) {
+            if (remove) return INVALID_ID;
+            break;
+        }
+        if (id_is_leaf(cur)) {
+            above = cur;
+            break;
+        }
+        if (remove && !__shfl_sync(kAll, (id_mask(cur) >> P.pi) & 1u, L)) return INVALID_ID;
+        uint64_t next = EMPTY_ID;
+        if ((int)lane == L) {
+            P.node = cur;
+            const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(I.children + 8ull * id_index(cur));
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const ulonglong2 w = __ldcg(src + k);
+                P.c[2 * k] = w.x;
+                P.c[2 * k + 1] = w.y;
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if ((uint32_t)k == P.pi) next = P.c[k];
+        }
+        cur = __shfl_sync(kAll, next, L);
+    }
+    if (remove && above == EMPTY_ID && id_is_branch(cur)) {  // at depth d
+        set_error(I, ERR_REF_PANIC, 80);  // "Branch node at max depth"
+        *ok = false;
+        return INVALID_ID;
+    }
+    // the values of the rows, and whether the voxel has its value already
+    const uint64_t met = above != EMPTY_ID ? above : cur;
+    uint32_t met_value = 0;
+    if (met != EMPTY_ID && id_is_leaf(met)) met_value = node_value_cg(I, id_index(met));
+    if (P.node == EMPTY_ID && (int)lane < d) {
+        P.leaf = above;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) P.c[k] = above;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) P.cv[k] = (P.node != EMPTY_ID && P.c[k] != EMPTY_ID) ? node_value_cg(I, id_index(P.c[k])) : 0u;
+    if (!remove && met != EMPTY_ID && id_is_leaf(met) && met_value == voxel) return INVALID_ID;
+    if (P.leaf != EMPTY_ID) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) P.cv[k] = met_value;
+    }
+    if (voxel && leaf_id <= LEAF_BUSY) {
+        bool created;
+        leaf_id = lane == 0 ? intern_leaf(I, voxel, &created) : EMPTY_ID;
+        leaf_id = __shfl_sync(kAll, leaf_id, 0);
+        if (leaf_id == EMPTY_ID) {
+            *ok = false;
             return INVALID_ID;
         }
-        const uint32_t index = cidx(x, y, z, depth, d);
-        if (!((id_mask(node) >> index) & 1u)) return INVALID_ID;
-        frames[depth] = node;
-        node = wchild(I, node, index);
-        ++depth;
     }
-    for (int k = d - 1; k >= depth && S.ok; --k) {  // remove_at_depth_leaf, built bottom-up
-        const uint32_t index = cidx(x, y, z, k, d);
-        uint64_t ch[8];
-        for (int j = 0; j < 8; ++j) ch[j] = node;
-        ch[index] = result;
-        const uint32_t types = ~(1u << index) | ((id_is_leaf(result) ? 1u : 0u) << index);
-        const uint32_t mask = ~(1u << index) | ((result != EMPTY_ID ? 1u : 0u) << index);
-        result = wbranch(S, ch, types, mask);
-    }
-    while (depth > 0 && S.ok) {  // remove_at_depth_branch on the way up
-        --depth;
-        const uint64_t pn = frames[depth];
-        const uint32_t index = cidx(x, y, z, depth, d);
-        const uint32_t mask = result == EMPTY_ID ? (id_mask(pn) & ~(1u << index)) : id_mask(pn);
-        if (mask == 0) {
-            result = EMPTY_ID;
-            continue;
+    // up to the first new node, a level at a time
+    cur = leaf_id;
+    uint32_t value = voxel;
+    uint64_t pos = 0;
+    bool reused = false;
+    uint64_t h = 0;
+    uint32_t types = 0, mask = 0, lod = 0;
+    int L = d - 1;
+    for (; L >= 0; --L) {
+        int what = 0;  // 0: no node, 1: found, 2: claimed, 3: failed
+        uint64_t id = EMPTY_ID;
+        if ((int)lane == L) {
+            id = cur;
+            if (set_level(P, remove, &id, &types, &mask)) {
+                put_child(P, id, value);
+                lod = calc_average8(P.cv);
+                h = branch_fingerprint(P.c, (types << 8) | mask);
+                id = EMPTY_ID;
+                what = set_claim(I, true, P.c, types, mask, h, &pos, &id, &reused) ? (id != EMPTY_ID ? 1 : 2) : 3;
+            }
         }
-        if (!id_is_branch(result)) {
-            set_error(I, ERR_REF_PANIC, 81);  // "Removing voxel should never produce a leaf node"
-            S.ok = false;
+        what = __shfl_sync(kAll, what, L);
+        if (what == 3) {
+            *ok = false;
             return INVALID_ID;
         }
-        uint64_t br[8];
-        for (int k = 0; k < 8; ++k) br[k] = wchild(I, pn, k);
-        br[index] = result;
-        result = wbranch(S, br, id_types(pn) & ~(1u << index), mask);
+        if (what == 2) break;
+        cur = __shfl_sync(kAll, id, L);
+        value = what == 0 ? (cur == EMPTY_ID ? 0u : value) : __shfl_sync(kAll, lod, L);
     }
-    return result;
+    if (L < 0) return cur;
+    // levels L .. 0 are new nodes: lane j <= L makes level j, tickets bottom up
+    const bool mine = (int)lane <= L;
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(&I.ctr->alloc_count, (unsigned long long)(L + 1));
+    // while the ticket is fetched: types and masks above level L, whose children are branches, and the values
+    if ((int)lane < L) {
+        uint64_t child = 2;  // some branch
+        (void)set_level(P, remove, &child, &types, &mask);
+    }
+    for (int j = L - 1; j >= 0; --j) {
+        const uint32_t below = __shfl_sync(kAll, lod, j + 1);
+        if ((int)lane == j) {
+            put_child(P, EMPTY_ID, below);
+            lod = calc_average8(P.cv);
+        }
+    }
+    base = __shfl_sync(kAll, base & kTicketMask, 0);
+    const unsigned long long t = base + (unsigned long long)(L - (int)lane);
+    const uint32_t idx = mine ? node_for_ticket(I, t, fc, ni) : 0u;
+    if (__any_sync(kAll, mine && idx == NO_NODE)) {
+        if ((int)lane == L) {
+            set_error(I, ERR_OOM, 1);
+            atomicExch((unsigned long long *)(I.table + pos), SLOT_TOMB);
+        }
+        *ok = false;
+        return INVALID_ID;
+    }
+    const uint64_t id = mine ? make_branch_id(idx, slot_generation(I, idx, t >= fc), types, mask) : EMPTY_ID;
+    const uint64_t child = __shfl_down_sync(kAll, id, 1);
+    bool claimed = (int)lane == L, failed = false;
+    if ((int)lane < L) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if ((uint32_t)k == P.pi) P.c[k] = child;
+        h = branch_fingerprint(P.c, (types << 8) | mask);
+        uint64_t other;
+        claimed = set_claim(I, false, P.c, types, mask, h, &pos, &other, &reused);
+        failed = !claimed;
+    }
+    failed = __any_sync(kAll, failed);
+    if (mine && !failed) write_branch(I, idx, P.c, types, mask, h, lod, t >= fc);
+    const unsigned re = __ballot_sync(kAll, mine && claimed && reused && !failed);
+    if (lane == 0 && re) atomicAdd(&I.ctr->alloc_count, (unsigned long long)__popc(re) << kTicketBits);
+    if (mine && claimed) publish_release((unsigned long long *)(I.table + pos), failed ? SLOT_TOMB : make_slot(slot_tag(h), idx));
+    if (failed) {
+        *ok = false;
+        return INVALID_ID;
+    }
+    __syncwarp();  // the next call reads these records in other lanes
+    return __shfl_sync(kAll, id, 0);
 }
 
 // One warp per tree group g: calls [begin[g], begin[g+1]) in call order.
-__global__ void __launch_bounds__(kThreads) trees_set_kernel(DevInterner I, const SetCalls c) {
+__global__ void __launch_bounds__(32) trees_set_kernel(DevInterner I, const SetCalls c) {
     if (blockIdx.x == 0 && threadIdx.x == 0) I.ctr->scratch[SC_RELEASE] = 0;
+    const unsigned lane = threadIdx.x & 31u;
     const uint32_t warps = gridDim.x * (blockDim.x / 32);
+    const unsigned long long fc = I.ctr->free_count, ni = I.ctr->next_index;  // fixed during the epoch
     for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / 32; g < c.n_groups; g += warps) {
         const uint32_t tree = c.group_tree[g];
         const int d = I.depths[tree];
         uint64_t root = I.roots[tree];
-        WSeq S{I, true};
-        for (uint32_t k = c.begin[g]; k < c.begin[g + 1] && S.ok; ++k) {
-            const int32_t x = c.xyz[3 * k], y = c.xyz[3 * k + 1], z = c.xyz[3 * k + 2];
-            const uint32_t v = c.values[k];
-            uint8_t changed = 0;
-            if (root != EMPTY_ID || v != 0) {
-                const uint64_t nw = v != 0 ? wset(S, root, x, y, z, d, v) : wremove(S, root, x, y, z, d);
-                if (!S.ok) break;
-                if (nw != INVALID_ID) {
-                    if (root != EMPTY_ID && nw == root) {  // assert_ne!(new_root_id, self.root_id)
-                        set_error(I, ERR_REF_PANIC, 82);
-                        break;
-                    }
-                    root = nw;
-                    changed = 1;
-                }
+        bool ok = true;
+        const uint32_t first = c.begin[g], end = c.begin[g + 1];
+        for (uint32_t k0 = first; k0 < end && ok; k0 += 32) {  // 32 calls' arguments at a time
+            const uint32_t m = end - k0 < 32 ? end - k0 : 32;
+            int32_t ax = 0, ay = 0, az = 0;
+            uint32_t av = 0;
+            if (lane < m) {
+                ax = c.xyz[3 * (uint64_t)(k0 + lane)];
+                ay = c.xyz[3 * (uint64_t)(k0 + lane) + 1];
+                az = c.xyz[3 * (uint64_t)(k0 + lane) + 2];
+                av = c.values[k0 + lane];
             }
-            if ((threadIdx.x & 31u) == 0 && c.changed) c.changed[c.order[k]] = changed;
+            uint8_t changed = 0;  // of call k0 + lane
+            uint32_t k = 0;
+            for (; k < m; ++k) {
+                const int32_t x = __shfl_sync(0xFFFFFFFFu, ax, k), y = __shfl_sync(0xFFFFFFFFu, ay, k),
+                              z = __shfl_sync(0xFFFFFFFFu, az, k);
+                const uint32_t v = __shfl_sync(0xFFFFFFFFu, av, k);
+                if (root == EMPTY_ID && v == 0) continue;
+                const uint64_t nw = warp_set(I, fc, ni, root, x, y, z, d, v, &ok);
+                if (!ok) break;
+                if (nw == INVALID_ID) continue;
+                if (root != EMPTY_ID && nw == root) {  // assert_ne!(new_root_id, self.root_id)
+                    set_error(I, ERR_REF_PANIC, 82);
+                    ok = false;
+                    break;
+                }
+                root = nw;
+                if (lane == k) changed = 1;
+            }
+            if (lane < k && c.changed) c.changed[c.order[k0 + lane]] = changed;
         }
-        if ((threadIdx.x & 31u) == 0) c.new_root[g] = root;
+        if (lane == 0) c.new_root[g] = root;
     }
 }
 
@@ -1725,20 +1866,13 @@ cudaError_t launch_get_many(const DevInterner &I, uint64_t n, const uint32_t *tr
 cudaError_t launch_release(const DevInterner &I, uint64_t *list, uint32_t *frontier_a, uint32_t *frontier_b,
                            uint64_t frontier_cap, int rounds, int num_sms, cudaStream_t s) {
     (void)frontier_cap;
-    const unsigned g = (unsigned)num_sms * 4;
+    DevInterner Ic = I;
+    const uint64_t *l = list;
+    void *args[] = {&Ic, &l, &frontier_a, &frontier_b, &rounds};
     count_launches(1);
-    (void)launch_pdl(release_advance_kernel, dim3(1), dim3(1), 0, s, I);  // clears the output count
-    count_launches(1);
-    (void)launch_pdl(release_roots_kernel, dim3(g), dim3(kThreads), 0, s, I, list, frontier_a);
-    uint32_t *in = frontier_a, *out = frontier_b;
-    for (int r = 0; r < rounds; ++r) {  // each kernel's last CTA advances the dying set
-        count_launches(1);
-        (void)launch_pdl(release_round_kernel, dim3(g), dim3(kThreads), release_smem(I.vbits), s, I, in, out);
-        uint32_t *t = in;
-        in = out;
-        out = t;
-    }
-    return cudaGetLastError();
+    // two CTAs an SM are resident at any register and shared-memory use of the kernel
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(release_kernel), dim3((unsigned)num_sms * 2),
+                                       dim3(kThreads), args, release_smem(I.vbits), s);
 }
 
 cudaError_t launch_tree_set(const DevInterner &I, uint32_t tree, int32_t x, int32_t y, int32_t z, uint32_t v,
@@ -1751,12 +1885,11 @@ cudaError_t launch_tree_set(const DevInterner &I, uint32_t tree, int32_t x, int3
 cudaError_t launch_trees_set(const DevInterner &I, const SetCalls &c, uint64_t *list, unsigned long long fc0,
                              unsigned long long ni0, uint32_t *frontier_a, uint32_t *frontier_b, int max_depth,
                              int num_sms, cudaStream_t s) {
-    const unsigned per_block = kThreads / 32;
-    unsigned g = (c.n_groups + per_block - 1) / per_block;
-    if (g > (unsigned)num_sms * 8) g = (unsigned)num_sms * 8;
+    unsigned g = c.n_groups;  // one-warp CTAs: few trees spread over the SMs
+    if (g > (unsigned)num_sms * 16) g = (unsigned)num_sms * 16;
     if (g == 0) g = 1;
     count_launches(1);
-    trees_set_kernel<<<g, kThreads, 0, s>>>(I, c);
+    trees_set_kernel<<<g, 32, 0, s>>>(I, c);
     cudaError_t e = launch_epoch_refcounts(I, num_sms, s);
     if (e != cudaSuccess) return e;
     unsigned gr = (c.n_groups + kThreads - 1) / kThreads;
