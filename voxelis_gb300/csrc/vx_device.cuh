@@ -248,25 +248,25 @@ __device__ __forceinline__ uint64_t make_slot(uint32_t tag, uint32_t idx) { retu
 
 // calc_average (core/voxel.rs:96-141): the mode of the 8 values. Distinct values are visited in
 // first-seen order; a later value replaces the current best when it is more frequent, or equally
-// frequent while the best is the default value and it is not. Fully unrolled on registers.
+// frequent while the best is the default value and it is not. So the result is the first value other than
+// the default that is as frequent as any, or the default when none is. Each of the 28 pairs is compared
+// once, fully unrolled on registers.
 __device__ __forceinline__ uint32_t calc_average8(const uint32_t v[8]) {
-    uint32_t best = v[0];
-    uint32_t best_cnt = 0;
+    uint32_t cnt[8] = {1, 1, 1, 1, 1, 1, 1, 1};
 #pragma unroll
-    for (int j = 0; j < 8; ++j) best_cnt += v[j] == v[0] ? 1u : 0u;
+    for (int k = 1; k < 8; ++k)
 #pragma unroll
-    for (int k = 1; k < 8; ++k) {
-        bool first = true;
-#pragma unroll
-        for (int j = 0; j < k; ++j) first = first && v[j] != v[k];
-        uint32_t cnt = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) cnt += v[j] == v[k] ? 1u : 0u;
-        if (first && (cnt > best_cnt || (cnt == best_cnt && best == 0 && v[k] != 0))) {
-            best = v[k];
-            best_cnt = cnt;
+        for (int j = 0; j < k; ++j) {
+            const uint32_t same = v[j] == v[k] ? 1u : 0u;
+            cnt[j] += same;
+            cnt[k] += same;
         }
-    }
+    uint32_t most = cnt[0];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) most = max(most, cnt[k]);
+    uint32_t best = 0;
+#pragma unroll
+    for (int k = 7; k >= 0; --k) best = (cnt[k] == most && v[k] != 0) ? v[k] : best;
     return best;
 }
 
