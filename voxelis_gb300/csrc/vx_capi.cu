@@ -8,6 +8,7 @@
 #include <atomic>
 #include <cstring>
 #include <functional>
+#include <mutex>
 #include <new>
 #include <string>
 #include <thread>
@@ -214,6 +215,8 @@ struct vx_interner {
     uint32_t *frontier = nullptr;  // 2 * capacity u32 (the single-thread queue aliases it under P3)
     uint64_t *seq_queue = nullptr;
     uint64_t seq_queue_cap = 0;
+    uint64_t *get_table = nullptr;  // kGetTableEntries words, filled and read by one call's launches
+    std::mutex get_mutex;           // queues a call's launches together: callers may read from several threads
     unsigned long long *d_live = nullptr;
     int *d_status = nullptr;
     // pinned staging
@@ -821,6 +824,7 @@ int vx_interner_create(uint64_t budget_bytes, int voxel_bits, uint32_t patch_fla
     alloc((void **)&D.table, slots * 8);
     alloc((void **)&D.leaf_table, ((size_t)1 << voxel_bits) * 8);
     alloc((void **)&it->frontier, 2 * cap * 4 + 64);
+    alloc((void **)&it->get_table, kGetTableEntries * 8);
     alloc((void **)&it->d_live, 2 * sizeof(unsigned long long));
     alloc((void **)&it->d_status, sizeof(int) * 4);
     if (patch_flags & VX_PATCH_P3) {
@@ -864,7 +868,7 @@ int vx_interner_destroy(vx_interner *it) {
     if (it->stream) cudaStreamSynchronize(it->stream);
     DevInterner &D = it->dev;
     void *ptrs[] = {D.children, D.values, D.refcount, D.generation, D.hash, D.ids, D.free_list, D.ctr, D.table,
-                    D.leaf_table, D.roots, D.depths, it->frontier, it->seq_queue, it->d_live, it->d_status};
+                    D.leaf_table, D.roots, D.depths, it->frontier, it->seq_queue, it->get_table, it->d_live, it->d_status};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     it->ws.release();
@@ -1575,11 +1579,22 @@ int vx_build_dense(vx_interner *it, uint32_t n, const vx_tree *trees, const void
     return st;
 }
 
+}  // extern "C"
+namespace {
+// Queues the gets of one call (device memory) on the interner's stream.
+cudaError_t queue_gets(vx_interner *it, uint64_t n, const uint32_t *trees, const int32_t *xyz, uint8_t *found, void *values) {
+    Phase ph(it, VX_PROF_GET);
+    std::lock_guard<std::mutex> lock(it->get_mutex);
+    const int k = get_table_levels(n, it->tree_count, depth_limit(it->flags) - 1);
+    return launch_get_many(it->dev, n, trees, xyz, found, values, it->get_table, k, it->tree_count, it->num_sms, it->stream);
+}
+}  // namespace
+extern "C" {
+
 int vx_get_many_async(vx_interner *it, uint64_t n, const vx_tree *trees_dev, const int32_t *xyz_dev,
                       uint8_t *found_dev, void *values_dev) {
     if (!it || (n && (!trees_dev || !xyz_dev || !found_dev || !values_dev))) return VX_E_INVALID_ARG;
-    Phase ph(it, VX_PROF_GET);
-    VX_CUDA(launch_get_many(it->dev, n, trees_dev, xyz_dev, found_dev, values_dev, it->num_sms, it->stream));
+    VX_CUDA(queue_gets(it, n, trees_dev, xyz_dev, found_dev, values_dev));
     return VX_OK;
 }
 
@@ -1588,10 +1603,7 @@ int vx_get_many(vx_interner *it, uint64_t n, const vx_tree *trees, const int32_t
     if (!it || (n && (!trees || !xyz || !found || !values))) return VX_E_INVALID_ARG;
     if (n == 0) return VX_OK;
     if (mem == VX_MEM_DEVICE) {
-        {
-            Phase ph(it, VX_PROF_GET);
-            VX_CUDA(launch_get_many(it->dev, n, trees, xyz, found, values, it->num_sms, it->stream));
-        }
+        VX_CUDA(queue_gets(it, n, trees, xyz, found, values));
         return sync_and_check(it);
     }
     const size_t vb = it->vbits / 8;
@@ -1606,10 +1618,7 @@ int vx_get_many(vx_interner *it, uint64_t n, const vx_tree *trees, const int32_t
         VX_CUDA(cudaMemcpyAsync(dt, trees, n * 4, cudaMemcpyHostToDevice, it->stream));
         VX_CUDA(cudaMemcpyAsync(dx, xyz, n * 12, cudaMemcpyHostToDevice, it->stream));
     }
-    {
-        Phase ph(it, VX_PROF_GET);
-        VX_CUDA(launch_get_many(it->dev, n, dt, dx, df, dv, it->num_sms, it->stream));
-    }
+    VX_CUDA(queue_gets(it, n, dt, dx, df, dv));
     {
         Phase ph(it, VX_PROF_COPY);
         VX_CUDA(cudaMemcpyAsync(found, df, n, cudaMemcpyDeviceToHost, it->stream));

@@ -140,8 +140,13 @@ enum : int { SC_RELEASE = 3, SC_REF_DONE = 6, SC_DONE = 7 };
 static_assert(SC_RELEASE == kScRelease, "release slot shared with vx_device.cuh");
 
 // ---- reads, releases, single-voxel operations, maintenance (vx_ops.cu) -------------------------
+// table (kGetTableEntries words of scratch) and k = get_table_levels(...): the nodes k levels below the roots
+// of the trees 0 .. n_trees - 1 are looked up first; k = 0: no table.
+constexpr uint64_t kGetTableEntries = 1u << 18;  // 2 MB an interner (2^21 entries: no faster on 4096 chunks, 6% on a deep tree)
+int get_table_levels(uint64_t n, uint32_t n_trees, int max_depth);
 cudaError_t launch_get_many(const DevInterner &I, uint64_t n, const uint32_t *trees, const int32_t *xyz,
-                            uint8_t *found, void *values, int num_sms, cudaStream_t s);
+                            uint8_t *found, void *values, uint64_t *table, int k, uint32_t n_trees, int num_sms,
+                            cudaStream_t s);
 // to_vec over trees of depth d into [y][z][x] grids: cubes [cube_begin, cube_begin + n_cubes) of side
 // min(32, 2^d), ordered (tree, cy, cz, cx); cube_begin must start a cy-slab and `out` points at that
 // slab's first element.

@@ -22,46 +22,68 @@ namespace {
 
 constexpr int kThreads = 256;
 
-template <class T>
+// The child of branch `node` in slot k, read through the read-only path; no load when the mask says EMPTY.
+__device__ __forceinline__ uint64_t get_child(const DevInterner &I, uint64_t node, uint32_t k) {
+    if (!((id_mask(node) >> k) & 1u)) return EMPTY_ID;
+    return __ldg(reinterpret_cast<const unsigned long long *>(I.children) + 8ull * id_index(node) + k);
+}
+
+// Large batches of gets start from a table of the nodes k levels below every root: one load instead of k
+// dependent ones. Tree t's entries are at t << 3k, by (y, z, x) of the node. Trees of less than k levels
+// have entries at their depth.
+__device__ __forceinline__ uint32_t get_entry(uint32_t x, uint32_t y, uint32_t z, int d, int k) {
+    return ((y >> (d - k)) << (2 * k)) | ((z >> (d - k)) << k) | (x >> (d - k));
+}
+
+__global__ void __launch_bounds__(kThreads) get_table_kernel(DevInterner I, uint32_t n_trees, int k, uint64_t *table) {
+    const uint64_t n = (uint64_t)n_trees << (3 * k);
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t t = (uint32_t)(i >> (3 * k)), e = (uint32_t)(i & ((1ull << (3 * k)) - 1ull));
+        const int d = I.depths[t];
+        if (d == TREE_UNUSED) continue;
+        const int kt = d < k ? d : k;
+        if (e >> (3 * kt)) continue;
+        const uint32_t m = (1u << kt) - 1u, x = e & m, z = (e >> kt) & m, y = e >> (2 * kt);
+        uint64_t node = I.roots[t];
+        for (int s = kt - 1; s >= 0 && node != EMPTY_ID && id_is_branch(node); --s)
+            node = get_child(I, node, ((x >> s) & 1u) | (((y >> s) & 1u) << 1) | (((z >> s) & 1u) << 2));
+        table[i] = node;
+    }
+}
+
+// One query a thread. (Two, four and eight chains of loads a thread, with 16-byte loads of the inputs, were
+// slower at every size: 4 M gets on 4096 chunks 46 us with one, 49, 51 and 71 us.)
+template <class T, bool TABLE>
 __global__ void __launch_bounds__(kThreads) get_kernel(DevInterner I, uint64_t n, const uint32_t *trees,
-                                                      const int32_t *xyz, uint8_t *found, T *values) {
+                                                      const int32_t *xyz, uint8_t *found, T *values,
+                                                      const uint64_t *table, int k, uint32_t n_trees) {
+    if (TABLE) pdl_wait();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     bool oob = false, bad = false;
     for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += stride) {
         const uint32_t t = __ldg(trees + q);
+        const uint32_t x = __ldg(xyz + 3 * q), y = __ldg(xyz + 3 * q + 1), z = __ldg(xyz + 3 * q + 2);
         const int d = t < I.tree_cap ? I.depths[t] : TREE_UNUSED;
-        const int32_t x = __ldg(xyz + 3 * q), y = __ldg(xyz + 3 * q + 1), z = __ldg(xyz + 3 * q + 2);
-        uint32_t val = 0;
-        uint8_t f = 0;
-        if (d == TREE_UNUSED) {
-            bad = true;
-        } else if (x < 0 || y < 0 || z < 0 || x >= (1 << d) || y >= (1 << d) || z >= (1 << d)) {
-            oob = true;
-        } else {
-            uint64_t node = I.roots[t];
-            int depth = 0;
-            while (node != EMPTY_ID) {
-                if (depth >= d) {
-                    const uint32_t v = node_value(I, id_index(node));
-                    if (v != 0) {
-                        val = v;
-                        f = 1;
-                    }
-                    break;
-                }
-                if (id_is_branch(node)) {
-                    const int shift = d - depth - 1;
-                    const uint32_t ci = ((x >> shift) & 1) | (((y >> shift) & 1) << 1) | (((z >> shift) & 1) << 2);
-                    node = __ldg(reinterpret_cast<const unsigned long long *>(I.children) + 8ull * id_index(node) + ci);
-                    ++depth;
-                } else {
-                    val = node_value(I, id_index(node));
-                    f = 1;
-                    break;
-                }
+        const uint32_t side = d == TREE_UNUSED ? 0u : 1u << d;
+        const bool in = x < side && y < side && z < side;
+        bad = bad || d == TREE_UNUSED;
+        oob = oob || (d != TREE_UNUSED && !in);
+        uint64_t node = EMPTY_ID;
+        int shift = -1;  // of the child slot's coordinate bits, -1 at depth d
+        if (in) {
+            shift = d - 1;
+            if (TABLE && t < n_trees) {  // (a replayed graph may name trees created since it was captured)
+                const int kt = d < k ? d : k;
+                node = __ldg((const unsigned long long *)table + ((uint64_t)t << (3 * k)) + get_entry(x, y, z, d, kt));
+                shift -= kt;
+            } else {
+                node = I.roots[t];
             }
         }
-        found[q] = f;
+        for (; shift >= 0 && node != EMPTY_ID && id_is_branch(node); --shift)
+            node = get_child(I, node, ((x >> shift) & 1) | (((y >> shift) & 1) << 1) | (((z >> shift) & 1) << 2));
+        const uint32_t val = node != EMPTY_ID ? (uint32_t)__ldg(reinterpret_cast<const T *>(I.values) + id_index(node)) : 0u;
+        found[q] = node != EMPTY_ID && (val != 0 || shift >= 0);  // at depth d a default value is no voxel
         values[q] = (T)val;
     }
     if (oob) set_error(I, ERR_OOB, 50);
@@ -1849,18 +1871,43 @@ cudaError_t launch_occupancy_many(const DevInterner &I, const uint8_t *grids, ui
     return cudaGetLastError();
 }
 
+// Levels the table of a call skips (0: no table). n queries over n_trees trees: no more entries than an
+// eighth of the queries, so that filling them stays small beside the reads, and than kGetTableEntries; from
+// two levels up, since one saves no more than it costs; and not for calls so small that the extra launch
+// shows (131 k gets on a tree of depth 9: 15.0 us with it, 13.7 without; 1 M: 22.7 and 26.0; 16 M: 141 and
+// 264; 4 M on 4096 trees of depth 5: 45.6 and 54.2; 262 k on 64 of them: 13.9 and 13.5).
+int get_table_levels(uint64_t n, uint32_t n_trees, int max_depth) {
+    if (n < (1u << 19) || n_trees == 0) return 0;
+    const uint64_t most = std::min<uint64_t>(kGetTableEntries, n / 8);
+    int k = 0;
+    while (k < max_depth && ((uint64_t)n_trees << (3 * (k + 1))) <= most) ++k;
+    return k >= 2 ? k : 0;
+}
+
 cudaError_t launch_get_many(const DevInterner &I, uint64_t n, const uint32_t *trees, const int32_t *xyz,
-                            uint8_t *found, void *values, int num_sms, cudaStream_t s) {
+                            uint8_t *found, void *values, uint64_t *table, int k, uint32_t n_trees, int num_sms,
+                            cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     uint64_t blocks = (n + kThreads - 1) / kThreads;
-    const uint64_t cap = (uint64_t)num_sms * 16;
+    const uint64_t cap = (uint64_t)num_sms * 64;
     if (blocks > cap) blocks = cap;
+    const unsigned g = (unsigned)blocks;
+    if (k > 0) {
+        uint64_t tb = (((uint64_t)n_trees << (3 * k)) + kThreads - 1) / kThreads;
+        if (tb > cap) tb = cap;
+        count_launches(1);
+        get_table_kernel<<<(unsigned)tb, kThreads, 0, s>>>(I, n_trees, k, table);
+    }
     count_launches(1);
-    if (I.vbits == 8)
-        get_kernel<uint8_t><<<(unsigned)blocks, kThreads, 0, s>>>(I, n, trees, xyz, found, (uint8_t *)values);
-    else
-        get_kernel<uint16_t><<<(unsigned)blocks, kThreads, 0, s>>>(I, n, trees, xyz, found, (uint16_t *)values);
-    return cudaGetLastError();
+    auto launch = [&](auto *v) -> cudaError_t {
+        using T = std::remove_pointer_t<decltype(v)>;
+        if (k > 0)
+            return launch_pdl(get_kernel<T, true>, dim3(g), dim3(kThreads), 0, s, I, n, trees, xyz, found, v,
+                              (const uint64_t *)table, k, n_trees);
+        get_kernel<T, false><<<g, kThreads, 0, s>>>(I, n, trees, xyz, found, v, nullptr, 0, 0);
+        return cudaGetLastError();
+    };
+    return I.vbits == 8 ? launch((uint8_t *)values) : launch((uint16_t *)values);
 }
 
 cudaError_t launch_release(const DevInterner &I, uint64_t *list, uint32_t *frontier_a, uint32_t *frontier_b,
