@@ -919,24 +919,8 @@ uint64_t vx_kernel_launches(void) { return vxg::g_launches.load(); }
 
 int vx_interner_reset(vx_interner *it) {
     if (!it) return VX_E_INVALID_ARG;
-    cudaStream_t s = it->stream;
-    VX_CUDA(cudaStreamSynchronize(s));
-    VX_CUDA(cudaMemsetAsync(it->dev.table, 0xFF, it->table_slots * 8, s));
-    VX_CUDA(cudaMemsetAsync(it->dev.leaf_table, 0, ((size_t)1 << it->vbits) * 8, s));
-    VX_CUDA(cudaMemsetAsync(it->dev.roots, 0, (size_t)it->tree_cap * 8, s));
-    VX_CUDA(cudaMemsetAsync(it->dev.ids, 0, it->capacity * 8, s));
-    VX_CUDA(cudaMemsetAsync(it->dev.refcount, 0, it->capacity * 4, s));
-    // the rest of the node records as vx_interner_create leaves them: recycled slots carry bumped
-    // generations (which become part of new BlockIds) and old records
-    VX_CUDA(cudaMemsetAsync(it->dev.generation, 0, it->capacity * 2, s));
-    VX_CUDA(cudaMemsetAsync(it->dev.children, 0, it->capacity * 64, s));
-    VX_CUDA(cudaMemsetAsync(it->dev.values, 0, it->capacity * (it->vbits / 8), s));
-    VX_CUDA(cudaMemsetAsync(it->dev.hash, 0, it->capacity * 8, s));
-    DevCounters c0{};
-    c0.next_index = 1;
-    *it->h_ctr = c0;
-    VX_CUDA(cudaMemcpyAsync(it->dev.ctr, it->h_ctr, sizeof(DevCounters), cudaMemcpyHostToDevice, s));
-    VX_CUDA(cudaStreamSynchronize(s));
+    // in stream order after what is queued; nothing here waits for it
+    VX_CUDA(launch_reset(it->dev, it->num_sms, it->stream));
     std::fill(it->tree_maybe_nonempty.begin(), it->tree_maybe_nonempty.end(), 0);
     it->all_trees_unknown = false;
     return VX_OK;

@@ -232,6 +232,8 @@ cudaError_t launch_trees_set(const DevInterner &I, const SetCalls &c, uint64_t *
 cudaError_t launch_tree_fill(const DevInterner &I, uint32_t tree, uint32_t v, uint64_t *queue,
                              uint64_t queue_cap, int *status_out, cudaStream_t s);
 cudaError_t launch_rehash(const DevInterner &I, uint64_t table_slots, int num_sms, cudaStream_t s);
+// The interner's device state as after creation (tree handles stay, their roots are EMPTY).
+cudaError_t launch_reset(const DevInterner &I, int num_sms, cudaStream_t s);
 cudaError_t launch_count_live(const DevInterner &I, unsigned long long *out2, int num_sms, cudaStream_t s);
 
 }  // namespace vxg

