@@ -218,10 +218,9 @@ struct vx_interner {
     uint64_t *get_table = nullptr;  // kGetTableEntries words, filled and read by one call's launches
     std::mutex get_mutex;           // queues a call's launches together: callers may read from several threads
     unsigned long long *d_live = nullptr;
-    int *d_status = nullptr;
     // pinned staging
     DevCounters *h_ctr = nullptr;
-    int *h_status = nullptr;
+    HostReply *h_reply = nullptr;
     unsigned long long *h_live = nullptr;
     std::string last_error;
     // instrumentation: event pairs recorded around the phases while profiling is on
@@ -313,6 +312,14 @@ int sync_and_check(vx_interner *it) {
     if (err & ERR_INVALID) return set_err(it, VX_E_INVALID_ARG, "unknown tree handle or depth mismatch" + where);
     if (err & ERR_OOB) return set_err(it, VX_E_OOB, "position out of bounds" + where);
     return set_err(it, VX_E_UNSUPPORTED, "unknown device error" + where);
+}
+
+// Waits for a one-tree call's reply; with an error bit set, the full check.
+int wait_reply(vx_interner *it) {
+    VX_CUDA(cudaStreamSynchronize(it->stream));
+    if (it->h_reply->error) return sync_and_check(it);
+    it->h_ctr->tombstones = it->h_reply->tombstones;
+    return VX_OK;
 }
 
 cudaError_t grow_tree_table(vx_interner *it, uint32_t need) {
@@ -826,7 +833,6 @@ int vx_interner_create(uint64_t budget_bytes, int voxel_bits, uint32_t patch_fla
     alloc((void **)&it->frontier, 2 * cap * 4 + 64);
     alloc((void **)&it->get_table, kGetTableEntries * 8);
     alloc((void **)&it->d_live, 2 * sizeof(unsigned long long));
-    alloc((void **)&it->d_status, sizeof(int) * 4);
     if (patch_flags & VX_PATCH_P3) {
         it->seq_queue_cap = std::max<uint64_t>(cap + 1, 32768);
         alloc((void **)&it->seq_queue, it->seq_queue_cap * 8);
@@ -835,7 +841,7 @@ int vx_interner_create(uint64_t budget_bytes, int voxel_bits, uint32_t patch_fla
         alloc((void **)&it->seq_queue, it->seq_queue_cap * 8);
     }
     if (ok && cudaMallocHost((void **)&it->h_ctr, sizeof(DevCounters)) != cudaSuccess) ok = false;
-    if (ok && cudaMallocHost((void **)&it->h_status, sizeof(int) * 4) != cudaSuccess) ok = false;
+    if (ok && cudaMallocHost((void **)&it->h_reply, sizeof(HostReply)) != cudaSuccess) ok = false;
     if (ok && cudaMallocHost((void **)&it->h_live, 2 * sizeof(unsigned long long)) != cudaSuccess) ok = false;
     if (!ok || grow_tree_table(it, 1024) != cudaSuccess) {
         vx_interner_destroy(it);
@@ -868,14 +874,14 @@ int vx_interner_destroy(vx_interner *it) {
     if (it->stream) cudaStreamSynchronize(it->stream);
     DevInterner &D = it->dev;
     void *ptrs[] = {D.children, D.values, D.refcount, D.generation, D.hash, D.ids, D.free_list, D.ctr, D.table,
-                    D.leaf_table, D.roots, D.depths, it->frontier, it->seq_queue, it->get_table, it->d_live, it->d_status};
+                    D.leaf_table, D.roots, D.depths, it->frontier, it->seq_queue, it->get_table, it->d_live};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     it->ws.release();
     it->staging.release();
     it->pinned.release();
     if (it->h_ctr) cudaFreeHost(it->h_ctr);
-    if (it->h_status) cudaFreeHost(it->h_status);
+    if (it->h_reply) cudaFreeHost(it->h_reply);
     if (it->h_live) cudaFreeHost(it->h_live);
     for (auto &m : it->marks) {
         cudaEventDestroy(m.second.first);
@@ -1065,9 +1071,8 @@ int vx_tree_create(vx_interner *it, int max_depth, vx_tree *out) {
 
 int vx_tree_fill(vx_interner *it, vx_tree tree, uint32_t value) {
     if (!it || !tree_ok(it, tree) || !value_fits(it, value)) return VX_E_INVALID_ARG;
-    VX_CUDA(launch_tree_fill(it->dev, tree, value, it->seq_queue, it->seq_queue_cap, it->d_status, it->stream));
-    VX_CUDA(cudaMemcpyAsync(it->h_status, it->d_status, sizeof(int), cudaMemcpyDeviceToHost, it->stream));
-    int st = sync_and_check(it);
+    VX_CUDA(launch_tree_fill(it->dev, tree, value, it->seq_queue, it->seq_queue_cap, it->h_reply, it->stream));
+    int st = wait_reply(it);
     it->tree_maybe_nonempty[tree] = value != 0;
     if (st == VX_OK) maybe_rehash(it);
     return st;
@@ -1103,11 +1108,10 @@ int vx_tree_set(vx_interner *it, vx_tree tree, int32_t x, int32_t y, int32_t z, 
     const int32_t side = 1 << it->tree_depth[tree];
     if (x < 0 || y < 0 || z < 0 || x >= side || y >= side || z >= side)
         return set_err(it, VX_E_OOB, "position out of bounds");
-    VX_CUDA(launch_tree_set(it->dev, tree, x, y, z, value, it->seq_queue, it->seq_queue_cap, it->d_status, it->stream));
-    VX_CUDA(cudaMemcpyAsync(it->h_status, it->d_status, sizeof(int), cudaMemcpyDeviceToHost, it->stream));
-    int st = sync_and_check(it);
-    if (changed) *changed = *it->h_status == 1;
-    if (*it->h_status == 1) it->tree_maybe_nonempty[tree] = 1;
+    VX_CUDA(launch_tree_set(it->dev, tree, x, y, z, value, it->seq_queue, it->seq_queue_cap, it->h_reply, it->stream));
+    int st = wait_reply(it);
+    if (changed) *changed = it->h_reply->status == 1;
+    if (it->h_reply->status == 1) it->tree_maybe_nonempty[tree] = 1;
     if (st == VX_OK) maybe_rehash(it);
     return st;
 }
@@ -1117,12 +1121,14 @@ int vx_tree_get(vx_interner *it, vx_tree tree, int32_t x, int32_t y, int32_t z, 
     const int32_t side = 1 << it->tree_depth[tree];
     if (x < 0 || y < 0 || z < 0 || x >= side || y >= side || z >= side)
         return set_err(it, VX_E_OOB, "position out of bounds");
-    int32_t xyz[3] = {x, y, z};
-    uint8_t f = 0;
-    uint16_t v = 0;
-    int st = vx_get_many(it, 1, &tree, xyz, &f, &v, VX_MEM_HOST);
-    *found = f;
-    *value = f ? (it->vbits == 8 ? (v & 0xFF) : v) : 0;
+    std::lock_guard<std::mutex> lock(it->get_mutex);  // readers share the reply
+    {
+        Phase ph(it, VX_PROF_GET);
+        VX_CUDA(launch_tree_get(it->dev, tree, x, y, z, it->h_reply, it->stream));
+    }
+    int st = wait_reply(it);
+    *found = it->h_reply->status;
+    *value = *found ? it->h_reply->value : 0;
     return st;
 }
 

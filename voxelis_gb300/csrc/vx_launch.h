@@ -207,10 +207,17 @@ cudaError_t launch_vtm_place(const DevInterner &I, const uint8_t *bytes, const V
 // breadth-first rounds, using two frontier buffers of `frontier_cap` entries.
 cudaError_t launch_release(const DevInterner &I, uint64_t *list, uint32_t *frontier_a, uint32_t *frontier_b,
                            uint64_t frontier_cap, int rounds, int num_sms, cudaStream_t s);
-// Single-voxel VoxTree::set / fill / clear executed by one thread with the reference's own
-// refcount order; the result status word is written to *status_out.
+// One-tree calls answer in pinned host memory, valid once the stream has been waited for.
+struct HostReply {
+    int status;
+    uint32_t value;
+    uint32_t error;               // the interner's sticky error bits
+    unsigned long long tombstones;
+};
+cudaError_t launch_tree_get(const DevInterner &I, uint32_t tree, int32_t x, int32_t y, int32_t z, HostReply *r, cudaStream_t s);
+// Single-voxel VoxTree::set / fill / clear with the reference's own refcount and release order.
 cudaError_t launch_tree_set(const DevInterner &I, uint32_t tree, int32_t x, int32_t y, int32_t z, uint32_t v,
-                            uint64_t *queue, uint64_t queue_cap, int *status_out, cudaStream_t s);
+                            uint64_t *queue, uint64_t queue_cap, HostReply *r, cudaStream_t s);
 // Many VoxTree::set calls (vx_trees_set_many): group g = the calls of tree group_tree[g], at
 // [begin[g], begin[g+1]) of xyz / values in call order; order[k] = the call's index for changed[].
 struct SetCalls {
@@ -229,8 +236,8 @@ struct SetCalls {
 cudaError_t launch_trees_set(const DevInterner &I, const SetCalls &c, uint64_t *list, unsigned long long fc0,
                              unsigned long long ni0, uint32_t *frontier_a, uint32_t *frontier_b, int max_depth,
                              int num_sms, cudaStream_t s);
-cudaError_t launch_tree_fill(const DevInterner &I, uint32_t tree, uint32_t v, uint64_t *queue,
-                             uint64_t queue_cap, int *status_out, cudaStream_t s);
+cudaError_t launch_tree_fill(const DevInterner &I, uint32_t tree, uint32_t v, uint64_t *queue, uint64_t queue_cap,
+                             HostReply *r, cudaStream_t s);
 cudaError_t launch_rehash(const DevInterner &I, uint64_t table_slots, int num_sms, cudaStream_t s);
 // The interner's device state as after creation (tree handles stay, their roots are EMPTY).
 cudaError_t launch_reset(const DevInterner &I, int num_sms, cudaStream_t s);

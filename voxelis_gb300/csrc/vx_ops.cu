@@ -122,6 +122,26 @@ __global__ void __launch_bounds__(kThreads) release_kernel(DevInterner I, const 
     bar.leave();
 }
 
+// The answer of a one-tree call, in pinned host memory: the kernel writes it there itself, so that the call
+// is one launch and one wait (a copy of the status and one of the counters took 8 us of a 29 us set, the
+// argument and result copies of a get 25 of 38).
+__device__ __forceinline__ void reply(const DevInterner &I, HostReply *r, int status, uint32_t value) {
+    r->status = status;
+    r->value = value;
+    r->error = *(volatile unsigned int *)&I.ctr->error;
+    r->tombstones = *(volatile unsigned long long *)&I.ctr->tombstones;
+}
+
+// VoxTree::get of one voxel inside the tree (voxtree.rs:145-159). status: found.
+__global__ void tree_get_kernel(DevInterner I, uint32_t tree, uint32_t x, uint32_t y, uint32_t z, HostReply *r) {
+    int shift = (int)I.depths[tree] - 1;
+    uint64_t node = I.roots[tree];
+    for (; shift >= 0 && node != EMPTY_ID && id_is_branch(node); --shift)
+        node = get_child(I, node, ((x >> shift) & 1) | (((y >> shift) & 1) << 1) | (((z >> shift) & 1) << 2));
+    const uint32_t val = node != EMPTY_ID ? node_value(I, id_index(node)) : 0u;
+    reply(I, r, node != EMPTY_ID && (val != 0 || shift >= 0), val);
+}
+
 // ---- single-thread reference-order operations ---------------------------------------------------
 struct Seq {
     DevInterner I;
@@ -492,7 +512,7 @@ __device__ uint64_t seq_remove(Seq &S, uint64_t root, int32_t x, int32_t y, int3
 // VoxTree::set (voxtree.rs:163-260). status: 0 unchanged, 1 changed, -1 error. Thread 0 runs the set, the
 // CTA the release of the replaced root.
 __global__ void __launch_bounds__(kSeqThreads) tree_set_kernel(DevInterner I, uint32_t tree, int32_t x, int32_t y, int32_t z,
-                                                               uint32_t v, uint64_t *queue, uint64_t queue_cap, int *status) {
+                                                               uint32_t v, uint64_t *queue, uint64_t queue_cap, HostReply *r) {
     __shared__ SeqShared sh;
     __shared__ uint64_t new_root;
     __shared__ int result;  // 0 unchanged, 1 to be installed, -1 error
@@ -519,7 +539,7 @@ __global__ void __launch_bounds__(kSeqThreads) tree_set_kernel(DevInterner I, ui
     if (result == 1 && root != EMPTY_ID) seq_release(S, sh, root);
     if (threadIdx.x == 0) {
         if (result == 1 && S.ok) I.roots[tree] = new_root;
-        *status = result == 1 && !S.ok ? -1 : result;
+        reply(I, r, result == 1 && !S.ok ? -1 : result, 0);
     }
 }
 
@@ -860,28 +880,21 @@ __global__ void __launch_bounds__(kThreads) trees_set_garbage_kernel(DevInterner
 
 // VoxTree::fill / clear (voxtree.rs:264-292). status: 1 if the tree was dirtied. One CTA.
 __global__ void __launch_bounds__(kSeqThreads) tree_fill_kernel(DevInterner I, uint32_t tree, uint32_t v, uint64_t *queue,
-                                                                uint64_t queue_cap, int *status) {
+                                                                uint64_t queue_cap, HostReply *r) {
     __shared__ SeqShared sh;
     Seq S{I, queue, queue_cap, true};
     const uint64_t root = I.roots[tree];
     __syncthreads();
     if (root != EMPTY_ID) seq_release(S, sh, root);
     if (threadIdx.x != 0) return;
-    *status = root != EMPTY_ID;
-    if (!S.ok) {
-        *status = -1;
-        return;
-    }
-    if (root != EMPTY_ID) I.roots[tree] = EMPTY_ID;
-    if (v != 0) {
+    int status = root != EMPTY_ID;
+    if (S.ok && root != EMPTY_ID) I.roots[tree] = EMPTY_ID;
+    if (S.ok && v != 0) {
         const uint64_t leaf = seq_leaf(S, v);
-        if (!S.ok) {
-            *status = -1;
-            return;
-        }
-        I.roots[tree] = leaf;
-        *status = 1;
+        if (S.ok) I.roots[tree] = leaf;
+        status = 1;
     }
+    reply(I, r, S.ok ? status : -1, 0);
 }
 
 // ---- maintenance -------------------------------------------------------------------------------
@@ -1962,10 +1975,16 @@ cudaError_t launch_release(const DevInterner &I, uint64_t *list, uint32_t *front
                                        dim3(kThreads), args, release_smem(I.vbits), s);
 }
 
-cudaError_t launch_tree_set(const DevInterner &I, uint32_t tree, int32_t x, int32_t y, int32_t z, uint32_t v,
-                            uint64_t *queue, uint64_t queue_cap, int *status_out, cudaStream_t s) {
+cudaError_t launch_tree_get(const DevInterner &I, uint32_t tree, int32_t x, int32_t y, int32_t z, HostReply *r, cudaStream_t s) {
     count_launches(1);
-    tree_set_kernel<<<1, kSeqThreads, 0, s>>>(I, tree, x, y, z, v, queue, queue_cap, status_out);
+    tree_get_kernel<<<1, 1, 0, s>>>(I, tree, x, y, z, r);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tree_set(const DevInterner &I, uint32_t tree, int32_t x, int32_t y, int32_t z, uint32_t v,
+                            uint64_t *queue, uint64_t queue_cap, HostReply *r, cudaStream_t s) {
+    count_launches(1);
+    tree_set_kernel<<<1, kSeqThreads, 0, s>>>(I, tree, x, y, z, v, queue, queue_cap, r);
     return cudaGetLastError();
 }
 
@@ -1986,10 +2005,10 @@ cudaError_t launch_trees_set(const DevInterner &I, const SetCalls &c, uint64_t *
     return launch_release(I, list, frontier_a, frontier_b, 0, max_depth + 2, num_sms, s);
 }
 
-cudaError_t launch_tree_fill(const DevInterner &I, uint32_t tree, uint32_t v, uint64_t *queue,
-                             uint64_t queue_cap, int *status_out, cudaStream_t s) {
+cudaError_t launch_tree_fill(const DevInterner &I, uint32_t tree, uint32_t v, uint64_t *queue, uint64_t queue_cap,
+                             HostReply *r, cudaStream_t s) {
     count_launches(1);
-    tree_fill_kernel<<<1, kSeqThreads, 0, s>>>(I, tree, v, queue, queue_cap, status_out);
+    tree_fill_kernel<<<1, kSeqThreads, 0, s>>>(I, tree, v, queue, queue_cap, r);
     return cudaGetLastError();
 }
 
