@@ -1305,7 +1305,7 @@ __global__ void __launch_bounds__(kThreads) occupancy_active_kernel(const unsign
 // one z, each by one warp with 5 shuffle steps. The global planes are the OR of the materials' (up to
 // three materials) or a plane of their own. Rows of 65 words keep the transposes' column reads free of
 // bank conflicts; 100 KB leave two CTAs to an SM, one writing while the other reads.
-// 4096 dune chunks in 1024 builders, 8 material slots (906 MB): 310 us with the dense expansion, 1750 us
+// 4096 dune chunks in 1024 builders, 8 material slots (906 MB): 297 us with the dense expansion, 1750 us
 // when separate kernels counted voxels (one atomic a warp and value, 812 us), cleared the outputs
 // (137 us) and ORed every line's bits into them with atomics (607 us).
 constexpr int kOccThreads = 512;
@@ -1361,32 +1361,38 @@ __device__ __forceinline__ uint32_t equal_bytes(uint32_t w, uint32_t splat) {
     return (z * 0x01020408u) >> 24;
 }
 
-// Calls f(k, w) for the 4-byte words w (voxels 4k .. 4k+3) of a row of S voxels; a row of 2 voxels is
+// Calls f(k, w, n) for the words of a row of S voxels in order: w is the 4 voxels from 4k on, and holds for n
+// voxels (16 when it repeats, one value along x being the usual case, else 4). A row of 2 voxels is
 // padded with zeros.
 template <class F>
 __device__ __forceinline__ void row_words(const uint8_t *row, uint32_t S, F f) {
     if (S >= 16) {
         for (uint32_t q = 0; q < S / 16; ++q) {
             const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row) + q);
-            f(4 * q, v.x);
-            f(4 * q + 1, v.y);
-            f(4 * q + 2, v.z);
-            f(4 * q + 3, v.w);
+            if (v.x == v.y && v.x == v.z && v.x == v.w) {
+                f(4 * q, v.x, 16u);
+            } else {
+                f(4 * q, v.x, 4u);
+                f(4 * q + 1, v.y, 4u);
+                f(4 * q + 2, v.z, 4u);
+                f(4 * q + 3, v.w, 4u);
+            }
         }
     } else if (S >= 4) {
-        for (uint32_t k = 0; k < S / 4; ++k) f(k, __ldg(reinterpret_cast<const uint32_t *>(row) + k));
+        for (uint32_t k = 0; k < S / 4; ++k) f(k, __ldg(reinterpret_cast<const uint32_t *>(row) + k), 4u);
     } else {
-        f(0, (uint32_t)__ldg(reinterpret_cast<const uint16_t *>(row)));
+        f(0, (uint32_t)__ldg(reinterpret_cast<const uint16_t *>(row)), 4u);
     }
 }
 
-// Two words at p (p[0], p[1]); wide: p is 16-byte aligned.
+// Two words at p (p[0], p[1]); wide: p is 16-byte aligned. The outputs are stored evict-first: they are several
+// times the L2's size, and the grids that the next sweep reads should stay there.
 __device__ __forceinline__ void store_words(unsigned long long *p, ulonglong2 v, bool wide) {
     if (wide) {
-        *reinterpret_cast<ulonglong2 *>(p) = v;
+        __stcs(reinterpret_cast<ulonglong2 *>(p), v);
     } else {
-        p[0] = v.x;
-        p[1] = v.y;
+        __stcs(p, v.x);
+        __stcs(p + 1, v.y);
     }
 }
 
@@ -1413,7 +1419,7 @@ __global__ void __launch_bounds__(kOccThreads, 2) occupancy_builders_kernel(
     for (uint32_t t = first; t != kNoTree; t = next[t]) {
         const uint8_t *g = grids + t * per_tree;
         for (uint32_t r = tid; r < rows; r += kOccThreads)
-            row_words(g + (size_t)r * S, S, [&](uint32_t, uint32_t w) {
+            row_words(g + (size_t)r * S, S, [&](uint32_t, uint32_t w, uint32_t) {
                 if (w == last) return;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) present[(w >> (8 * k)) & 0xFFu] = 1;
@@ -1479,13 +1485,14 @@ __global__ void __launch_bounds__(kOccThreads, 2) occupancy_builders_kernel(
             bad = bad || !inside;
             for (uint32_t r = tid; r < rows; r += kOccThreads) {
                 uint64_t m[kOccPlanes] = {0, 0, 0};
-                row_words(g + (size_t)r * S, S, [&](uint32_t k, uint32_t w) {
+                row_words(g + (size_t)r * S, S, [&](uint32_t k, uint32_t w, uint32_t n) {
                     if (w == 0) return;
 #pragma unroll
                     for (int p = 0; p < kOccPlanes; ++p) {
                         if (want[p] == kOccNone) continue;
                         uint32_t e = equal_bytes(w, splat[p]);
                         if (want[p] == kOccAny) e ^= 0xFu;
+                        if (n == 16) e *= 0x1111u;
                         m[p] |= (uint64_t)e << (4 * k);
                     }
                 });
@@ -1546,14 +1553,14 @@ __global__ void __launch_bounds__(kOccThreads, 2) occupancy_builders_kernel(
                 ga |= u;
                 gb |= v;
                 if (out[p]) {
-                    out[p][word] = u;
-                    out[p][word + 32] = v;
+                    __stcs(out[p] + word, (unsigned long long)u);
+                    __stcs(out[p] + word + 32, (unsigned long long)v);
                 }
             }
             if (with_global) {
                 if (by_or) {
-                    gout[word] = ga;
-                    gout[word + 32] = gb;
+                    __stcs(gout + word, (unsigned long long)ga);
+                    __stcs(gout + word + 32, (unsigned long long)gb);
                 }
                 if (xz)
                     ay |= ga | gb;
