@@ -771,18 +771,23 @@ __device__ __forceinline__ void apply_single(const DevInterner &I, const ApplyAr
             if (s == a.max_depth - 1) leaf_refs_flush(I, L);
             if (!bar.sync()) return;
         }
-        if (t0) epoch_finalize_body(I);
+        if (t0) {
+            epoch_finalize_body(I);
+            ctr->scratch[SC_FREE_BASE] = ctr->free_count;
+        }
         release_roots_range(I, a.release_list, frontier_a, &ctr->rel_count[0], cta_base, stride);
         const LeafDrops D = leaf_drops_init(I, leaf_smem);  // the leaf counts were flushed before the last barrier
         if (!bar.sync()) return;
         // round r reads set r % 3 and writes set (r + 1) % 3; set (r + 2) % 3 was read by round r - 1
         // and is written by round r + 1, so it is cleared now
         uint32_t *fr[2] = {frontier_a, frontier_b};
+        uint64_t free_base = *(volatile unsigned long long *)&ctr->scratch[SC_FREE_BASE];
         for (int r = 0; r < rounds; ++r) {
-            if (*(volatile unsigned long long *)&ctr->rel_count[r % 3] == 0) break;  // the same answer in every CTA
+            const uint64_t n = *(volatile unsigned long long *)&ctr->rel_count[r % 3];
+            if (n == 0) break;  // the same answer in every CTA
             if (t0) ctr->rel_count[(r + 2) % 3] = 0;
-            release_round_range(I, D, fr[r & 1], fr[(r + 1) & 1], &ctr->rel_count[r % 3], &ctr->rel_count[(r + 1) % 3],
-                                cta_base, stride);
+            release_round_range(I, D, fr[r & 1], fr[(r + 1) & 1], n, free_base, &ctr->rel_count[(r + 1) % 3], cta_base, stride);
+            free_base += n;
             if (!bar.sync()) return;
         }
     }

@@ -598,6 +598,8 @@ struct GridBarrier {
 // Counter slot of the listed roots' number in DevCounters::scratch (the batched-apply launcher's table
 // lists every slot).
 constexpr int kScRelease = 3;
+// Slot of the free list's length at the start of the release rounds (written before the barrier in front of them).
+constexpr int kScFreeBase = 4;
 
 __device__ __forceinline__ void push_dying(uint32_t *list, unsigned long long *count, bool push, uint32_t idx) {
     const unsigned m = __ballot_sync(0xFFFFFFFFu, push);
@@ -684,14 +686,15 @@ __device__ __forceinline__ bool drop_refs(const DevInterner &I, uint32_t idx, ui
     return old == n;
 }
 
-// Retires the *n_in dying nodes of `in`: their children lose one reference each (children reaching
+// Retires the n dying nodes of `in`: their children lose one reference each (children reaching
 // zero are the next dying set, appended to `out` and counted in *n_out) and the nodes are recycled. A thread
 // takes a node; the counts of its branch children are decremented together, those of leaves in D, which
-// the CTA flushes at the end. The whole CTA calls it.
+// the CTA flushes at the end. Node j of the set goes to place free_base + j of the free list, and one thread
+// adds the set to the counters: a place and a count taken by every warp serialise at the two counters (an apply of
+// 6.3 M bottom groups and its undo, 3.2 M nodes released by each, 6.17 against 6.38 ms). The whole CTA calls it.
 __device__ __forceinline__ void release_round_range(const DevInterner &I, const LeafDrops &D, const uint32_t *in,
-                                                    uint32_t *out, const unsigned long long *n_in,
+                                                    uint32_t *out, uint64_t n, uint64_t free_base,
                                                     unsigned long long *n_out, uint64_t cta_base, uint64_t stride) {
-    const uint64_t n = *n_in;
     const unsigned lane = threadIdx.x & 31u;
     if (cta_base >= n) return;
     for (uint64_t base = cta_base; base < n; base += stride) {
@@ -743,18 +746,19 @@ __device__ __forceinline__ void release_round_range(const DevInterner &I, const 
             for (int k = 0; k < 8; ++k)
                 if ((dies >> k) & 1u) out[at++] = id_index(c[k]);
         }
-        const bool rec = in_range && id != 0;
-        if (in_range && id == 0) set_error(I, ERR_INTERNAL, 62);
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, rec);
-        unsigned long long fbase = 0;
-        if (m) {
-            const int leader = __ffs(m) - 1;
-            if ((int)lane == leader) fbase = atomicAdd(&I.ctr->free_count, (unsigned long long)__popc(m));
-            fbase = __shfl_sync(0xFFFFFFFFu, fbase, leader);
+        const unsigned leaves = __ballot_sync(0xFFFFFFFFu, in_range && id_is_leaf(id));
+        if (lane == 0 && leaves) atomicAdd(&I.ctr->tombstones, 0ull - (unsigned long long)__popc(leaves));
+        if (!in_range) continue;
+        if (id != 0) {
+            recycle_node(I, idx, id, h, gen, free_base + j);
+        } else {
+            I.free_list[free_base + j] = idx;
+            set_error(I, ERR_INTERNAL, 62);
         }
-        const unsigned tomb = __ballot_sync(0xFFFFFFFFu, rec && id_is_branch(id));
-        if (lane == 0 && tomb) atomicAdd(&I.ctr->tombstones, (unsigned long long)__popc(tomb));
-        if (rec) recycle_node(I, idx, id, h, gen, fbase + __popc(m & ((1u << lane) - 1u)));
+    }
+    if (cta_base == 0 && threadIdx.x == 0) {
+        I.ctr->free_count = free_base + n;
+        atomicAdd(&I.ctr->tombstones, n);
     }
     __syncthreads();
     for (uint32_t s = threadIdx.x; s < D.slots; s += blockDim.x) {  // slots: a multiple of the CTA's warps

@@ -136,8 +136,8 @@ cudaError_t launch_apply(const DevInterner &I, const ApplyArgs &a, int mode, boo
 cudaError_t launch_apply_single(const DevInterner &I, const ApplyArgs &a, bool check_depths, bool clear_pass,
                                 uint32_t *frontier_a, uint32_t *frontier_b, int rounds, int num_sms, cudaStream_t s);
 // Counter slots (DevCounters::scratch indices).
-enum : int { SC_RELEASE = 3, SC_REF_DONE = 6, SC_DONE = 7 };
-static_assert(SC_RELEASE == kScRelease, "release slot shared with vx_device.cuh");
+enum : int { SC_RELEASE = 3, SC_FREE_BASE = 4, SC_REF_DONE = 6, SC_DONE = 7 };
+static_assert(SC_RELEASE == kScRelease && SC_FREE_BASE == kScFreeBase, "release slots shared with vx_device.cuh");
 
 // ---- reads, releases, single-voxel operations, maintenance (vx_ops.cu) -------------------------
 // table (kGetTableEntries words of scratch) and k = get_table_levels(...): the nodes k levels below the roots

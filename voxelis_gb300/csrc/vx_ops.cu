@@ -103,15 +103,18 @@ __global__ void __launch_bounds__(kThreads) release_kernel(DevInterner I, const 
     if (!bar.usable()) return;
     const LeafDrops D = leaf_drops_init(I, release_mem);
     // the counts are zero between launches: the rounds clear them, and the last one read is empty
+    if (t0) ctr->scratch[SC_FREE_BASE] = ctr->free_count;
     release_roots_range(I, list, frontier_a, &ctr->rel_count[0], cta_base, stride);
     if (!bar.sync()) return;
     uint32_t *fr[2] = {frontier_a, frontier_b};
+    uint64_t free_base = *(volatile unsigned long long *)&ctr->scratch[SC_FREE_BASE];
     int r = 0;
     for (; r < rounds; ++r) {
-        if (*(volatile unsigned long long *)&ctr->rel_count[r % 3] == 0) break;  // the same answer in every CTA
+        const uint64_t n = *(volatile unsigned long long *)&ctr->rel_count[r % 3];
+        if (n == 0) break;  // the same answer in every CTA
         if (t0) ctr->rel_count[(r + 2) % 3] = 0;
-        release_round_range(I, D, fr[r & 1], fr[(r + 1) & 1], &ctr->rel_count[r % 3], &ctr->rel_count[(r + 1) % 3],
-                            cta_base, stride);
+        release_round_range(I, D, fr[r & 1], fr[(r + 1) & 1], n, free_base, &ctr->rel_count[(r + 1) % 3], cta_base, stride);
+        free_base += n;
         if (!bar.sync()) return;
     }
     if (t0) {  // set r % 3 was read by every CTA before its last barrier, or is the empty one
