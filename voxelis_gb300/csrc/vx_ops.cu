@@ -580,8 +580,7 @@ __device__ __forceinline__ bool set_claim(const DevInterner &I, bool find, const
     uint64_t pos = h & I.table_mask;
     uint32_t probes = 0, tomb = 0, rounds = 0;
     for (;;) {
-        uint64_t s = ld_probe(I.table + pos);
-        if (s == SLOT_TOMB && tomb == 0) tomb = probes + 1;
+        uint64_t s = probe_sector(I, tag, pos, probes, tomb);
         if (s == SLOT_EMPTY) {
             if (tomb) {
                 probes = tomb - 1;
@@ -608,8 +607,11 @@ __device__ __forceinline__ bool set_claim(const DevInterner &I, bool find, const
             }
             if (key_equal(I, (uint32_t)s, c, types, mask, id)) return true;
         }
-        pos = (pos + 1) & I.table_mask;
-        if (++probes > I.max_probes) {
+        if (s != SLOT_TOMB) {
+            pos = (pos + 1) & I.table_mask;
+            ++probes;
+        }
+        if (probes > I.max_probes) {
             set_error(I, ERR_TABLE_FULL, 1);
             return false;
         }

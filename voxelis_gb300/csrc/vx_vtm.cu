@@ -340,18 +340,19 @@ __device__ void vtm_insert(const DevInterner &I, uint32_t idx, const uint64_t c[
                            uint64_t h) {
     const uint32_t tag = slot_tag(h);
     uint64_t pos = h & I.table_mask;
-    for (uint32_t probes = 0; probes <= I.max_probes; ++probes) {
-        uint64_t s = ld_probe(I.table + pos);
+    uint32_t probes = 0, tomb = 0;
+    while (probes <= I.max_probes) {
+        uint64_t s = probe_sector(I, tag, pos, probes, tomb);
         if (s == SLOT_EMPTY) {
             const unsigned long long prev =
                 atom_cas_acq_rel((unsigned long long *)(I.table + pos), SLOT_EMPTY, make_slot(tag, idx));
             if (prev == SLOT_EMPTY) return;
             s = prev;
         }
-        if ((uint32_t)(s >> 32) == tag && s != SLOT_TOMB && (uint32_t)s != IDX_BUSY &&
-            key_equal(I, (uint32_t)s, c, types, mask))
-            return;
+        if (s == SLOT_TOMB) continue;
+        if ((uint32_t)(s >> 32) == tag && (uint32_t)s != IDX_BUSY && key_equal(I, (uint32_t)s, c, types, mask)) return;
         pos = (pos + 1) & I.table_mask;
+        ++probes;
     }
     set_error(I, ERR_TABLE_FULL, 52);
 }
