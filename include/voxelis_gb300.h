@@ -264,6 +264,17 @@ int vx_stage_spheres(int chunk_depth, int32_t nx, int32_t ny, int32_t nz, uint32
                      const int32_t *radii, const uint32_t *values, uint64_t cap_items, uint32_t *item_chunks,
                      uint64_t cap_records, uint32_t *rec_item, uint32_t *rec_group, uint8_t *rec_set,
                      uint8_t *rec_clear, uint16_t *rec_vals, uint64_t *n_items, uint64_t *n_records);
+/* The same on the interner's stream, written by the device: the records and, for each item, its tree handle, its
+ * chunk and the sphere that touches it. plan_host: 32 * cap_items bytes of pinned memory that stay as they are
+ * until the stream has passed, plan_dev: as many of device memory; rec_vals_dev and plan_dev are 16-byte aligned. The
+ * counts are known when it returns. VX_E_UNSUPPORTED, and nothing queued, when a chunk is touched by two of the
+ * spheres or chunk_depth is above 8: vx_stage_spheres takes those. */
+int vx_stage_spheres_async(vx_interner *it, const vx_world *world, uint32_t n, const int32_t *centers,
+                           const int32_t *radii, const uint32_t *values, uint64_t cap_items, void *plan_host,
+                           void *plan_dev, uint32_t *item_trees_dev, uint32_t *item_chunks_dev,
+                           uint32_t *item_ranks_dev, uint64_t cap_records, uint32_t *rec_item_dev,
+                           uint32_t *rec_group_dev, uint8_t *rec_set_dev, uint8_t *rec_clear_dev,
+                           uint16_t *rec_vals_dev, uint64_t *n_items, uint64_t *n_records);
 /* n host -> device copies (dst_dev[k] <- src_host[k], bytes[k]) on the interner's stream, one
  * cudaMemcpyAsync each: a serving loop stages a wave's arrays with one call. No reference
  * counterpart (host plumbing of the serving loop). */

@@ -157,6 +157,7 @@ GPU_SIGNATURES = {
     "world_hold_async": [_P, _P, _U32, _P, _P, _P, _P, _P],
     "world_get_at_async": [_P, _P, _U64, _P, _P, _P, _P, _P, _U32],
     "world_release_async": [_P, _P, _U32, _P, _P, _P],
+    "stage_spheres_async": [_P, _P, _U32, _P, _P, _P, _U64, _P, _P, _P, _P, _P, _U64, _P, _P, _P, _P, _P, _PU64, _PU64],
     "copy_to_device_async": [_P, _U32, _P, _P, _P],
     "tune_get": [_P, _PI, _PI],
     "tune_set_launch": [_P, _I],

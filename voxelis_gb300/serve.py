@@ -17,8 +17,9 @@ reference each) and the get reads every chunk edited at or after its cut at the 
 (vx_world_get_at_async); the holds are released after the wave's gets (vx_world_release_async). So
 every get sees exactly the edits that arrived before it, every result equals the one-by-one result,
 and a backlog forms large waves. Requests that arrive while a wave is on the GPU are admitted into
-the next one, which is staged on the host (vx_stage_spheres, pinned buffers, async copies) while the
-device works. Edits are admitted only while the interner's free node headroom covers a conservative
+the next one. The device writes a wave's records itself from its spheres (vx_stage_spheres_async); the
+host stages (vx_stage_spheres, pinned buffers, async copies) only worlds of deep chunks and requests that
+name too few chunks. Edits are admitted only while the interner's free node headroom covers a conservative
 estimate of the nodes they can create; replaced roots are released (nodes recycled with a new
 generation) by every apply, and the branch table is rebuilt from live nodes when deletions pile up
 (vx_interner_maintain).
@@ -30,7 +31,8 @@ import time
 import numpy as np
 
 from . import workloads as W
-from ._abi import VX_PATCH_P1, VX_PATCH_P4, VX_PATCH_P5, vx_interner_stats, vx_world, gpu_lib
+from ._abi import (VX_E_UNSUPPORTED, VX_PATCH_P1, VX_PATCH_P4, VX_PATCH_P5, vx_interner_stats, vx_world,
+                   gpu_lib)
 
 EDIT, GET = 0, 1
 
@@ -142,7 +144,7 @@ class Server:
         self.hset = [dict(items=pin(cap_items, torch.int32), item_trees=pin(cap_items, torch.int32),
                           ri=pin(cap_recs, torch.int32), rg=pin(cap_recs, torch.int32), rs=pin(cap_recs, torch.uint8),
                           rc=pin(cap_recs, torch.uint8), rv=pin(cap_recs * 8, torch.int16),
-                          ranks=pin(cap_items, torch.int32)) for _ in range(2)]
+                          ranks=pin(cap_items, torch.int32), plan=pin(8 * cap_items, torch.int32)) for _ in range(2)]
         for k, hs in enumerate(self.hset):  # numpy views of the pinned buffers (no torch call per wave)
             hs["k"] = k
             hs["np"] = {"items": hs["items"].numpy(), "item_trees": hs["item_trees"].numpy(),
@@ -167,6 +169,11 @@ class Server:
         self.copies = [{"dst": np.array([t.data_ptr() for t in dsts], np.uint64),
                         "src": np.array([hs[k].data_ptr() for k in names], np.uint64),
                         "bytes": np.zeros(len(names), np.uint64)} for hs in self.hset]
+        # the addresses vx_stage_spheres_async takes behind the spheres (the plan's pinned side is the set's)
+        self.d_plan = torch.empty(8 * cap_items, dtype=torch.int32, device=dev)
+        self.stage_items = [C.c_void_p(t.data_ptr()) for t in (self.d_plan, self.d_item_trees, self.d_item_chunks,
+                                                               self.d_ranks)]
+        self.stage_recs = [C.c_void_p(t.data_ptr()) for t in (self.d_ri, self.d_rg, self.d_rs, self.d_rc, self.d_rv)]
         self.d_pts = torch.empty((max_wave_gets, self.ppg, 3), dtype=torch.int32, device=dev)
         self.pool_ptr = [p.data_ptr() for p in self.pool_h]
         self.get_dst = np.array([self.d_pts[k].data_ptr() for k in range(max_wave_gets)], np.uint64)
@@ -224,6 +231,30 @@ class Server:
         return edits, gets, taken
 
     # -- staging and launch ----------------------------------------------------------------------------
+    def _stage_on_host(self, hs, edits, cen, rad, val, hold):
+        """The wave's records written by the host into the pinned set `hs` and copied: (items, records)."""
+        w = self.w
+        P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+        ni, nr = C.c_uint64(), C.c_uint64()
+        st = self.stage(w.depth, w.nx, w.ny, w.nz, len(edits), C.c_void_p(cen.ctypes.data), C.c_void_p(rad.ctypes.data),
+                        C.c_void_p(val.ctypes.data), C.c_uint64(self.cap_items), P(hs["items"]),
+                        C.c_uint64(self.cap_recs), P(hs["ri"]), P(hs["rg"]), P(hs["rs"]), P(hs["rc"]),
+                        P(hs["rv"]), C.byref(ni), C.byref(nr))
+        if st != 0:
+            raise RuntimeError("vx_stage_spheres failed: %d" % st)
+        ni, nr = ni.value, nr.value
+        if ni:
+            hn = hs["np"]
+            np.take(w.trees.view(np.int32), hn["items"][:ni], out=hn["item_trees"][:ni])
+            if hold:  # each item's chunk belongs to exactly one of the wave's edits: its rank
+                rank_of = {c: k for k, e in enumerate(edits) for c in e["chunks"]}
+                hn["ranks"][:ni] = [rank_of[int(c)] for c in hn["items"][:ni]]
+            cp = self.copies[hs["k"]]
+            hb = 4 * ni if hold else 0
+            cp["bytes"][:] = (4 * ni, 4 * nr, 4 * nr, nr, nr, 16 * nr, hb, hb)
+            w.call("copy_to_device_async", 8, cp["dst"].ctypes.data, cp["src"].ctypes.data, cp["bytes"].ctypes.data)
+        return ni, nr
+
     def launch(self, edits, gets):
         """Queues a wave: its edits as one batched apply, then its gets (each a (request, cut) pair),
         with the edited chunks' roots held for the gets that must not see every edit."""
@@ -234,36 +265,28 @@ class Server:
         ni = 0
         hold = bool(edits) and any(cut < len(edits) for _, cut in gets)
         if edits:
-            n = len(edits)
             cen = np.array([e["center"] for e in edits], np.int32)
             rad = np.array([e["radius"] for e in edits], np.int32)
             val = np.array([e["value"] for e in edits], np.uint32)
             ni, nr = C.c_uint64(), C.c_uint64()
-            st = self.stage(w.depth, w.nx, w.ny, w.nz, n, C.c_void_p(cen.ctypes.data), C.c_void_p(rad.ctypes.data),
-                            C.c_void_p(val.ctypes.data), C.c_uint64(self.cap_items), P(hs["items"]),
-                            C.c_uint64(self.cap_recs), P(hs["ri"]), P(hs["rg"]), P(hs["rs"]), P(hs["rc"]),
-                            P(hs["rv"]), C.byref(ni), C.byref(nr))
-            if st != 0:
+            st = self.lib.status("stage_spheres_async", w.h, C.byref(w.wdesc), len(edits), cen.ctypes.data, rad.ctypes.data,
+                                 val.ctypes.data, self.cap_items, P(hs["plan"]), *self.stage_items, self.cap_recs,
+                                 *self.stage_recs, C.byref(ni), C.byref(nr))
+            if st == VX_E_UNSUPPORTED:
+                ni, nr = self._stage_on_host(hs, edits, cen, rad, val, hold)
+            elif st != 0:
                 raise RuntimeError("vx_stage_spheres failed: %d" % st)
-            ni, nr = ni.value, nr.value
+            else:
+                ni, nr = ni.value, nr.value
             self.records += nr
             self.items += ni
             hold = hold and ni > 0
             if ni:
-                hn = hs["np"]
-                np.take(w.trees.view(np.int32), hn["items"][:ni], out=hn["item_trees"][:ni])
-                if hold:  # each item's chunk belongs to exactly one of the wave's edits: its rank
-                    rank_of = {c: k for k, e in enumerate(edits) for c in e["chunks"]}
-                    hn["ranks"][:ni] = [rank_of[int(c)] for c in hn["items"][:ni]]
-                cp = self.copies[hs["k"]]
-                hb = 4 * ni if hold else 0
-                cp["bytes"][:] = (4 * ni, 4 * nr, 4 * nr, nr, nr, 16 * nr, hb, hb)
-                w.call("copy_to_device_async", 8, cp["dst"].ctypes.data, cp["src"].ctypes.data, cp["bytes"].ctypes.data)
                 if hold:
                     w.call("world_hold_async", C.byref(w.wdesc), ni, P(self.d_item_chunks), P(self.d_ranks),
                            P(self.d_held), P(w.old_roots), P(w.edit_rank))
                 w.call("apply_groups_async", ni, P(self.d_item_trees), P(self.d_flags), P(self.d_fill), nr,
-                       P(self.d_ri), P(self.d_rg), P(self.d_rs), P(self.d_rc), P(self.d_rv), None, w.depth)
+                       *self.stage_recs, None, w.depth)
         if gets:  # the gets' point sets in one call, then one batched world get each
             ng = len(gets)
             self.points += ng * self.ppg
