@@ -237,9 +237,10 @@ int vx_trees_set_many(vx_interner *it, uint64_t n, const vx_tree *trees, const i
 int vx_tune_set(vx_interner *it, int apply_threads, int apply_blocks_per_sm);
 int vx_tune_get(vx_interner *it, int *apply_threads, int *apply_blocks_per_sm);
 /* How a batched apply is launched (no counterpart in the reference; autotuned): 1 (the default) runs
- * the whole apply, its level passes and the release of the replaced roots as one cooperative launch
- * whose phases meet at grid barriers (blocks per SM capped by what can be resident); 0 launches one
- * kernel per phase. Results are identical. */
+ * the whole apply, its level passes and the release of the replaced roots as one launch: one cluster for a small
+ * apply, else a cooperative launch whose phases meet at grid barriers (blocks per SM capped by what can be
+ * resident), and a kernel per phase for the sizes at which that is faster; 0 launches one kernel per phase at
+ * every size. Results are identical. */
 int vx_tune_set_launch(vx_interner *it, int single_launch);
 int vx_tune_get_launch(vx_interner *it, int *single_launch);
 /* Geometry of the dense builds' quad memo (no counterpart in the reference; autotuned): about the
