@@ -246,50 +246,60 @@ __device__ uint64_t seq_branch(Seq &S, const uint64_t c[8], uint32_t types, uint
     return INVALID_ID;
 }
 
-// dec_ref_recursive (interner/mod.rs:419-534) with its fixed queue (grown under P3), by one CTA of
-// kSeqThreads: 32 queue entries at a time, 8 threads each (one per child), with the queue, the counts and
+// dec_ref_recursive (interner/mod.rs:419-534) with its fixed queue (grown under P3), by one CTA: a step's
+// queue entries at a time, 8 threads each (one per child), with the queue, the counts and
 // the order of the free list as the one-by-one loop leaves them. A child whose references all come from
 // this step's entries dies and is queued where its last reference stands in the order of (entry, child);
 // the occurrences of a dying child find that place through a small shared table. Entries of one step do
 // not name each other (a queued node has lost every reference), and counts that say otherwise end the
 // call as the underflow they are.
 // Bound by the latency of a step's dependent loads (count and children, the children's counts, the table
-// slot): clearing an edited 32^3 chunk took 2030 us in one thread, 108 us like this.
-constexpr int kSeqThreads = 256;
-constexpr uint32_t kSeqLast = 512;  // slots of the table of dying children (at most 256 distinct ones)
-constexpr uint32_t kSeqRing = 512;  // queue entries also kept in shared memory, the newest ones
+// slot), about 2 us: clearing an edited 32^3 chunk took 2030 us in one thread, 108 us in steps of 32 entries. While
+// more than 32 entries wait a step takes 128 (a CTA of 1024): 76 us against 110 for 4000 edited voxels of 32^3, 242
+// against 467 for 20000 of 64^3; a few nodes are released by 256 threads as before (37 us, 45 when all 1024 took part).
+constexpr int kSetThreads = 256;   // releases of a replaced path: narrow steps only
+constexpr int kFillThreads = 1024;  // releases of whole trees
 
+template <int kCta>
 struct SeqShared {
-    uint64_t ring[kSeqRing];
-    uint32_t key[kSeqLast], last[kSeqLast];  // node index + 1; last place of it among (entry, child)
-    uint32_t pushes[kSeqThreads / 32], deaths[kSeqThreads / 32];
-    unsigned long long w, free_count;  // end of the queue; length of the free list
+    static constexpr uint32_t kRing = 2 * kCta;  // queue entries also kept in shared memory, the newest ones
+    static constexpr uint32_t kLast = 2 * kCta;  // slots of the table of dying children
+    static constexpr int kHomeShift = kCta == 256 ? 23 : 21;
+    static_assert(kLast == 1u << (32 - kHomeShift), "the table's hash fills it");
+    uint64_t ring[kRing];
+    uint32_t key[kLast], last[kLast];  // node index + 1; last place of it among (entry, child)
+    uint32_t pushes[kCta / 32], deaths[kCta / 32];
+    unsigned long long r, w, free_count;  // place and end of the queue; length of the free list
     int ok;
 };
 
-// The whole CTA calls it; S.ok and the queue are the same in every thread.
-__device__ void seq_release(Seq &S, SeqShared &sh, uint64_t root) {
+// Barrier of the kN threads that take part in a step.
+template <int kN, int kCta>
+__device__ __forceinline__ void seq_bar() {
+    if (kN == kCta)
+        __syncthreads();
+    else
+        asm volatile("bar.sync 1, %0;" ::"n"(kN) : "memory");
+}
+
+// Steps of kN / 8 entries by the CTA's first kN threads, until the queue is empty or its length asks for the
+// other width. S.ok and the queue are the same in every thread.
+template <int kN, int kCta>
+__device__ void seq_steps(Seq &S, SeqShared<kCta> &sh) {
     const DevInterner &I = S.I;
     const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, e = tid >> 3, k = tid & 7u;
     const unsigned lt = (1u << lane) - 1u;
-    for (uint32_t s = tid; s < kSeqLast; s += kSeqThreads) sh.key[s] = 0, sh.last[s] = 0;
-    if (tid == 0) {
-        sh.ring[0] = root;
-        sh.w = 1;
-        sh.free_count = I.ctr->free_count;
-        sh.ok = 1;
-    }
-    __syncthreads();
-    for (uint64_t r = 0;;) {
+    for (uint64_t r = sh.r;;) {
         const uint64_t w = sh.w, fc = sh.free_count;
         if (r >= w || !sh.ok) break;
-        const uint32_t m = w - r < kSeqThreads / 8 ? (uint32_t)(w - r) : kSeqThreads / 8;
+        if (kCta != kSetThreads && (w - r > kSetThreads / 8) != (kN == kCta)) break;
+        const uint32_t m = w - r < kN / 8 ? (uint32_t)(w - r) : kN / 8;
         const bool have = e < m;
         uint64_t child = EMPTY_ID, node = 0, h = 0;
         uint32_t ref = 0, gen = 0, ci = 0;
         if (have) {
             const uint64_t at = r + e;
-            ci = id_index(w - at <= kSeqRing ? sh.ring[at % kSeqRing] : __ldcg((const unsigned long long *)S.queue + at));
+            ci = id_index(w - at <= sh.kRing ? sh.ring[at % sh.kRing] : __ldcg((const unsigned long long *)S.queue + at));
             ref = __ldcg(I.refcount + ci);
             child = ld_cg(I.children + 8ull * ci + k);
             if (k == 0) {
@@ -303,10 +313,10 @@ __device__ void seq_release(Seq &S, SeqShared &sh, uint64_t root) {
         const uint32_t cc = id_index(child);
         const unsigned rec = __ballot_sync(0xFFFFFFFFu, dying && k == 0);
         if (lane == 0) sh.deaths[warp] = __popc(rec);
-        __syncthreads();  // every record of this step has been read
+        seq_bar<kN, kCta>();  // every record of this step has been read
         uint32_t gone = 0, first = 0;
 #pragma unroll
-        for (unsigned x = 0; x < kSeqThreads / 32; ++x) {
+        for (unsigned x = 0; x < kN / 32; ++x) {
             if (x < warp) first += sh.deaths[x];
             gone += sh.deaths[x];
         }
@@ -328,35 +338,35 @@ __device__ void seq_release(Seq &S, SeqShared &sh, uint64_t root) {
         }
         const unsigned tomb = __ballot_sync(0xFFFFFFFFu, dying && k == 0 && id_is_branch(node));
         if (lane == 0 && tomb) atomicAdd(&I.ctr->tombstones, (unsigned long long)__popc(tomb));
-        const uint32_t home = (cc * 0x9E3779B1u) >> 23;
+        const uint32_t home = (cc * 0x9E3779B1u) >> sh.kHomeShift;
         if (child != EMPTY_ID && old == 1)  // the last reference: the child dies
-            for (uint32_t slot = home; atomicCAS(sh.key + slot, 0u, cc + 1u) != 0u;) slot = (slot + 1) & (kSeqLast - 1u);
-        __syncthreads();
+            for (uint32_t slot = home; atomicCAS(sh.key + slot, 0u, cc + 1u) != 0u;) slot = (slot + 1) & (sh.kLast - 1u);
+        seq_bar<kN, kCta>();
         // the occurrences of each dying child find the last place of it
         uint32_t slot = home;
         bool dead = false;
         if (child != EMPTY_ID)
-            for (;; slot = (slot + 1) & (kSeqLast - 1u)) {  // at most 256 keys in 512 slots
+            for (;; slot = (slot + 1) & (sh.kLast - 1u)) {  // half of the slots stay free
                 const uint32_t t = *(volatile uint32_t *)(sh.key + slot);
                 dead = t == cc + 1u;
                 if (dead || t == 0) break;
             }
         if (dead) atomicMax(sh.last + slot, tid);
-        __syncthreads();
+        seq_bar<kN, kCta>();
         const bool push = dead && sh.last[slot] == tid;
         const unsigned b = __ballot_sync(0xFFFFFFFFu, push);
         if (lane == 0) sh.pushes[warp] = __popc(b);
-        __syncthreads();
+        seq_bar<kN, kCta>();
         uint32_t before = 0, all = 0;
 #pragma unroll
-        for (unsigned x = 0; x < kSeqThreads / 32; ++x) {
+        for (unsigned x = 0; x < kN / 32; ++x) {
             if (x < warp) before += sh.pushes[x];
             all += sh.pushes[x];
         }
         const bool full = w + all > S.queue_cap;
         if (push && !full) {
             const uint64_t at = w + before + __popc(b & lt);
-            sh.ring[at % kSeqRing] = child;
+            sh.ring[at % sh.kRing] = child;
             S.queue[at] = child;
             I.refcount[cc] = 1;  // its queue entry takes the last one
         }
@@ -373,9 +383,32 @@ __device__ void seq_release(Seq &S, SeqShared &sh, uint64_t root) {
             sh.w = w + all;
         }
         r += m;
-        __syncthreads();
+        if (tid == 0) sh.r = r;
+        seq_bar<kN, kCta>();
     }
-    if (tid == 0) I.ctr->free_count = sh.free_count;
+}
+
+// The whole CTA calls it.
+template <int kCta>
+__device__ void seq_release(Seq &S, SeqShared<kCta> &sh, uint64_t root) {
+    const unsigned tid = threadIdx.x;
+    for (uint32_t s = tid; s < sh.kLast; s += kCta) sh.key[s] = 0, sh.last[s] = 0;
+    if (tid == 0) {
+        sh.ring[0] = root;
+        sh.r = 0;
+        sh.w = 1;
+        sh.free_count = S.I.ctr->free_count;
+        sh.ok = 1;
+    }
+    __syncthreads();
+    for (;;) {
+        if (tid < kSetThreads) seq_steps<kSetThreads, kCta>(S, sh);
+        __syncthreads();
+        if (kCta == kSetThreads || sh.r >= sh.w || !sh.ok) break;
+        seq_steps<kCta, kCta>(S, sh);
+        __syncthreads();  // every thread has seen the end of its steps before the next ones move it
+    }
+    if (tid == 0) S.I.ctr->free_count = sh.free_count;
     S.ok = sh.ok != 0;
     __syncthreads();
 }
@@ -514,9 +547,9 @@ __device__ uint64_t seq_remove(Seq &S, uint64_t root, int32_t x, int32_t y, int3
 
 // VoxTree::set (voxtree.rs:163-260). status: 0 unchanged, 1 changed, -1 error. Thread 0 runs the set, the
 // CTA the release of the replaced root.
-__global__ void __launch_bounds__(kSeqThreads) tree_set_kernel(DevInterner I, uint32_t tree, int32_t x, int32_t y, int32_t z,
+__global__ void __launch_bounds__(kSetThreads) tree_set_kernel(DevInterner I, uint32_t tree, int32_t x, int32_t y, int32_t z,
                                                                uint32_t v, uint64_t *queue, uint64_t queue_cap, HostReply *r) {
-    __shared__ SeqShared sh;
+    __shared__ SeqShared<kSetThreads> sh;
     __shared__ uint64_t new_root;
     __shared__ int result;  // 0 unchanged, 1 to be installed, -1 error
     Seq S{I, queue, queue_cap, true};
@@ -884,9 +917,9 @@ __global__ void __launch_bounds__(kThreads) trees_set_garbage_kernel(DevInterner
 }
 
 // VoxTree::fill / clear (voxtree.rs:264-292). status: 1 if the tree was dirtied. One CTA.
-__global__ void __launch_bounds__(kSeqThreads) tree_fill_kernel(DevInterner I, uint32_t tree, uint32_t v, uint64_t *queue,
+__global__ void __launch_bounds__(kFillThreads) tree_fill_kernel(DevInterner I, uint32_t tree, uint32_t v, uint64_t *queue,
                                                                 uint64_t queue_cap, HostReply *r) {
-    __shared__ SeqShared sh;
+    __shared__ SeqShared<kFillThreads> sh;
     Seq S{I, queue, queue_cap, true};
     const uint64_t root = I.roots[tree];
     __syncthreads();
@@ -1996,7 +2029,7 @@ cudaError_t launch_tree_get(const DevInterner &I, uint32_t tree, int32_t x, int3
 cudaError_t launch_tree_set(const DevInterner &I, uint32_t tree, int32_t x, int32_t y, int32_t z, uint32_t v,
                             uint64_t *queue, uint64_t queue_cap, HostReply *r, cudaStream_t s) {
     count_launches(1);
-    tree_set_kernel<<<1, kSeqThreads, 0, s>>>(I, tree, x, y, z, v, queue, queue_cap, r);
+    tree_set_kernel<<<1, kSetThreads, 0, s>>>(I, tree, x, y, z, v, queue, queue_cap, r);
     return cudaGetLastError();
 }
 
@@ -2020,7 +2053,7 @@ cudaError_t launch_trees_set(const DevInterner &I, const SetCalls &c, uint64_t *
 cudaError_t launch_tree_fill(const DevInterner &I, uint32_t tree, uint32_t v, uint64_t *queue, uint64_t queue_cap,
                              HostReply *r, cudaStream_t s) {
     count_launches(1);
-    tree_fill_kernel<<<1, kSeqThreads, 0, s>>>(I, tree, v, queue, queue_cap, r);
+    tree_fill_kernel<<<1, kFillThreads, 0, s>>>(I, tree, v, queue, queue_cap, r);
     return cudaGetLastError();
 }
 
