@@ -1972,10 +1972,10 @@ cudaError_t launch_occupancy_many(const DevInterner &I, const uint8_t *grids, ui
 // Levels the table of a call skips (0: no table). n queries over n_trees trees: no more entries than an
 // eighth of the queries, so that filling them stays small beside the reads, and than kGetTableEntries; from
 // two levels up, since one saves no more than it costs; and not for calls so small that the extra launch
-// shows (131 k gets on a tree of depth 9: 15.0 us with it, 13.7 without; 1 M: 22.7 and 26.0; 16 M: 141 and
-// 264; 4 M on 4096 trees of depth 5: 45.6 and 54.2; 262 k on 64 of them: 13.9 and 13.5).
+// shows. A call and its wait on a tree of depth 9: 31.4 us with the table and 31.4 without for 524 K gets, 35.1 and
+// 37.4 for 1 M, 59 and 76 for 4 M; on 1000 trees of depth 4 30.6 and 28.3, 33.0 and 32.2, 51 and 54.
 int get_table_levels(uint64_t n, uint32_t n_trees, int max_depth) {
-    if (n < (1u << 19) || n_trees == 0) return 0;
+    if (n < (1u << 20) || n_trees == 0) return 0;
     const uint64_t most = std::min<uint64_t>(kGetTableEntries, n / 8);
     int k = 0;
     while (k < max_depth && ((uint64_t)n_trees << (3 * (k + 1))) <= most) ++k;
