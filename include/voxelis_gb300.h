@@ -239,7 +239,7 @@ int vx_tune_get(vx_interner *it, int *apply_threads, int *apply_blocks_per_sm);
 /* How a batched apply is launched (no counterpart in the reference; autotuned): 1 (the default) runs
  * the whole apply, its level passes and the release of the replaced roots as one launch: one cluster for a small
  * apply, else a cooperative launch whose phases meet at grid barriers (blocks per SM capped by what can be
- * resident), and a kernel per phase for the sizes at which that is faster; 0 launches one kernel per phase at
+ * resident), and a kernel per phase for the depths and sizes at which that is faster; 0 launches one kernel per phase at
  * every size. Results are identical. */
 int vx_tune_set_launch(vx_interner *it, int single_launch);
 int vx_tune_get_launch(vx_interner *it, int *single_launch);

@@ -11,9 +11,9 @@ PATCHES = VX_PATCH_P1 | VX_PATCH_P2 | VX_PATCH_P3 | VX_PATCH_P4 | VX_PATCH_P5
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("records", [(1 << 17) - 1, 1 << 17, (1 << 19) - 1, 1 << 19])
-def test_apply_around_the_line(oracle_lib, gpu_lib, records):
+def test_apply_around_the_line(oracle_lib, gpu_lib, records, depth=7):
     rng = np.random.default_rng(records)
-    depth, items = 7, 3
+    items = 3
     its, trees = [], []
     for lib in (oracle_lib, gpu_lib):
         its.append(VoxInterner(1 << 28, 8, PATCHES, lib=lib))
@@ -39,3 +39,9 @@ def test_apply_around_the_line(oracle_lib, gpu_lib, records):
         for key in a:
             np.testing.assert_array_equal(a[key], b[key], err_msg="%s after step %d" % (key, step))
         assert its[0].stats()["alive_nodes"] == its[1].stats()["alive_nodes"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("records", [(1 << 17) - 1, 1 << 17, (1 << 19) - 1, 1 << 19])
+def test_deep_trees_around_the_line(oracle_lib, gpu_lib, records):
+    test_apply_around_the_line(oracle_lib, gpu_lib, records, depth=8)

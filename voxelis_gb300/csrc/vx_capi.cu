@@ -512,12 +512,13 @@ int carve_apply(vx_interner *it, uint32_t n, uint64_t R, int max_depth, bool own
     return VX_OK;
 }
 
-// From this many records on, up to where the single launch shares its bottom groups out in turn, the phases run
-// faster as launches that start early (programmatic dependents) than behind grid barriers. Launches against the
-// single one, an apply: 432 against 395 us for 32 K records of a tree of depth 9, 446 against 435 for 64 K, 479
-// against 534 for 128 K, 588 against 656 for 261 K; of chunks 290 against 319 for 153 K, 431 against 455 for 399 K,
-// 485 against 488 for 580 K; 649 against 642 for 823 K, 2623 against 2279 for 6.3 M.
+// Deep trees of so many records run faster as launches that start early (programmatic dependents) than behind the
+// single launch's barriers, two a level. Launches against the single one, an apply of a tree of depth 9: 429 against
+// 388 us for 32 K records, 446 against 427 for 64 K, 486 against 515 for 128 K, 583 against 615 for 261 K; of depth 8
+// 417 against 429 for 125 K, 487 against 499 for 248 K; of depth 7 399 and 402 for 172 K. Chunks: 292 and 296 for
+// 153 K, 315 against 301 for 191 K, 431 against 425 for 399 K, 515 against 507 for 784 K.
 constexpr uint64_t kLaunchesFrom = 1ull << 17, kLaunchesTo = 1ull << 19;
+constexpr int kLaunchesDepth = 8;
 
 // The set phase (its kernels count references as they create nodes and close the allocation epoch)
 // and its release, then (P4) the clear pass with its own epoch and release. No host synchronisation.
@@ -526,7 +527,7 @@ int apply_sequence(vx_interner *it, ApplyArgs &a, bool clear_pass, bool check_de
     // the roots that die are the first dying set, retired by the first release pass; a root heads a
     // subtree of height at most max_depth, whose leaves are retired by pass max_depth + 1
     const int rounds = a.max_depth > 0 && a.max_depth < 10 ? a.max_depth + 1 : 11;
-    if (it->apply_single && (a.n_records < kLaunchesFrom || a.n_records >= kLaunchesTo)) {
+    if (it->apply_single && (a.max_depth < kLaunchesDepth || a.n_records < kLaunchesFrom || a.n_records >= kLaunchesTo)) {
         Phase ph(it, VX_PROF_APPLY);
         VX_CUDA(launch_apply_single(it->dev, a, check_depths, clear_pass, it->frontier, it->frontier + it->capacity,
                                     rounds, it->num_sms, s));
