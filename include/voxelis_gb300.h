@@ -227,7 +227,8 @@ int vx_apply_groups_async(vx_interner *it, uint32_t n_items, const vx_tree *tree
  * voxtree.rs:373-705): the same result as calling vx_tree_set(trees[k], xyz[3k..3k+2], values[k])
  * for k = 0 .. n-1 in order (value 0 removes the voxel; the DAG, reference counts and live nodes are
  * those of the one-by-one calls), in one device pass: the calls of one tree run in order, one warp
- * per tree, trees in parallel; refcounts are settled and the replaced nodes released at the end, so
+ * per tree (four calls a tree and more: one per octant of it, and the root last), trees in parallel; refcounts
+ * are settled and the replaced nodes released at the end, so
  * the calls need up to depth + 1 free nodes each until then (VX_E_OOM otherwise). changed[k] (may be
  * NULL) mirrors call k's bool result. Every position is checked first (VX_E_OOB, nothing applied). */
 int vx_trees_set_many(vx_interner *it, uint64_t n, const vx_tree *trees, const int32_t *xyz,

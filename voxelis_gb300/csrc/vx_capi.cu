@@ -1363,9 +1363,11 @@ int vx_trees_set_many(vx_interner *it, uint64_t n, const vx_tree *trees, const i
     }
     begin.push_back((uint32_t)n);
     const size_t G = group_tree.size();
-    const size_t list_cap = G + (size_t)n * (dmax + 1) + 16;  // old roots + every node the calls can create
+    const bool octants = trees_set_octants((uint32_t)G, n, it->num_sms);
+    // old roots + every node the calls can create, twice where the octants' calls may be run again in order
+    const size_t list_cap = G + (size_t)n * (dmax + 1) * (octants ? 2 : 1) + 16;
     // the arguments are laid out alike in pinned and in device memory: one copy
-    VX_CUDA(it->ws.reserve(Carve::need({G * 4, (G + 1) * 4, n * 12, n * 4, n * 4, n, G * 8, list_cap * 8})));
+    VX_CUDA(it->ws.reserve(Carve::need({G * 4, (G + 1) * 4, n * 12, n * 4, n * 4, n, G * 8, list_cap * 8, n * 8})));
     VX_CUDA(it->pinned.reserve(Carve::need({G * 4, (G + 1) * 4, n * 12, n * 4, n * 4, n})));
     Carve hc(it->pinned.p), c(it->ws.p);
     uint32_t *h_group = hc.take<uint32_t>(G), *d_group = c.take<uint32_t>(G);
@@ -1377,6 +1379,7 @@ int vx_trees_set_many(vx_interner *it, uint64_t n, const vx_tree *trees, const i
     uint8_t *ch = hc.take<uint8_t>(n), *d_changed = c.take<uint8_t>(n);
     uint64_t *d_roots = c.take<uint64_t>(G);
     uint64_t *d_list = c.take<uint64_t>(list_cap);
+    uint64_t *d_results = octants ? c.take<uint64_t>(n) : nullptr;
     cudaStream_t s = it->stream;
     std::copy(group_tree.begin(), group_tree.end(), h_group);
     std::copy(begin.begin(), begin.end(), h_begin);
@@ -1387,7 +1390,7 @@ int vx_trees_set_many(vx_interner *it, uint64_t n, const vx_tree *trees, const i
         h_vals[k] = values[o];
     }
     VX_CUDA(cudaMemcpyAsync(d_group, h_group, in_bytes, cudaMemcpyHostToDevice, s));
-    SetCalls calls{(uint32_t)G, d_group, d_begin, d_xyz, d_vals, d_order, d_changed, d_roots};
+    SetCalls calls{(uint32_t)G, d_group, d_begin, d_xyz, d_vals, d_order, d_changed, d_roots, d_results};
     {
         Phase ph(it, VX_PROF_APPLY);
         VX_CUDA(launch_trees_set(it->dev, calls, d_list, fc0, ni0, it->frontier, it->frontier + it->capacity, dmax,

@@ -229,10 +229,14 @@ struct SetCalls {
     const uint32_t *order;
     uint8_t *changed;    // per call, may be null
     uint64_t *new_root;  // per group (scratch)
+    uint64_t *results;   // per call (scratch): its octant's new id; null: one warp per tree
 };
-// Runs the calls (one warp per tree), counts the created nodes' references, moves the roots and
-// releases the first roots and the created nodes left unreferenced. fc0 / ni0: the interner's
-// free_count and next_index before the call; `list` holds n_groups + every node the calls can create.
+// Whether a call's trees are taken an octant a warp.
+bool trees_set_octants(uint32_t n_trees, uint64_t n_calls, int num_sms);
+// Runs the calls (one warp per tree or, with `results`, one per octant of each tree), counts the created
+// nodes' references, moves the roots and releases the first roots and the created nodes left unreferenced.
+// fc0 / ni0: the interner's free_count and next_index before the call; `list` holds n_groups + every node the
+// calls can create.
 cudaError_t launch_trees_set(const DevInterner &I, const SetCalls &c, uint64_t *list, unsigned long long fc0,
                              unsigned long long ni0, uint32_t *frontier_a, uint32_t *frontier_b, int max_depth,
                              int num_sms, cudaStream_t s);
