@@ -878,6 +878,7 @@ int vx_interner_create(uint64_t budget_bytes, int voxel_bits, uint32_t patch_fla
         alloc((void **)&it->seq_queue, it->seq_queue_cap * 8);
     }
     if (ok && cudaMallocHost((void **)&it->h_ctr, sizeof(DevCounters)) != cudaSuccess) ok = false;
+    if (ok && it->pinned.reserve(1) != cudaSuccess) ok = false;  // room for small calls: the first one does not wait for it
     if (ok && cudaMallocHost((void **)&it->h_reply, sizeof(HostReply)) != cudaSuccess) ok = false;
     if (ok && cudaMallocHost((void **)&it->h_live, 2 * sizeof(unsigned long long)) != cudaSuccess) ok = false;
     if (!ok || grow_tree_table(it, 1024) != cudaSuccess) {
