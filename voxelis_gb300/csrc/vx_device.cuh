@@ -50,7 +50,7 @@ constexpr uint8_t TREE_UNUSED = 0xFF;  // depth marker of a free tree slot
 
 // Bounds of every wait. The copy waits of the dense kernels (TMA tiles, and the drain of a warp's
 // own copies after giving up) always use SPIN_LIMIT; the waits on other threads (leaf creation, grid
-// barriers, scan look-back) use the interner's spin_limit and the warp-intern loop its round_limit,
+// barriers) use the interner's spin_limit and the warp-intern loop its round_limit,
 // both settable per interner (vx_interner_set_limits) and SPIN_LIMIT / ROUND_LIMIT by default.
 constexpr uint32_t SPIN_LIMIT = 1u << 22;   // bounded waits (~tens of ms with nanosleep)
 constexpr uint32_t ROUND_LIMIT = 1u << 20;  // bounded warp-intern rounds

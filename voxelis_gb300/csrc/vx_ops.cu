@@ -1,16 +1,19 @@
 // Batched reads, releases, single-voxel edits and table maintenance.
 //
 //   get_many      VoxTree::get -> get_at_depth (voxtree.rs:145-159, utils/common.rs:122-156), one
-//                 thread per query descending at most d levels through the L2-resident node array.
+//                 thread per query descending at most d levels through the L2-resident node array;
+//                 large batches start from a table of the nodes some levels below every root.
 //   release       dec_ref_recursive (interner/mod.rs:419-534) for many roots at once, breadth
 //                 first: a round decrements the children of the nodes that died in the previous
 //                 round; a child whose count reaches zero dies in the next round. Dead nodes leave
 //                 their table, are cleared, get a new generation and go on the free list
-//                 (recycle, interner/mod.rs:566-625).
+//                 (recycle, interner/mod.rs:566-625). All rounds in one cooperative launch.
 //   set / fill    VoxTree::set (voxtree.rs:163-260, 393-706) and fill/clear (voxtree.rs:264-292)
-//                 run by a single thread with the reference's own refcount order (hit: give back
-//                 the children's references, interner/mod.rs:767-772), its LIFO free list and its
-//                 32768-entry release queue (P3 lifts the limit).
+//                 by one CTA with the reference's own refcount order (hit: give back the children's
+//                 references, interner/mod.rs:767-772), its LIFO free list and its 32768-entry
+//                 release queue (P3 lifts the limit); one thread walks the path.
+//   set many      many VoxTree::set calls at once, each tree's (or octant's) in call order.
+//   to_dense      to_vec, a thread per quad; occupancy masks, a CTA per builder; serialisation.
 //   rehash        rebuilds the branch table from the live nodes once tombstones accumulate.
 #include <algorithm>
 #include <type_traits>
