@@ -462,10 +462,7 @@ __device__ __forceinline__ void bottom_records(const DevInterner &I, const Apply
                 types &= ~modified;
                 mask &= ~modified;
                 changed = 1;
-                if (mask) {
-                    want_branch = true;
-                    lod = calc_average8(cv);
-                }
+                if (mask) want_branch = true;
             }
         } else if (active && uniform) {  // voxtree.rs:826, 887-896
             bool created;
@@ -518,12 +515,14 @@ __device__ __forceinline__ void bottom_records(const DevInterner &I, const Apply
             }
             if (modified) {
                 want_branch = true;
-                lod = calc_average8(cv);
                 changed = 1;
             }
         }
         bool created;
-        const uint64_t id = warp_intern_branch_inl(I, want_branch, c, types, mask, lod, &created);
+        const uint64_t id = warp_intern_branch_inl(I, want_branch, c, types, mask, [&] {
+            if (want_branch) lod = calc_average8(cv);
+            return lod;
+        }, &created);
         if (created) add_child_refs(I, L, c, cv);
         if (want_branch) out = id;
         if (in) {
@@ -545,14 +544,16 @@ __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyA
         const bool in = p < n_par;
         uint64_t c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         uint32_t cv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        uint32_t types = 0, mask = 0, lod = 0;
-        uint32_t i = 0, r0 = 0;
+        uint32_t types = 0, mask = 0;
+        uint32_t i = 0, path = 0, d = 0;
         bool want_branch = false, changed = false;
         uint64_t out = EMPTY_ID;
         uint32_t out_val = 0;
         if (in) {
-            r0 = a.p_rec[s][p];
+            const uint32_t r0 = a.p_rec[s][p];
             i = a.rec_item[r0];
+            path = a.rec_group[r0] >> (3 * s);
+            d = a.it_depth[i];
             const uint32_t b = a.p_start[s][p];
             uint32_t e = p + 1 < n_par ? a.p_start[s][p + 1] : n_child;
             if (e > n_child) e = n_child;
@@ -631,10 +632,7 @@ __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyA
                         else
                             mask |= 1u << k;
                     }
-                if (mask) {
-                    want_branch = true;
-                    lod = calc_average8(cv);
-                }
+                if (mask) want_branch = true;
             } else {
                 const uint32_t existing_mask = eq != EMPTY_ID ? id_mask(eq) : 0u;
                 const uint32_t inv = (~mask) & 0xFFu;
@@ -671,23 +669,22 @@ __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyA
                     if (cloned) add_ref_delta(I, c[0], 7 - 2 * __popc(cloned));  // Q6
                 } else {
                     want_branch = true;
-                    lod = calc_average8(cv);
                 }
             }
         }
         bool created;
-        const uint64_t id = warp_intern_branch_inl(I, want_branch, c, types, mask, lod, &created);
+        const uint64_t id = warp_intern_branch_inl(I, want_branch, c, types, mask, [&] {
+            if (want_branch) out_val = calc_average8(cv);
+            return out_val;
+        }, &created);
         if (created) add_child_refs(I, L, c, cv);
         if (!in) continue;
-        if (want_branch) {
-            out = id;
-            out_val = lod;
-        }
-        if ((uint32_t)a.it_depth[i] - 1u == s) {
+        if (want_branch) out = id;
+        if (d - 1u == s) {
             if (changed) finish_item(I, a, mode, i, out);
         } else {
             a.e_id[s & 1][p] = out;
-            a.e_val[s & 1][p] = entry_word(out_val, a.rec_group[r0] >> (3 * s), changed);
+            a.e_val[s & 1][p] = entry_word(out_val, path, changed);
         }
     }
 }

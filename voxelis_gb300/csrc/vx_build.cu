@@ -637,7 +637,7 @@ __device__ __forceinline__ void reduce_parent_cached(const DevInterner &I, const
     if (__any_sync(0xFFFFFFFFu, need)) {
         if (need) lod = calc_average8(cv);
         bool created;
-        const uint64_t nid = warp_intern_branch_inl(I, need, c, types, mask, lod, &created);
+        const uint64_t nid = warp_intern_branch_inl(I, need, c, types, mask, [=] { return lod; }, &created);
         if (need) {
             id = nid;
             if (nid != EMPTY_ID) nc_insert(N, c, 1u, nid, lod);
@@ -1886,7 +1886,7 @@ __device__ __forceinline__ void reduce_parent_dedup(const DevInterner &I, bool i
     const bool probe = is_branch && !follow;
     const uint32_t lod = probe ? calc_average8(cv) : 0;
     bool created;
-    uint64_t id = warp_intern_branch_inl(I, probe, c, types, mask, lod, &created, h);
+    uint64_t id = warp_intern_branch_inl(I, probe, c, types, mask, [=] { return lod; }, &created, h);
     if (created_out) *created_out = created;
     const uint64_t lead_id = __shfl_sync(0xFFFFFFFFu, id, leader);
     const uint32_t lead_lod = __shfl_sync(0xFFFFFFFFu, lod, leader);

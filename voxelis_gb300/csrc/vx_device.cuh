@@ -393,8 +393,12 @@ __device__ __forceinline__ uint64_t probe_sector(const DevInterner &I, uint32_t 
 #ifndef VX_INTERN_INLINE
 #define VX_INTERN_INLINE __noinline__
 #endif
+// lod_of() gives the LOD value of a new node. It is called once, behind the first probe, so that a caller whose
+// children's values are still on their way does not wait for them before it (an apply of 261 K records of a tree of
+// depth 9 577 us against 588, of 16 K 363 against 373).
+template <class Lod>
 __device__ __forceinline__ uint64_t warp_intern_branch_inl(const DevInterner &I, bool active, const uint64_t c[8],
-                                                           uint32_t types, uint32_t mask, uint32_t lod, bool *created,
+                                                           uint32_t types, uint32_t mask, Lod lod_of, bool *created,
                                                            uint64_t h_in = 0) {
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t tm = (types << 8) | mask;
@@ -414,6 +418,7 @@ __device__ __forceinline__ uint64_t warp_intern_branch_inl(const DevInterner &I,
         pos = h & I.table_mask;
     }
     bool claimed = false;
+    uint32_t lod = 0;
     for (uint32_t round = 0;; ++round) {
         bool waiting = false;
         if (!done && !claimed) {
@@ -453,6 +458,7 @@ __device__ __forceinline__ uint64_t warp_intern_branch_inl(const DevInterner &I,
                 }
             }
         }
+        if (round == 0) lod = lod_of();
         const bool last = round >= I.round_limit;
         const unsigned cm = __ballot_sync(0xFFFFFFFFu, claimed);
         if (cm && (last || !__any_sync(0xFFFFFFFFu, !done && !claimed && !waiting))) {
@@ -496,7 +502,7 @@ __device__ __forceinline__ uint64_t warp_intern_branch_inl(const DevInterner &I,
 static __device__ VX_INTERN_INLINE uint64_t warp_intern_branch(const DevInterner &I, bool active, const uint64_t c[8],
                                                        uint32_t types, uint32_t mask, uint32_t lod, bool *created,
                                                        uint64_t h_in = 0) {
-    return warp_intern_branch_inl(I, active, c, types, mask, lod, created, h_in);
+    return warp_intern_branch_inl(I, active, c, types, mask, [=] { return lod; }, created, h_in);
 }
 
 // Find-or-create of the leaf for value v (v != 0) through the direct-mapped leaf table.
