@@ -488,7 +488,7 @@ int carve_apply(vx_interner *it, uint32_t n, uint64_t R, int max_depth, bool own
         a.it_old = c.take<uint64_t>(n);
         a.it_panic = c.take<uint8_t>(n);
         a.it_changed = c.take<uint8_t>(n);
-        a.release_list = c.take<uint64_t>(n);
+        a.release_list = c.take<uint64_t>(2 * (size_t)n);  // old roots of the set phase, and of the clear pass
         a.part = c.take<uint32_t>((size_t)kPartWords * ctas);
         a.warp_off = c.take<uint32_t>((size_t)kPlanWords * ctas * 16);
         a.level_n = c.take<uint32_t>(kPartWords);
@@ -536,12 +536,13 @@ int apply_sequence(vx_interner *it, ApplyArgs &a, bool clear_pass, bool check_de
     for (int mode = 0; mode < (clear_pass ? 2 : 1); ++mode) {
         {
             PhaseSwitch ps(it, VX_PROF_BOTTOM, VX_PROF_APPLY);
-            VX_CUDA(launch_apply(it->dev, a, mode, check_depths, it->num_sms, s, &PhaseSwitch::next, &ps));
+            VX_CUDA(launch_apply(it->dev, a, mode, check_depths, clear_pass && mode == 0, it->num_sms, s, &PhaseSwitch::next,
+                                 &ps));
         }
         {
             Phase ph(it, VX_PROF_RELEASE);
             VX_CUDA(launch_release(it->dev, a.release_list, it->frontier, it->frontier + it->capacity, it->capacity,
-                                   rounds, it->num_sms, s));
+                                   rounds, it->num_sms, s, clear_pass && mode == 0));
         }
     }
     return VX_OK;

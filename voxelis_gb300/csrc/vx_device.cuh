@@ -639,6 +639,8 @@ struct GridBarrier {
 constexpr int kScRelease = 3;
 // Slot of the free list's length at the start of the release rounds (written before the barrier in front of them).
 constexpr int kScFreeBase = 4;
+// Slot that says whether the release of an apply's set phase waits for that of its clear pass.
+constexpr int kScDefer = 5;
 
 __device__ __forceinline__ void push_dying(uint32_t *list, unsigned long long *count, bool push, uint32_t idx) {
     const unsigned m = __ballot_sync(0xFFFFFFFFu, push);

@@ -122,22 +122,24 @@ struct ApplyArgs {
     uint64_t *e_id[2];
     uint32_t *e_val[2];
     uint32_t *it_first;          // [n_items + 1] first record of each item (host staging of an apply)
-    uint64_t *release_list;      // [n_items]
+    uint64_t *release_list;      // [2 * n_items]
 };
 // Most CTAs of a launch (sizes part and warp_off).
 uint32_t apply_max_ctas(int num_sms, int blocks_per_sm);
 // The set phase (mode 0, with the item depth check when check_depths) or the clear pass (mode 1) in one
 // launch per phase; the caller releases the replaced roots. levels_begin(levels_ctx), when given, runs on
 // the host between the bottom groups' launch and the levels' (the profiler marks its phases there).
-cudaError_t launch_apply(const DevInterner &I, const ApplyArgs &a, int mode, bool check_depths, int num_sms, cudaStream_t s,
+// With clear_follows, the release between the two may wait for the clear pass's (launch_release, may_wait).
+cudaError_t launch_apply(const DevInterner &I, const ApplyArgs &a, int mode, bool check_depths, bool clear_follows,
+                         int num_sms, cudaStream_t s,
                          void (*levels_begin)(void *) = nullptr, void *levels_ctx = nullptr);
 // The same sequence (with the clear pass when clear_pass and the release of the replaced roots in `rounds`
 // rounds) as one launch whose phases are separated by barriers.
 cudaError_t launch_apply_single(const DevInterner &I, const ApplyArgs &a, bool check_depths, bool clear_pass,
                                 uint32_t *frontier_a, uint32_t *frontier_b, int rounds, int num_sms, cudaStream_t s);
 // Counter slots (DevCounters::scratch indices).
-enum : int { SC_RELEASE = 3, SC_FREE_BASE = 4, SC_REF_DONE = 6, SC_DONE = 7 };
-static_assert(SC_RELEASE == kScRelease && SC_FREE_BASE == kScFreeBase, "release slots shared with vx_device.cuh");
+enum : int { SC_RELEASE = 3, SC_FREE_BASE = 4, SC_DEFER = 5, SC_REF_DONE = 6, SC_DONE = 7 };
+static_assert(SC_RELEASE == kScRelease && SC_FREE_BASE == kScFreeBase && SC_DEFER == kScDefer, "release slots shared with vx_device.cuh");
 
 // ---- reads, releases, single-voxel operations, maintenance (vx_ops.cu) -------------------------
 // table (kGetTableEntries words of scratch) and k = get_table_levels(...): the nodes k levels below the roots
@@ -206,7 +208,7 @@ cudaError_t launch_vtm_place(const DevInterner &I, const uint8_t *bytes, const V
 // Releases the roots listed in `list` (count at ctr->scratch[SC_RELEASE]) with `rounds`
 // breadth-first rounds, using two frontier buffers of `frontier_cap` entries.
 cudaError_t launch_release(const DevInterner &I, uint64_t *list, uint32_t *frontier_a, uint32_t *frontier_b,
-                           uint64_t frontier_cap, int rounds, int num_sms, cudaStream_t s);
+                           uint64_t frontier_cap, int rounds, int num_sms, cudaStream_t s, bool may_wait = false);
 // One-tree calls answer in pinned host memory, valid once the stream has been waited for.
 struct HostReply {
     int status;

@@ -97,8 +97,9 @@ __global__ void __launch_bounds__(kThreads) get_kernel(DevInterner I, uint64_t n
 // The listed roots and then rounds until no node dies, one cooperative launch with a grid barrier after each
 // (a launch per round, empty ones too, took 18 us a round on the few hundred nodes of a served wave).
 __global__ void __launch_bounds__(kThreads) release_kernel(DevInterner I, const uint64_t *list, uint32_t *frontier_a,
-                                                           uint32_t *frontier_b, int rounds) {
+                                                           uint32_t *frontier_b, int rounds, int may_wait) {
     extern __shared__ uint32_t release_mem[];
+    if (may_wait && *(volatile unsigned long long *)&I.ctr->scratch[SC_DEFER]) return;  // the list waits for the next release
     const uint64_t cta_base = (uint64_t)blockIdx.x * blockDim.x, stride = (uint64_t)gridDim.x * blockDim.x;
     const bool t0 = cta_base + threadIdx.x == 0;
     DevCounters *ctr = I.ctr;
@@ -2164,11 +2165,12 @@ cudaError_t launch_get_many(const DevInterner &I, uint64_t n, const uint32_t *tr
 }
 
 cudaError_t launch_release(const DevInterner &I, uint64_t *list, uint32_t *frontier_a, uint32_t *frontier_b,
-                           uint64_t frontier_cap, int rounds, int num_sms, cudaStream_t s) {
+                           uint64_t frontier_cap, int rounds, int num_sms, cudaStream_t s, bool may_wait) {
     (void)frontier_cap;
     DevInterner Ic = I;
     const uint64_t *l = list;
-    void *args[] = {&Ic, &l, &frontier_a, &frontier_b, &rounds};
+    int wait = may_wait ? 1 : 0;
+    void *args[] = {&Ic, &l, &frontier_a, &frontier_b, &rounds, &wait};
     count_launches(1);
     // two CTAs an SM are resident at any register and shared-memory use of the kernel
     return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(release_kernel), dim3((unsigned)num_sms * 2),
