@@ -116,7 +116,7 @@ int vx_interner_destroy(vx_interner *it);
 /* Bounds of the device's waits for this interner (no counterpart in the reference, whose waits
  * cannot fail): max_probes branch-table probes per insert before VX_E_TABLE_FULL (at most the table's
  * slots; 1..65536 by default), round_limit rounds of the warp-cooperative insert loop and spin_limit
- * iterations of a wait on another thread (a leaf being created, a grid barrier, a scan's look-back)
+ * iterations of a wait on another thread (a leaf being created, a grid barrier)
  * before VX_E_TIMEOUT. Later calls use the new values; every wait ends, and the context stays usable
  * (vx_interner_reset clears the sticky status). Defaults: 2^20 rounds, 2^22 spins. */
 int vx_interner_set_limits(vx_interner *it, uint32_t max_probes, uint32_t round_limit, uint32_t spin_limit);
@@ -410,7 +410,7 @@ int vx_interner_maintain(vx_interner *it);
 /* Returns the interner to its freshly created state (no nodes, empty tables, every slot's
  * generation back to 0); tree handles stay valid and their roots become EMPTY. Same result as
  * destroying it and creating a new interner with the same budget, without reallocating device
- * memory. */
+ * memory. Ordered on the interner's stream; the call does not wait for it. */
 int vx_interner_reset(vx_interner *it);
 
 #ifdef __cplusplus

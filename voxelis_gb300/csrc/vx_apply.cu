@@ -716,11 +716,11 @@ __device__ __forceinline__ void phase_bottom(const DevInterner &I, const ApplyAr
     bottom_records(I, a, mode, L, in_turn);
 }
 
-// Whether the release of the roots that the set phase replaced can wait for the clear pass and go with its own: half
-// of the release rounds less (an apply of a tree of depth 9 541 us against 577 for 261 K records, 301 against 363 for
-// 16 K). Counts are sums and no
-// count that the set phase left can fall before, so only the free nodes decide: what the clear pass can make at
-// most has to be free without the set phase's dead. One thread, after the set phase's epoch is closed.
+// Whether the release of the roots that the set phase replaced can wait for the clear pass and go with its own,
+// which leaves out half of the release rounds (an apply of a tree of depth 9 541 us against 577 for 261 K records,
+// 301 against 363 for 16 K). Counts are sums and no count that the set phase left can fall before, so only the free
+// nodes decide: what the clear pass can make at most has to be free without the set phase's dead. One thread, after
+// the set phase's epoch is closed.
 __device__ bool release_can_wait(const DevInterner &I, const uint32_t *total, int max_depth) {
     if (total[0] == 0) return false;  // no clear pass
     uint64_t most = total[0];
