@@ -1962,18 +1962,19 @@ int vx_occupancy_masks_async(vx_interner *it, uint32_t n_builders, uint32_t n_tr
     if (it->vbits != 8) return set_err(it, VX_E_UNSUPPORTED, "the batched occupancy masks take 8-bit voxels");
     if (max_depth < 1 || max_depth > 6) return set_err(it, VX_E_INVALID_ARG, "occupancy masks need MaxDepth 1..6");
     const size_t per = (size_t)1 << (3 * max_depth);
-    VX_CUDA(it->ws.reserve(Carve::need({per * n_trees, (size_t)n_builders * 4, (size_t)n_trees * 4})));
+    VX_CUDA(it->ws.reserve(Carve::need({per * n_trees, (size_t)n_builders * 8, (size_t)n_trees * 4, occupancy_listed_words(n_builders) * 4})));
     Carve c(it->ws.p);
     uint8_t *dg = c.take<uint8_t>(per * n_trees);
-    uint32_t *head = c.take<uint32_t>(n_builders);
+    uint32_t *head = c.take<uint32_t>(2 * (size_t)n_builders);
     uint32_t *next = c.take<uint32_t>(n_trees);
+    uint32_t *listed = c.take<uint32_t>(occupancy_listed_words(n_builders));
     cudaStream_t s = it->stream;
     Phase ph(it, VX_PROF_GET);
     const int lc = max_depth < 5 ? max_depth : 5;
     VX_CUDA(launch_to_dense(it->dev, trees_dev, max_depth, 0, (uint64_t)n_trees << (3 * (max_depth - lc)), dg,
                             it->num_sms, s));
     VX_CUDA(launch_occupancy_many(it->dev, dg, n_trees, max_depth, builder_of_dev, offsets_dev, n_builders, head,
-                                  next, max_materials, material_ids_dev,
+                                  next, listed, max_materials, material_ids_dev,
                                   reinterpret_cast<unsigned long long *>(material_counts_dev), n_materials_dev,
                                   reinterpret_cast<unsigned long long *>(global_dev),
                                   reinterpret_cast<unsigned long long *>(material_masks_dev),

@@ -160,11 +160,12 @@ cudaError_t launch_occupancy(const DevInterner &I, const void *grids, uint32_t n
                              unsigned long long *counts, uint32_t *slot, uint32_t *ids, unsigned long long *mcounts,
                              uint32_t *n_mat, uint32_t mat_cap, unsigned long long *global, unsigned long long *per_mat,
                              unsigned long long *active, int num_sms, cudaStream_t s);
-// Batched occupancy masks, 8-bit voxels: tree t goes to builder builder_of[t]; head (one word a builder)
-// and next (one a tree) are scratch. Every word of the outputs is written.
+// Batched occupancy masks, 8-bit voxels: tree t goes to builder builder_of[t]; head (two words a builder), next
+// (one a tree) and listed (occupancy_listed_words) are scratch. Every word of the outputs is written.
+size_t occupancy_listed_words(uint32_t n_builders);
 cudaError_t launch_occupancy_many(const DevInterner &I, const uint8_t *grids, uint32_t n_trees, int d,
                                   const uint32_t *builder_of, const uint32_t *offsets, uint32_t n_builders,
-                                  uint32_t *head, uint32_t *next, uint32_t max_mat, uint32_t *ids,
+                                  uint32_t *head, uint32_t *next, uint32_t *listed, uint32_t max_mat, uint32_t *ids,
                                   unsigned long long *mcounts, uint32_t *n_mat, unsigned long long *global,
                                   unsigned long long *per_mat, unsigned long long *active, int num_sms, cudaStream_t s);
 // Model serialisation: plan (renumbering, record sizes, offsets, total bytes into *total), then
