@@ -1499,7 +1499,7 @@ __global__ void __launch_bounds__(kThreads) occupancy_active_kernel(const unsign
 // one z, each by one warp with 5 shuffle steps. The global planes are the OR of the materials' (up to
 // three materials) or a plane of their own. Rows of 65 words keep the transposes' column reads free of
 // bank conflicts; 100 KB leave two CTAs to an SM, one writing while the other reads.
-// 4096 dune chunks in 1024 builders, 8 material slots (906 MB): 297 us with the dense expansion, 1750 us
+// 4096 dune chunks in 1024 builders, 8 material slots (906 MB): 302 us with the dense expansion, 1750 us
 // when separate kernels counted voxels (one atomic a warp and value, 812 us), cleared the outputs
 // (137 us) and ORed every line's bits into them with atomics (607 us).
 // Calls with fewer builders than SMs take 1024 threads for each: what bounds them is one CTA's share of the rows
@@ -1652,13 +1652,16 @@ __global__ void __launch_bounds__(kOccThreads, 1024 / kOccThreads) occupancy_bui
         const uint32_t x = offsets[3 * t], y = offsets[3 * t + 1], z = offsets[3 * t + 2];
         return x <= 64 - S && y <= 64 - S && z <= 64 - S ? x | y << 8 | z << 16 : 0xFFFFFFFFu;
     };
+    bool whole = false;  // all of them are there
     const auto load_trees = [&](bool first) {
+        if (whole) return list_n;
         __syncthreads();
         if (first) {
+            const uint32_t t = tid < kOccListed ? listed[(size_t)b * kOccListed + tid] : 0u;  // beside their number
             const uint32_t n = min(head[gridDim.x + b] + 1u, kOccListed);
             if (tid < n) {
-                list_s[tid] = listed[(size_t)b * kOccListed + tid];
-                ofs_s[tid] = offsets_of(list_s[tid]);
+                list_s[tid] = t;
+                ofs_s[tid] = offsets_of(t);
             }
             if (tid == 0) {
                 list_n = n;
@@ -1674,6 +1677,7 @@ __global__ void __launch_bounds__(kOccThreads, 1024 / kOccThreads) occupancy_bui
             list_next = t;
         }
         __syncthreads();
+        whole = first && list_next == kNoTree;
         return list_n;
     };
     const bool wide = ((reinterpret_cast<uintptr_t>(global) | reinterpret_cast<uintptr_t>(per_mat)) & 15u) == 0;
