@@ -32,8 +32,11 @@ __device__ __forceinline__ uint64_t get_child(const DevInterner &I, uint64_t nod
 }
 
 // Large batches of gets start from a table of the nodes k levels below every root: one load instead of k
-// dependent ones. Tree t's entries are at t << 3k, by (y, z, x) of the node. Trees of less than k levels
-// have entries at their depth.
+// dependent ones. Tree t's entries are at t << 3k, by (y, z, x) of the node. In a tree of d <= k levels they are the
+// nodes of depth d - 1: a leaf met above depth d is a voxel whatever its value, one at depth d only when that is not
+// the default, and an entry does not say where its leaf was met.
+__device__ __forceinline__ int get_levels(int d, int k) { return d > k ? k : (d > 0 ? d - 1 : 0); }
+
 __device__ __forceinline__ uint32_t get_entry(uint32_t x, uint32_t y, uint32_t z, int d, int k) {
     return ((y >> (d - k)) << (2 * k)) | ((z >> (d - k)) << k) | (x >> (d - k));
 }
@@ -44,7 +47,7 @@ __global__ void __launch_bounds__(kThreads) get_table_kernel(DevInterner I, uint
         const uint32_t t = (uint32_t)(i >> (3 * k)), e = (uint32_t)(i & ((1ull << (3 * k)) - 1ull));
         const int d = I.depths[t];
         if (d == TREE_UNUSED) continue;
-        const int kt = d < k ? d : k;
+        const int kt = get_levels(d, k);
         if (e >> (3 * kt)) continue;
         const uint32_t m = (1u << kt) - 1u, x = e & m, z = (e >> kt) & m, y = e >> (2 * kt);
         uint64_t node = I.roots[t];
@@ -76,7 +79,7 @@ __global__ void __launch_bounds__(kThreads) get_kernel(DevInterner I, uint64_t n
         if (in) {
             shift = d - 1;
             if (TABLE && t < n_trees) {  // (a replayed graph may name trees created since it was captured)
-                const int kt = d < k ? d : k;
+                const int kt = get_levels(d, k);
                 node = __ldg((const unsigned long long *)table + ((uint64_t)t << (3 * k)) + get_entry(x, y, z, d, kt));
                 shift -= kt;
             } else {
