@@ -139,7 +139,8 @@ __device__ __forceinline__ void leaf_refs_flush(const DevInterner &I, const Leaf
 
 // ---- items ---------------------------------------------------------------------------------------
 // Depth of item i: given by the host, or (check_depths) read from the tree table with the checks of a
-// device-resident call, an item that fails them counting as a tree of depth 2.
+// device-resident call. An item that fails them counts as a tree of depth 1, of which no record heads a parent:
+// nothing of it is applied.
 __device__ __forceinline__ int item_depth_of(const DevInterner &I, const ApplyArgs &a, uint32_t i, bool check_depths,
                                              bool *bad = nullptr) {
     if (!check_depths) return a.it_depth[i];
@@ -152,7 +153,7 @@ __device__ __forceinline__ int item_depth_of(const DevInterner &I, const ApplyAr
     }
     if (d == TREE_UNUSED || d > a.max_depth || d < 2 || (i > 0 && d > prev)) {
         if (bad) *bad = true;
-        return 2;
+        return 1;
     }
     return d;
 }
@@ -162,15 +163,15 @@ __device__ __forceinline__ uint64_t item_root(const DevInterner &I, const ApplyA
     return t < I.tree_cap ? I.roots[t] : EMPTY_ID;
 }
 
-// Phase 0 of item i (set phase).
-__device__ __forceinline__ void prep_item(const DevInterner &I, const ApplyArgs &a, uint32_t i) {
+// Phase 0 of item i (set phase); refused: it failed the checks of its depth.
+__device__ __forceinline__ void prep_item(const DevInterner &I, const ApplyArgs &a, uint32_t i, bool refused) {
     const uint64_t old = item_root(I, a, i);
     const uint8_t f = a.it_flags[i];
     uint64_t init = old;
     a.it_old[i] = old;
-    a.it_panic[i] = 0;
+    a.it_panic[i] = refused;
     a.it_changed[i] = 0;
-    if (f & 1) {
+    if ((f & 1) && !refused) {
         bool created;
         const uint64_t fill = intern_leaf(I, a.it_fill[i], &created);
         init = fill;
@@ -179,17 +180,36 @@ __device__ __forceinline__ void prep_item(const DevInterner &I, const ApplyArgs 
     a.it_init[i] = init;
 }
 
-// The root of item i is nw (mode 0: the set phase, voxtree.rs:303-328; mode 1: the clear pass).
+// Whether item i has records: by the host's counts, or by a search in the sorted records of a device-resident call.
+__device__ __forceinline__ bool item_has_records(const ApplyArgs &a, uint32_t i) {
+    if (a.it_first) return a.it_first[i] < a.it_first[i + 1];
+    uint32_t lo = 0, hi = a.n_records;
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if (a.rec_item[mid] < i)
+            lo = mid + 1;
+        else
+            hi = mid;
+    }
+    return lo < a.n_records && a.rec_item[lo] == i;
+}
+
+// The root of item i is nw (mode 0: the set phase, voxtree.rs:303-328; mode 1: the clear pass). Once an item and
+// mode, whatever the records are (release_list has a place for each, and a root is released once): the first to
+// come takes the item's word, it_old of the set phase and it_init of the clear pass. Records in order name an item's
+// root once; others are an error.
 __device__ __forceinline__ void finish_item(const DevInterner &I, const ApplyArgs &a, int mode, uint32_t i, uint64_t nw) {
     const uint32_t t = a.it_tree[i];
-    if (t >= I.tree_cap) return;
-    uint64_t old;
+    if (t >= I.tree_cap || (mode == 0 && a.it_panic[i])) return;
+    uint64_t old = atomicExch((unsigned long long *)(mode ? a.it_init : a.it_old) + i, INVALID_ID);
+    if (old == INVALID_ID) {
+        set_error(I, ERR_INVALID, 48);
+        return;
+    }
     if (mode == 1) {
         old = I.roots[t];
         if (nw != EMPTY_ID) atomicAdd(I.refcount + id_index(nw), 1u);
     } else {
-        if (a.it_panic[i]) return;
-        old = a.it_old[i];
         if ((a.it_flags[i] & 3) && nw != EMPTY_ID) atomicAdd(I.refcount + id_index(nw), 1u);  // the tree's root reference
         if (old != EMPTY_ID && nw == old && !(I.flags & (1u << 4))) {  // assert_ne!(new_root_id, self.root_id) (voxtree.rs:311)
             set_error(I, ERR_REF_PANIC, 41);
@@ -231,20 +251,20 @@ struct Tiles {
     }
 };
 
-// Steps that record r (of item i and group g, depth d) heads: 1 .. the result. Whole warp, lanes in order.
-__device__ __forceinline__ uint32_t head_steps(const ApplyArgs &a, uint64_t r, bool in, uint32_t i, uint32_t g, int d,
-                                               bool *first = nullptr) {
+// Whether a tree of depth d has bottom group g.
+__device__ __forceinline__ bool group_in_tree(uint32_t g, int d) { return g >> (3 * (d - 1)) == 0; }
+
+// Steps that record r (of item i and group g, depth d) heads: 1 .. the result, none for a group outside the tree.
+// The one of an item that heads all d - 1 is its first. Whole warp, lanes in order.
+__device__ __forceinline__ uint32_t head_steps(const ApplyArgs &a, uint64_t r, bool in, uint32_t i, uint32_t g, int d) {
     uint32_t ip = __shfl_up_sync(0xFFFFFFFFu, i, 1), gp = __shfl_up_sync(0xFFFFFFFFu, g, 1);
-    if (!in) return 0;
+    if (!in || !group_in_tree(g, d)) return 0;
     const uint32_t top = (uint32_t)d - 1u;
     if ((threadIdx.x & 31u) == 0 && r > 0) {
         ip = a.rec_item[r - 1];
         gp = a.rec_group[r - 1];
     }
-    if (r == 0 || ip != i) {
-        if (first) *first = true;
-        return top;
-    }
+    if (r == 0 || ip != i) return top;
     const uint32_t x = g ^ gp, s = x ? (31u - __clz(x)) / 3u : 0u;
     return s < top ? s : top;
 }
@@ -261,11 +281,10 @@ __device__ __forceinline__ void plan_count(const DevInterner &I, const ApplyArgs
         const bool in = r < a.n_records;
         const uint32_t i = in ? a.rec_item[r] : 0u, g = in ? a.rec_group[r] : 0u;
         const int d = in ? item_depth_of(I, a, i, check_depths) : 2;
-        bool first = false;
-        const uint32_t hs = head_steps(a, r, in, i, g, d, &first);
+        const uint32_t hs = head_steps(a, r, in, i, g, d);
         if (lane < kPlanWords) a.tile_base[(uint64_t)tile * kPlanWords + lane] = acc;
         // the first record of an item heads every step up to its root's
-        for (unsigned h = __ballot_sync(0xFFFFFFFFu, first); h; h &= h - 1) {
+        for (unsigned h = __ballot_sync(0xFFFFFFFFu, hs && hs == (uint32_t)d - 1u); h; h &= h - 1) {
             const uint32_t root_step = __shfl_sync(0xFFFFFFFFu, hs, __ffs(h) - 1);
             if (lane == kRootWord + root_step) ++acc;
         }
@@ -377,6 +396,10 @@ __device__ __forceinline__ void bottom_records(const DevInterner &I, const Apply
         if (in) {
             set = mode ? a.rec_clear[r] : a.rec_set[r];
             if (set == 0 || a.it_panic[i]) active = false;
+            if (!group_in_tree(g, d)) {
+                set_error(I, ERR_INVALID, 49);
+                active = false;
+            }
         }
         if (active || hs) cur = mode ? item_root(I, a, i) : a.it_init[i];
         // descend to depth d-1 (voxtree.rs:792-822); at step s the node is the old one of the parent there
@@ -680,8 +703,9 @@ __device__ __forceinline__ void parents_range(const DevInterner &I, const ApplyA
         if (created) add_child_refs(I, L, c, cv);
         if (!in) continue;
         if (want_branch) out = id;
-        if (d - 1u == s) {
-            if (changed) finish_item(I, a, mode, i, out);
+        if (d - 1u == s) {  // (a fill without the patches bit is the root that unchanged records leave)
+            if (changed || (mode == 0 && !(a.it_flags[i] & 2))) finish_item(I, a, mode, i, changed ? out : a.it_init[i]);
+            a.e_val[s & 1][p] = 0;  // no entry of the next step's (records out of order may leave it within a run)
         } else {
             a.e_id[s & 1][p] = out;
             a.e_val[s & 1][p] = entry_word(out_val, path, changed);
@@ -696,23 +720,23 @@ __device__ __forceinline__ void phase_plan(const DevInterner &I, const ApplyArgs
     const uint64_t gt = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
     if (gt == 0) I.ctr->scratch[SC_RELEASE] = 0;
     for (uint64_t i = gt; i < a.n_items; i += stride) {
+        bool bad = false;
         if (check_depths) {
-            bool bad = false;
             const_cast<uint8_t *>(a.it_depth)[i] = (uint8_t)item_depth_of(I, a, (uint32_t)i, true, &bad);
             if (bad) set_error(I, ERR_INVALID, 46);
         }
-        prep_item(I, a, (uint32_t)i);
+        prep_item(I, a, (uint32_t)i, bad);
     }
     plan_count(I, a, check_depths, cnt_s);
 }
 
-// Phase 1, and the roots of the items that have none of it.
+// Phase 1, and the roots of the items without patches and records.
 __device__ __forceinline__ void phase_bottom(const DevInterner &I, const ApplyArgs &a, int mode, const LeafRefs &L,
                                              bool in_turn) {
     const uint64_t gt = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
     if (mode == 0)
         for (uint64_t i = gt; i < a.n_items; i += stride)
-            if (!(a.it_flags[i] & 2)) finish_item(I, a, 0, (uint32_t)i, a.it_init[i]);
+            if (!(a.it_flags[i] & 2) && !item_has_records(a, (uint32_t)i)) finish_item(I, a, 0, (uint32_t)i, a.it_init[i]);
     bottom_records(I, a, mode, L, in_turn);
 }
 
