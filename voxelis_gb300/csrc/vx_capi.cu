@@ -216,7 +216,8 @@ struct vx_interner {
     uint32_t *frontier = nullptr;  // 2 * capacity u32 (the single-thread queue aliases it under P3)
     uint64_t *seq_queue = nullptr;
     uint64_t seq_queue_cap = 0;
-    uint64_t *get_table = nullptr;  // kGetTableEntries words, filled and read by one call's launches
+    uint64_t *get_table = nullptr;  // kGetTableEntries words, filled and read by one call's launches, one call after
+                                    // the other: the stream orders them (a change of stream waits for the old one)
     std::mutex get_mutex;           // queues a call's launches together: callers may read from several threads
     unsigned long long *d_live = nullptr;
     // pinned staging
@@ -1640,7 +1641,13 @@ namespace {
 cudaError_t queue_gets(vx_interner *it, uint64_t n, const uint32_t *trees, const int32_t *xyz, uint8_t *found, void *values) {
     Phase ph(it, VX_PROF_GET);
     std::lock_guard<std::mutex> lock(it->get_mutex);
-    const int k = get_table_levels(n, it->tree_count, depth_limit(it->flags) - 1);
+    int k = get_table_levels(n, it->tree_count, depth_limit(it->flags) - 1);
+    if (k > 0) {  // graphs may be replayed side by side, on any streams: those reads share no table
+        cudaStreamCaptureStatus capture;
+        const cudaError_t e = cudaStreamIsCapturing(it->stream, &capture);
+        if (e != cudaSuccess) return e;
+        if (capture != cudaStreamCaptureStatusNone) k = 0;
+    }
     return launch_get_many(it->dev, n, trees, xyz, found, values, it->get_table, k, it->tree_count, it->num_sms, it->stream);
 }
 }  // namespace

@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kThreads) get_kernel(DevInterner I, uint64_t n
         int shift = -1;  // of the child slot's coordinate bits, -1 at depth d
         if (in) {
             shift = d - 1;
-            if (TABLE && t < n_trees) {  // (a replayed graph may name trees created since it was captured)
+            if (TABLE && t < n_trees) {  // (handles past the known ones: t < tree_cap)
                 const int kt = get_levels(d, k);
                 node = __ldg((const unsigned long long *)table + ((uint64_t)t << (3 * k)) + get_entry(x, y, z, d, kt));
                 shift -= kt;
