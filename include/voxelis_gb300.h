@@ -24,7 +24,9 @@
  *   - All device work is ordered on the interner's stream (vx_interner_set_stream). Calls that
  *     return results in host memory synchronise that stream before returning; the *_async calls
  *     do not, and their status is reported by the next vx_interner_sync.
- *   - One writer at a time per interner, as in the reference (&mut VoxInterner).
+ *   - One writer at a time per interner, as in the reference (&mut VoxInterner). Between writes several
+ *     threads may read voxels at once (vx_tree_get, vx_get_many, vx_get_many_async, vx_tree_to_dense,
+ *     vx_trees_to_dense, vx_trees_to_dense_async): the calls take turns. Every other call is made alone.
  */
 #ifndef VOXELIS_GB300_H
 #define VOXELIS_GB300_H

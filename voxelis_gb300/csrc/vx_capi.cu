@@ -218,7 +218,8 @@ struct vx_interner {
     uint64_t seq_queue_cap = 0;
     uint64_t *get_table = nullptr;  // kGetTableEntries words, filled and read by one call's launches, one call after
                                     // the other: the stream orders them (a change of stream waits for the old one)
-    std::mutex get_mutex;           // queues a call's launches together: callers may read from several threads
+    std::mutex read_mutex;          // held by the calls that read voxels, from their checks to their results: they share
+                                    // staging, pinned memory, the counters, the reply, the table and the last error
     unsigned long long *d_live = nullptr;
     // pinned staging
     DevCounters *h_ctr = nullptr;
@@ -1158,10 +1159,10 @@ int vx_tree_set(vx_interner *it, vx_tree tree, int32_t x, int32_t y, int32_t z, 
 
 int vx_tree_get(vx_interner *it, vx_tree tree, int32_t x, int32_t y, int32_t z, int *found, uint32_t *value) {
     if (!it || !found || !value || !tree_ok(it, tree)) return VX_E_INVALID_ARG;
+    std::lock_guard<std::mutex> lock(it->read_mutex);
     const int32_t side = 1 << it->tree_depth[tree];
     if (x < 0 || y < 0 || z < 0 || x >= side || y >= side || z >= side)
         return set_err(it, VX_E_OOB, "position out of bounds");
-    std::lock_guard<std::mutex> lock(it->get_mutex);  // readers share the reply
     {
         Phase ph(it, VX_PROF_GET);
         VX_CUDA(launch_tree_get(it->dev, tree, x, y, z, it->h_reply, it->stream));
@@ -1637,10 +1638,9 @@ int vx_build_dense(vx_interner *it, uint32_t n, const vx_tree *trees, const void
 
 }  // extern "C"
 namespace {
-// Queues the gets of one call (device memory) on the interner's stream.
+// Queues the gets of one call (device memory) on the interner's stream. The caller holds read_mutex.
 cudaError_t queue_gets(vx_interner *it, uint64_t n, const uint32_t *trees, const int32_t *xyz, uint8_t *found, void *values) {
     Phase ph(it, VX_PROF_GET);
-    std::lock_guard<std::mutex> lock(it->get_mutex);
     int k = get_table_levels(n, it->tree_count, depth_limit(it->flags) - 1);
     if (k > 0) {  // graphs may be replayed side by side, on any streams: those reads share no table
         cudaStreamCaptureStatus capture;
@@ -1656,6 +1656,7 @@ extern "C" {
 int vx_get_many_async(vx_interner *it, uint64_t n, const vx_tree *trees_dev, const int32_t *xyz_dev,
                       uint8_t *found_dev, void *values_dev) {
     if (!it || (n && (!trees_dev || !xyz_dev || !found_dev || !values_dev))) return VX_E_INVALID_ARG;
+    std::lock_guard<std::mutex> lock(it->read_mutex);
     VX_CUDA(queue_gets(it, n, trees_dev, xyz_dev, found_dev, values_dev));
     return VX_OK;
 }
@@ -1668,6 +1669,7 @@ int vx_get_many(vx_interner *it, uint64_t n, const vx_tree *trees, const int32_t
                 vx_mem mem) {
     if (!it || (n && (!trees || !xyz || !found || !values))) return VX_E_INVALID_ARG;
     if (n == 0) return VX_OK;
+    std::lock_guard<std::mutex> lock(it->read_mutex);
     if (mem == VX_MEM_DEVICE) {
         VX_CUDA(queue_gets(it, n, trees, xyz, found, values));
         return sync_and_check(it);
@@ -1816,6 +1818,7 @@ int vx_validate(vx_interner *it, uint32_t n_trees, const vx_tree *trees) {
 
 int vx_trees_to_dense_async(vx_interner *it, uint32_t n, const vx_tree *trees_dev, int depth, void *out_dev) {
     if (!it || depth < 1 || depth > 10 || (n && (!trees_dev || !out_dev))) return VX_E_INVALID_ARG;
+    std::lock_guard<std::mutex> lock(it->read_mutex);
     if (reinterpret_cast<uintptr_t>(out_dev) % 16) return set_err(it, VX_E_INVALID_ARG, "out_dev must be 16-byte aligned");
     if (n == 0) return VX_OK;
     const int lc = depth < 5 ? depth : 5;
@@ -1828,6 +1831,7 @@ int vx_trees_to_dense_async(vx_interner *it, uint32_t n, const vx_tree *trees_de
 int vx_trees_to_dense(vx_interner *it, uint32_t n, const vx_tree *trees, void *out, vx_mem mem) {
     if (!it || (n && (!trees || !out))) return VX_E_INVALID_ARG;
     if (n == 0) return VX_OK;
+    std::lock_guard<std::mutex> lock(it->read_mutex);
     const int d = tree_ok(it, trees[0]) ? (int)it->tree_depth[trees[0]] : -1;
     for (uint32_t k = 0; k < n; ++k)
         if (!tree_ok(it, trees[k]) || it->tree_depth[trees[k]] != d) return VX_E_INVALID_ARG;
