@@ -412,7 +412,8 @@ int vx_interner_maintain(vx_interner *it);
 /* Returns the interner to its freshly created state (no nodes, empty tables, every slot's
  * generation back to 0); tree handles stay valid and their roots become EMPTY. Same result as
  * destroying it and creating a new interner with the same budget, without reallocating device
- * memory. Ordered on the interner's stream; the call does not wait for it. */
+ * memory. What was queued before it on the interner's stream is done when it returns; the reset itself is
+ * ordered on that stream. */
 int vx_interner_reset(vx_interner *it);
 
 #ifdef __cplusplus
