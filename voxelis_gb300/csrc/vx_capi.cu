@@ -8,6 +8,7 @@
 #include <atomic>
 #include <cstring>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -1337,6 +1338,15 @@ int vx_apply_groups_async(vx_interner *it, uint32_t n_items, const vx_tree *tree
     return VX_OK;
 }
 
+}  // extern "C"
+namespace {
+// So many calls of one vx_trees_set_many go through pinned memory, which the interner keeps (25 bytes a call): 138 us
+// against 147 for 1024 calls on 64 trees of depth 5, 621 against 630 for 8192, 4.20 ms against 4.21 for 65536; larger
+// ones gain nothing (17.7 ms and 17.7 for 262144 on 4096 trees).
+constexpr uint64_t kPinnedSets = 1ull << 16;
+}  // namespace
+extern "C" {
+
 int vx_trees_set_many(vx_interner *it, uint64_t n, const vx_tree *trees, const int32_t *xyz, const uint32_t *values,
                       uint8_t *changed) {
     if (!it || (n && (!trees || !xyz || !values))) return VX_E_INVALID_ARG;
@@ -1372,10 +1382,15 @@ int vx_trees_set_many(vx_interner *it, uint64_t n, const vx_tree *trees, const i
     const bool octants = trees_set_octants((uint32_t)G, n, it->num_sms);
     // old roots + every node the calls can create, twice where the octants' calls may be run again in order
     const size_t list_cap = G + (size_t)n * (dmax + 1) * (octants ? 2 : 1) + 16;
-    // the arguments are laid out alike in pinned and in device memory: one copy
+    // the arguments are laid out alike in host and in device memory: one copy
     VX_CUDA(it->ws.reserve(Carve::need({G * 4, (G + 1) * 4, n * 12, n * 4, n * 4, n, G * 8, list_cap * 8, n * 8})));
-    VX_CUDA(it->pinned.reserve(Carve::need({G * 4, (G + 1) * 4, n * 12, n * 4, n * 4, n})));
-    Carve hc(it->pinned.p), c(it->ws.p);
+    const size_t host_bytes = Carve::need({G * 4, (G + 1) * 4, n * 12, n * 4, n * 4, n});
+    std::unique_ptr<char[]> pageable;
+    if (n <= kPinnedSets)
+        VX_CUDA(it->pinned.reserve(host_bytes));
+    else
+        pageable.reset(new char[host_bytes]);
+    Carve hc(pageable ? pageable.get() : it->pinned.p), c(it->ws.p);
     uint32_t *h_group = hc.take<uint32_t>(G), *d_group = c.take<uint32_t>(G);
     uint32_t *h_begin = hc.take<uint32_t>(G + 1), *d_begin = c.take<uint32_t>(G + 1);
     int32_t *h_xyz = hc.take<int32_t>(3 * n), *d_xyz = c.take<int32_t>(3 * n);
