@@ -99,7 +99,10 @@ __global__ void __launch_bounds__(kThreads) get_kernel(DevInterner I, uint64_t n
 // ---- release (bodies in vx_device.cuh, shared with the single-launch apply) ------------------------
 // The listed roots and then rounds until no node dies, one cooperative launch with a grid barrier after each
 // (a launch per round, empty ones too, took 18 us a round on the few hundred nodes of a served wave).
-__global__ void __launch_bounds__(kThreads) release_kernel(DevInterner I, const uint64_t *list, uint32_t *frontier_a,
+// kReleaseCtas an SM, all resident, as the barrier needs: the bounds hold the registers to it, and release_smem is at
+// most 32 KB.
+constexpr int kReleaseCtas = 2;
+__global__ void __launch_bounds__(kThreads, kReleaseCtas) release_kernel(DevInterner I, const uint64_t *list, uint32_t *frontier_a,
                                                            uint32_t *frontier_b, int rounds, int may_wait) {
     extern __shared__ uint32_t release_mem[];
     if (may_wait && *(volatile unsigned long long *)&I.ctr->scratch[SC_DEFER]) return;  // the list waits for the next release
@@ -2257,8 +2260,7 @@ cudaError_t launch_release(const DevInterner &I, uint64_t *list, uint32_t *front
     int wait = may_wait ? 1 : 0;
     void *args[] = {&Ic, &l, &frontier_a, &frontier_b, &rounds, &wait};
     count_launches(1);
-    // two CTAs an SM are resident at any register and shared-memory use of the kernel
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(release_kernel), dim3((unsigned)num_sms * 2),
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(release_kernel), dim3((unsigned)num_sms * kReleaseCtas),
                                        dim3(kThreads), args, release_smem(I.vbits), s);
 }
 
