@@ -798,12 +798,13 @@ __global__ void __launch_bounds__(512, VX_APPLY_MIN_BLOCKS) apply_parents_kernel
 }
 
 // ---- the whole apply in one launch ---------------------------------------------------------------------
-// One cluster: its hardware barrier.
+// One cluster: its hardware barrier, in the form that a warp's threads may come to apart (phases end behind
+// branches of single threads).
 struct ClusterBarrier {
     __device__ explicit ClusterBarrier(const DevInterner &) {}
     __device__ bool usable() { return true; }
     __device__ bool sync() {
-        asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
         return true;
     }
     __device__ void leave() {}
