@@ -544,8 +544,8 @@ int apply_sequence(vx_interner *it, ApplyArgs &a, bool clear_pass, bool check_de
         }
         {
             Phase ph(it, VX_PROF_RELEASE);
-            VX_CUDA(launch_release(it->dev, a.release_list, it->frontier, it->frontier + it->capacity, it->capacity,
-                                   rounds, it->num_sms, s, clear_pass && mode == 0));
+            VX_CUDA(launch_release(it->dev, a.release_list, it->frontier, it->frontier + it->capacity, rounds, it->num_sms, s,
+                                   clear_pass && mode == 0));
         }
     }
     return VX_OK;
@@ -802,8 +802,8 @@ void interner_set_error(vx_interner *it, const char *msg) {
 // breadth-first rounds, on the interner's stream.
 int interner_release_list(vx_interner *it, uint64_t *list_dev, int rounds) {
     Phase ph(it, VX_PROF_RELEASE);
-    VX_CUDA(launch_release(it->dev, list_dev, it->frontier, it->frontier + it->capacity, it->capacity, rounds,
-                           it->num_sms, it->stream));
+    VX_CUDA(launch_release(it->dev, list_dev, it->frontier, it->frontier + it->capacity, rounds, it->num_sms,
+                           it->stream));
     return VX_OK;
 }
 }  // namespace vxg

@@ -114,12 +114,6 @@ __host__ __device__ __forceinline__ uint64_t make_branch_id(uint32_t index, uint
            ((uint64_t)(gen & 0x7FFF) << 32) | index;
 }
 
-// Sibling-prefix mask PATH_MASKS[d][k] (voxtree.rs:41-105), closed form.
-__host__ __device__ __forceinline__ uint32_t path_mask(int d, int k) {
-    if (d <= 0 || k > d - 1) return 0;
-    return ((1u << (3 * (k + 1))) - 1u) << (3 * (d - 1 - k));
-}
-
 // ---- memory helpers --------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t ld_volatile(const uint64_t *p) { return *(const volatile uint64_t *)p; }
 // Acquire load of a table slot: the node record published before the slot is visible after it.

@@ -207,9 +207,10 @@ cudaError_t launch_vtm_place(const DevInterner &I, const uint8_t *bytes, const V
                              const uint32_t *chunk_off, const uint32_t *trees, int32_t *positions, int num_sms,
                              cudaStream_t s);
 // Releases the roots listed in `list` (count at ctr->scratch[SC_RELEASE]) with `rounds`
-// breadth-first rounds, using two frontier buffers of `frontier_cap` entries.
+// breadth-first rounds, using two frontier buffers of as many entries as the interner has nodes. With may_wait the
+// roots stay listed where the apply left them for its clear pass.
 cudaError_t launch_release(const DevInterner &I, uint64_t *list, uint32_t *frontier_a, uint32_t *frontier_b,
-                           uint64_t frontier_cap, int rounds, int num_sms, cudaStream_t s, bool may_wait = false);
+                           int rounds, int num_sms, cudaStream_t s, bool may_wait = false);
 // One-tree calls answer in pinned host memory, valid once the stream has been waited for.
 struct HostReply {
     int status;

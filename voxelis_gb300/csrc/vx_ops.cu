@@ -2253,8 +2253,7 @@ cudaError_t launch_get_many(const DevInterner &I, uint64_t n, const uint32_t *tr
 }
 
 cudaError_t launch_release(const DevInterner &I, uint64_t *list, uint32_t *frontier_a, uint32_t *frontier_b,
-                           uint64_t frontier_cap, int rounds, int num_sms, cudaStream_t s, bool may_wait) {
-    (void)frontier_cap;
+                           int rounds, int num_sms, cudaStream_t s, bool may_wait) {
     DevInterner Ic = I;
     const uint64_t *l = list;
     int wait = may_wait ? 1 : 0;
@@ -2302,7 +2301,7 @@ cudaError_t launch_trees_set(const DevInterner &I, const SetCalls &c, uint64_t *
     count_launches(2);
     trees_set_roots_kernel<<<gr ? gr : 1, kThreads, 0, s>>>(I, c, list);
     trees_set_garbage_kernel<<<(unsigned)num_sms * 4, kThreads, 0, s>>>(I, fc0, ni0, list);
-    return launch_release(I, list, frontier_a, frontier_b, 0, max_depth + 2, num_sms, s);
+    return launch_release(I, list, frontier_a, frontier_b, max_depth + 2, num_sms, s);
 }
 
 cudaError_t launch_tree_fill(const DevInterner &I, uint32_t tree, uint32_t v, uint64_t *queue, uint64_t queue_cap,
