@@ -516,11 +516,15 @@ int carve_apply(vx_interner *it, uint32_t n, uint64_t R, int max_depth, bool own
 }
 
 // Deep trees of so many records run faster as launches that start early (programmatic dependents) than behind the
-// single launch's barriers, two a level. Launches against the single one, an apply of a tree of depth 9: 429 against
-// 388 us for 32 K records, 446 against 427 for 64 K, 486 against 515 for 128 K, 583 against 615 for 261 K; of depth 8
-// 417 against 429 for 125 K, 487 against 499 for 248 K; of depth 7 399 and 402 for 172 K. Chunks: 292 and 296 for
-// 153 K, 315 against 301 for 191 K, 431 against 425 for 399 K, 515 against 507 for 784 K.
-constexpr uint64_t kLaunchesFrom = 1ull << 17, kLaunchesTo = 1ull << 19;
+// single launch's barriers, two a level. Launches against the single one, an apply (us):
+//   records    98-100 K   136-140 K  192-200 K  248-262 K  282-300 K  334-360 K  394-430 K  451-500 K
+//   depth 8    327 / 327  348 / 364  393 / 398  420 / 433  446 / 453  516 / 498  531 / 520  577 / 567
+//   depth 9    381 / 383  401 / 431  474 / 484  519 / 537  540 / 555  615 / 604  657 / 654  688 / 684
+//   depth 10   444 / 444  488 / 525  585 / 584  646 / 678  690 / 711  762 / 763  810 / 818  866 / 881
+// From 530 K records on launches lead again, by 1 to 5 % (depth 8 656 / 675 for 530 K, depth 9 900 / 911 for 783 K,
+// depth 10 946 / 997 for 599 K and 1292 / 1318 for 998 K), which the rule leaves to the one launch so far. Depth 7
+// 399 / 402 for 172 K. Chunks: 292 / 296 for 153 K, 315 / 301 for 191 K, 431 / 425 for 399 K, 515 / 507 for 784 K.
+constexpr uint64_t kLaunchesFrom = 1ull << 17, kLaunchesTo = 5ull << 16;
 constexpr int kLaunchesDepth = 8;
 
 // The set phase (its kernels count references as they create nodes and close the allocation epoch)
