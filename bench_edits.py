@@ -272,8 +272,8 @@ def measure(args, full_line=False):
         "batched_over_per_chunk": pc_ms / apply_ms,
         "phases_ms_per_step": phases_ms,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": B.profiled_traffic("apply_edits_uneven192.md"),
-                     "kernel": "whole apply sequence (bottom groups, level passes, refcount epoch, release)",
+                     "traffic": B.profiled_traffic("apply_grid_uneven1536.md"),
+                     "kernel": "the whole apply (plan, bottom groups, level passes, epoch, release)",
                      "algorithmic_bytes": int(algo), "peak_kind": peak_kind},
         "e2e": {"value": n_edits / (e2e_ms * 1e-3), "unit": "edits/s", "ms": e2e_ms,
                 "h2d_bytes_per_step": int(R * 26 + n * 16), "d2h_bytes_per_step": int(n), "same_dag": e2e_same},
